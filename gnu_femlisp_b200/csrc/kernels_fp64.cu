@@ -4,10 +4,10 @@
 // arrays): A[s * Np + i] = A(i, i + off_s), Np = node count rounded up to a
 // multiple of 64 so that every slot array starts on a 512-byte boundary.
 // Column indices are implicit (off_s = ox + M oy + M^2 oz), so the matvec
-// streams only matrix values: 128-bit loads of two consecutive rows per
-// thread, coalesced across the warp.  Entries outside the grid, in eliminated
-// Dirichlet columns and structurally absent Q2 couplings are stored as zeros,
-// which lets neighbour indices be clamped to the vector instead of tested.
+// streams only matrix values, coalesced across the warp (a row per thread).
+// Entries outside the grid, in eliminated Dirichlet columns and structurally
+// absent Q2 couplings are stored as zeros, which lets neighbour indices be
+// clamped to the vector instead of tested.
 #include <algorithm>
 #include <cstring>
 #include <type_traits>
@@ -16,6 +16,14 @@
 namespace fmg {
 
 std::atomic<long long> g_launches{0};
+
+// The Q1 row kernels: 128 threads, four blocks per SM.  The bound matters for
+// its effect on register allocation: without it ptxas keeps the 3D kernels at
+// 32-40 registers by moving each load down to its multiply-add, and a row
+// waits for memory several times; with it (up to 128 registers) all 54 loads
+// of a row are in flight at once.  Two to eight blocks measured alike.
+constexpr int kRowT = 128;
+constexpr int kRowMinBlocks = 4;
 
 template <int D, int P>
 struct St {
@@ -320,54 +328,72 @@ __device__ __forceinline__ Reduce batch_reduce(Reduce R, unsigned bq) {
 }
 
 // ----------------------------------------------------------------- matvec
-// y = A x (RES = false) or r = b - A x (RES = true, b may alias r); with DOT
-// the chunk reduction of (y, dv) is fused in (DR4096 order).
-template <int D, int P, bool RES, bool DOT>
-__global__ void __launch_bounds__(kBlock)
-k_spmv(const double* __restrict__ A, long long N, long long Np, long long M,
-       const double* __restrict__ x, const double* b, double* y, const double* __restrict__ dv,
-       Reduce R) {
-  constexpr int NS = St<D, P>::NS;
-  __shared__ double smem[8];
+// One Q1 row: sum_s A(i, s) x(i + off_s) over the 3^D slots in slot order; dg
+// gets the diagonal.  All 2 x 3^D loads are issued before the first
+// multiply-add, so a row waits for memory once.  Neighbours outside the level
+// meet stored zeros and are clamped to its first or last node.
+// Bound by HBM on large levels (257^3 nodes: 556 us per matvec, 7.0 TB/s; 659
+// us with two rows per thread and eight such steps per block, the loads then
+// waited for slot by slot) and by one memory round trip on small ones (17^3:
+// 5.3 us instead of 39 us, where that form gave work to two blocks only).  A
+// fused dot product needs that form's thread-to-row map, so the reduction is
+// a pass of its own (257^3: 42 us, less than the fused form lost).
+template <int D>
+__device__ __forceinline__ double q1_row_sum(const double* __restrict__ A, long long Np, int N, int M,
+                                             const double* __restrict__ x, int i, double& dg) {
+  constexpr int NS = St<D, 1>::NS, C = St<D, 1>::CENTER;
+  double av[NS], xv[NS];
+  const double* a = A + i;
+#pragma unroll
+  for (int s = 0; s < NS; ++s) av[s] = __ldg(a + s * Np);
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    const int o = (s % 3 - 1) + (D > 1 ? M * ((s / 3) % 3 - 1) : 0) + (D > 2 ? M * M * (s / 9 - 1) : 0);
+    xv[s] = __ldg(x + min(max(i + o, 0), N - 1));
+  }
+  dg = av[C];
+  double sum = 0.0;
+#pragma unroll
+  for (int s = 0; s < NS; ++s) sum = fma(av[s], xv[s], sum);
+  return sum;
+}
+
+// y = A x (RES = false) or r = b - A x (RES = true, b may alias r) on a Q1
+// level, one row per thread
+template <int D, bool RES>
+__global__ void __launch_bounds__(kRowT, kRowMinBlocks)
+k_row_q1(const double* __restrict__ A, int N, long long Np, int M, const double* __restrict__ x, const double* b,
+         double* y) {
+  const int i = blockIdx.x * kRowT + threadIdx.x;
+  if (i >= N) return;
   const long long bq = blockIdx.y;  // problem of a batched level
-  A += bq * NS * Np;
+  A += bq * St<D, 1>::NS * Np;
   x += bq * Np;
   y += bq * Np;
-  if (RES) b += bq * Np;
-  if (DOT) {
-    dv += bq * Np;
-    R = batch_reduce(R, (unsigned)bq);
-  }
-  const long long base = (long long)blockIdx.x * kChunk + 2 * threadIdx.x;
-  double acc = 0.0;
-#pragma unroll 1
-  for (int m = 0; m < kPairsPerThread; ++m) {
-    const long long i0 = base + 512LL * m;
-    if (i0 >= N) break;
-    const bool two = i0 + 1 < N;
-    double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-    for (int s = 0; s < NS; ++s) {
-      const long long o = slot_off<D, P>(s, M);
-      const double2 a = __ldg(reinterpret_cast<const double2*>(A + (long long)s * Np + i0));
-      const double x0 = __ldg(x + clampi(i0 + o, N));
-      const double x1 = __ldg(x + clampi(i0 + 1 + o, N));
-      s0 = fma(a.x, x0, s0);
-      s1 = fma(a.y, x1, s1);
-    }
-    double y0 = s0, y1 = s1;
-    if (RES) {
-      y0 = b[i0] - s0;
-      if (two) y1 = b[i0 + 1] - s1;
-    }
-    y[i0] = y0;
-    if (two) y[i0 + 1] = y1;
-    if (DOT) {
-      acc = fma(y0, dv[i0], acc);
-      if (two) acc = fma(y1, dv[i0 + 1], acc);
-    }
-  }
-  if (DOT) dr_finish(acc, R, smem);
+  const double bi = RES ? b[bq * Np + i] : 0.0;
+  double dg;
+  const double s = q1_row_sum<D>(A, Np, N, M, x, i, dg);
+  y[i] = RES ? bi - s : s;
+}
+
+// compute-residual fused with the following <jacobi> step on a Q1 level:
+// t = (b - A x)/d, xout = x + w t, r := t
+template <int D>
+__global__ void __launch_bounds__(kRowT, kRowMinBlocks)
+k_row_jacobi_q1(const double* __restrict__ A, int N, long long Np, int M, double damp,
+                const double* __restrict__ omega, const double* __restrict__ x, const double* b,
+                double* __restrict__ xout, double* r, int write_r) {
+  const int i = blockIdx.x * kRowT + threadIdx.x;
+  if (i >= N) return;
+  const long long bq = blockIdx.y;  // problem of a batched level
+  A += bq * St<D, 1>::NS * Np;
+  x += bq * Np;
+  const double bi = b[bq * Np + i], xi = __ldg(x + i), w = omega ? __ldg(omega + bq * Np + i) : damp;
+  double dg;
+  const double s = q1_row_sum<D>(A, Np, N, M, x, i, dg);
+  const double t = (bi - s) / dg;
+  if (write_r) r[bq * Np + i] = t;
+  xout[bq * Np + i] = fma(w, t, xi);
 }
 
 // k_jacobi on a scalar Q2 level (the diagonal sits at the node's colour-major place)
@@ -642,64 +668,6 @@ k_jacobi(const double* __restrict__ Dg, long long N, double damp, const double* 
   if (write_r) r[i] = t;
   const double w = omega ? omega[i] : damp;
   x[i] = fma(w, t, x[i]);
-}
-
-// compute-residual fused with the following <jacobi> step:
-// t = (b - A x)/d, xout = x + w t, r := t; optional fused (xout, dv) reduction
-template <int D, int P, bool DOT>
-__global__ void __launch_bounds__(kBlock)
-k_jacobi_res(const double* __restrict__ A, long long N, long long Np, long long M, double damp,
-             const double* __restrict__ omega, const double* __restrict__ x, const double* b,
-             double* __restrict__ xout, double* r, int write_r, const double* __restrict__ dv,
-             Reduce R) {
-  constexpr int NS = St<D, P>::NS;
-  constexpr int C = St<D, P>::CENTER;
-  __shared__ double smem[8];
-  const long long bq = blockIdx.y;  // problem of a batched level
-  A += bq * NS * Np;
-  x += bq * Np;
-  b += bq * Np;
-  xout += bq * Np;
-  r += bq * Np;
-  if (omega) omega += bq * Np;
-  if (DOT) {
-    dv += bq * Np;
-    R = batch_reduce(R, (unsigned)bq);
-  }
-  const long long base = (long long)blockIdx.x * kChunk + 2 * threadIdx.x;
-  double acc = 0.0;
-#pragma unroll 1
-  for (int m = 0; m < kPairsPerThread; ++m) {
-    const long long i0 = base + 512LL * m;
-    if (i0 >= N) break;
-    const bool two = i0 + 1 < N;
-    double s0 = 0.0, s1 = 0.0, d0 = 1.0, d1 = 1.0;
-#pragma unroll
-    for (int s = 0; s < NS; ++s) {
-      const long long o = slot_off<D, P>(s, M);
-      const double2 a = __ldg(reinterpret_cast<const double2*>(A + (long long)s * Np + i0));
-      if (s == C) { d0 = a.x; d1 = a.y; }
-      const double x0 = __ldg(x + clampi(i0 + o, N));
-      const double x1 = __ldg(x + clampi(i0 + 1 + o, N));
-      s0 = fma(a.x, x0, s0);
-      s1 = fma(a.y, x1, s1);
-    }
-    {
-      const double t = (b[i0] - s0) / d0;
-      if (write_r) r[i0] = t;
-      const double xn = fma(omega ? omega[i0] : damp, t, x[i0]);
-      xout[i0] = xn;
-      if (DOT) acc = fma(xn, dv[i0], acc);
-    }
-    if (two) {
-      const double t = (b[i0 + 1] - s1) / d1;
-      if (write_r) r[i0 + 1] = t;
-      const double xn = fma(omega ? omega[i0 + 1] : damp, t, x[i0 + 1]);
-      xout[i0 + 1] = xn;
-      if (DOT) acc = fma(xn, dv[i0 + 1], acc);
-    }
-  }
-  if (DOT) dr_finish(acc, R, smem);
 }
 
 // one colour of the multicolour <sor> sweep on a Q1 level (P = 1): rows with
@@ -1167,6 +1135,109 @@ __device__ __forceinline__ bool face_dir(int c, int M, int k, int dmask) {
   return (c == 0 && ((dmask >> (2 * k)) & 1)) || (c == M - 1 && ((dmask >> (2 * k + 1)) & 1));
 }
 
+// rc_J = I^T rf at coarse node cJ (constrained).  A z plane's loads (up to 25)
+// are issued before its multiply-adds, which run in z, y, x order; positions
+// outside the level and Dirichlet nodes are skipped.  (3D Q1, 129^3 coarse
+// nodes: 64 us, 138 us with each load waiting for the previous term; one
+// memory wait per plane on small levels, 12.4 -> 6 us at 33^3.)
+template <int D, int P>
+__device__ __forceinline__ double restrict_node(const int cJ[3], int MC, int MF, int dmask,
+                                                const double* __restrict__ rf) {
+#pragma unroll
+  for (int k = 0; k < D; ++k)
+    if (face_dir(cJ[k], MC, k, dmask)) return 0.0;
+  constexpr int R = P == 1 ? 3 : 5;
+  // per direction: fine coordinate and weight of each position, and whether it is met
+  int f[3][R];
+  double w[3][R];
+  bool on[3][R];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    if (k >= D) continue;
+    long long off[5] = {0, 0, 0, 0, 0};
+    double wk[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    const int cnt = restrict_1d<P>(cJ[k], off, wk);
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      f[k][q] = 2 * cJ[k] + (int)off[q];
+      w[k][q] = wk[q];
+      on[k][q] = q < cnt && f[k][q] >= 0 && f[k][q] < MF && !face_dir(f[k][q], MF, k, dmask);
+    }
+  }
+  double acc = 0.0;
+#pragma unroll
+  for (int z = 0; z < (D > 2 ? R : 1); ++z) {
+    double v[R * R];
+#pragma unroll
+    for (int y = 0; y < (D > 1 ? R : 1); ++y)
+#pragma unroll
+      for (int q = 0; q < R; ++q)
+        if (on[0][q] && (D < 2 || on[1][y]) && (D < 3 || on[2][z]))
+          v[y * R + q] = __ldg(rf + f[0][q] + (long long)MF * ((D > 1 ? f[1][y] : 0) +
+                                                               (long long)MF * (D > 2 ? f[2][z] : 0)));
+#pragma unroll
+    for (int y = 0; y < (D > 1 ? R : 1); ++y)
+#pragma unroll
+      for (int q = 0; q < R; ++q)
+        if (on[0][q] && (D < 2 || on[1][y]) && (D < 3 || on[2][z])) {
+          double ww = w[0][q];
+          if (D > 1) ww = ww * w[1][y];
+          if (D > 2) ww = ww * w[2][z];
+          acc = fma(ww, v[y * R + q], acc);
+        }
+  }
+  return acc;
+}
+
+// (I xc) at fine node fi, not a Dirichlet node (constrained); all loads first
+// (3D Q1, 257^3 fine nodes: 197 us, 469 us with a load per term)
+template <int D, int P>
+__device__ __forceinline__ double prolong_node(const int fi[3], int MF, int MC, int dmask,
+                                               const double* __restrict__ xc) {
+  constexpr int R = P == 1 ? 2 : 3;
+  int j[3][R];
+  double w[3][R];
+  bool on[3][R];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    if (k >= D) continue;
+    long long J[3] = {0, 0, 0};
+    double wk[3] = {0.0, 0.0, 0.0};
+    const int cnt = prolong_1d<P>(fi[k], J, wk);
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      j[k][q] = (int)J[q];
+      w[k][q] = wk[q];
+      on[k][q] = q < cnt && !face_dir(j[k][q], MC, k, dmask);
+    }
+  }
+  constexpr int NY = D > 1 ? R : 1, NZ = D > 2 ? R : 1;
+  double v[NZ * NY * R];
+#pragma unroll
+  for (int z = 0; z < NZ; ++z)
+#pragma unroll
+    for (int y = 0; y < NY; ++y)
+#pragma unroll
+      for (int q = 0; q < R; ++q)
+        if (on[0][q] && (D < 2 || on[1][y]) && (D < 3 || on[2][z]))
+          v[(z * NY + y) * R + q] = __ldg(xc + j[0][q] + (long long)MC * ((D > 1 ? j[1][y] : 0) +
+                                                                          (long long)MC * (D > 2 ? j[2][z] : 0)));
+  double acc = 0.0;
+#pragma unroll
+  for (int z = 0; z < NZ; ++z)
+#pragma unroll
+    for (int y = 0; y < NY; ++y)
+#pragma unroll
+      for (int q = 0; q < R; ++q)
+        if (on[0][q] && (D < 2 || on[1][y]) && (D < 3 || on[2][z])) {
+          double ww = w[0][q];
+          if (D > 1) ww = ww * w[1][y];
+          if (D > 2) ww = ww * w[2][z];
+          acc = fma(ww, v[(z * NY + y) * R + q], acc);
+        }
+  return acc;
+}
+
 // rc := I^T rf (constrained), rhs_c := rc, sol_c := 0 (restrict + its :after
 // methods for the correction scheme, multigrid.lisp:202-224)
 template <int D, int P>
@@ -1185,27 +1256,7 @@ k_restrict(int MC, int MF, int dmask, const double* __restrict__ rf, double* __r
                      D > 2 ? (int)blockIdx.z : 0};
   if (cJ[0] >= MC || cJ[1] >= MC) return;
   const long long J = cJ[0] + (long long)MC * (cJ[1] + (long long)MC * cJ[2]);
-  bool dj = false;
-  for (int k = 0; k < D; ++k) dj = dj || face_dir(cJ[k], MC, k, dmask);
-  double acc = 0.0;
-  if (!dj) {
-    long long off[3][5] = {{0}, {0}, {0}};
-    double w[3][5] = {{1.0}, {1.0}, {1.0}};
-    int cnt[3] = {1, 1, 1};
-    for (int k = 0; k < D; ++k) cnt[k] = restrict_1d<P>(cJ[k], off[k], w[k]);
-    for (int z = 0; z < cnt[2]; ++z)
-      for (int y = 0; y < cnt[1]; ++y)
-        for (int xx = 0; xx < cnt[0]; ++xx) {
-          const int fi[3] = {2 * cJ[0] + (int)off[0][xx], 2 * cJ[1] + (int)off[1][y], 2 * cJ[2] + (int)off[2][z]};
-          bool skip = false;
-          for (int k = 0; k < D; ++k) skip = skip || fi[k] < 0 || fi[k] >= MF || face_dir(fi[k], MF, k, dmask);
-          if (skip) continue;
-          double ww = w[0][xx];
-          if (D > 1) ww = ww * w[1][y];
-          if (D > 2) ww = ww * w[2][z];
-          acc = fma(ww, rf[fi[0] + (long long)MF * (fi[1] + (long long)MF * fi[2])], acc);
-        }
-  }
+  const double acc = restrict_node<D, P>(cJ, MC, MF, dmask, rf);
   rc[J] = acc;
   rhsc[J] = acc;
   solc[J] = 0.0;
@@ -1225,27 +1276,12 @@ k_prolong(int MF, int MC, int dmask, const double* __restrict__ xc, double* __re
   const int fi[3] = {(int)(blockIdx.x * 32 + threadIdx.x), D > 1 ? (int)(blockIdx.y * 8 + threadIdx.y) : 0,
                      D > 2 ? (int)blockIdx.z : 0};
   if (fi[0] >= MF || fi[1] >= MF) return;
+#pragma unroll
   for (int k = 0; k < D; ++k)
     if (face_dir(fi[k], MF, k, dmask)) return;
   const long long i = fi[0] + (long long)MF * (fi[1] + (long long)MF * fi[2]);
-  long long J[3][3] = {{0}, {0}, {0}};
-  double w[3][3] = {{1.0}, {1.0}, {1.0}};
-  int cnt[3] = {1, 1, 1};
-  for (int k = 0; k < D; ++k) cnt[k] = prolong_1d<P>(fi[k], J[k], w[k]);
-  double acc = 0.0;
-  for (int z = 0; z < cnt[2]; ++z)
-    for (int y = 0; y < cnt[1]; ++y)
-      for (int xx = 0; xx < cnt[0]; ++xx) {
-        const int cj[3] = {(int)J[0][xx], (int)J[1][y], (int)J[2][z]};
-        bool dj = false;
-        for (int k = 0; k < D; ++k) dj = dj || face_dir(cj[k], MC, k, dmask);
-        if (dj) continue;
-        double ww = w[0][xx];
-        if (D > 1) ww = ww * w[1][y];
-        if (D > 2) ww = ww * w[2][z];
-        acc = fma(ww, xc[cj[0] + (long long)MC * (cj[1] + (long long)MC * cj[2])], acc);
-      }
-  xf[i] = xf[i] + acc;
+  const double xi = xf[i];
+  xf[i] = xi + prolong_node<D, P>(fi, MF, MC, dmask, xc);
 }
 
 // -------------------------------------------------------------- coarse LU
@@ -2466,14 +2502,12 @@ void launch_spmv(const LevelView& L, const double* x, const double* b, double* y
     if (dv) launch_dot(y, dv, L.N, *R, st);
     return;
   }
-  const dim3 g(nchunks(L.N), (unsigned)L.nb);
-  Reduce r0 = R ? *R : Reduce{};
+  const dim3 g(grid1(L.N, kRowT), (unsigned)L.nb);
   Q1_DISPATCH(L.dim, {
-    if (b && dv) k_spmv<D, 1, true, true><<<g, kBlock, 0, st>>>(L.A, L.N, L.Np, L.M, x, b, y, dv, r0);
-    else if (b) k_spmv<D, 1, true, false><<<g, kBlock, 0, st>>>(L.A, L.N, L.Np, L.M, x, b, y, dv, r0);
-    else if (dv) k_spmv<D, 1, false, true><<<g, kBlock, 0, st>>>(L.A, L.N, L.Np, L.M, x, b, y, dv, r0);
-    else k_spmv<D, 1, false, false><<<g, kBlock, 0, st>>>(L.A, L.N, L.Np, L.M, x, b, y, dv, r0);
+    if (b) k_row_q1<D, true><<<g, kRowT, 0, st>>>(L.A, (int)L.N, L.Np, (int)L.M, x, b, y);
+    else k_row_q1<D, false><<<g, kRowT, 0, st>>>(L.A, (int)L.N, L.Np, (int)L.M, x, b, y);
   });
+  if (dv) launch_dot_b(y, dv, L.N, L.Np, L.nb, *R, st);
 }
 
 void launch_jacobi(const LevelView& L, double damp, double* x, double* r, bool write_r, cudaStream_t st) {
@@ -2528,14 +2562,12 @@ void launch_jacobi_res(const LevelView& L, double damp, const double* x, const d
     if (dv) launch_dot(xout, dv, L.N, *R, st);
     return;
   }
-  const dim3 g(nchunks(L.N), (unsigned)L.nb);
-  Reduce r0 = R ? *R : Reduce{};
+  const dim3 g(grid1(L.N, kRowT), (unsigned)L.nb);
   Q1_DISPATCH(L.dim, {
-    if (dv) k_jacobi_res<D, 1, true><<<g, kBlock, 0, st>>>(L.A, L.N, L.Np, L.M, damp, L.omega, x, b, xout, r,
-                                                             write_r ? 1 : 0, dv, r0);
-    else k_jacobi_res<D, 1, false><<<g, kBlock, 0, st>>>(L.A, L.N, L.Np, L.M, damp, L.omega, x, b, xout, r,
-                                                         write_r ? 1 : 0, dv, r0);
+    k_row_jacobi_q1<D><<<g, kRowT, 0, st>>>(L.A, (int)L.N, L.Np, (int)L.M, damp, L.omega, x, b, xout, r,
+                                            write_r ? 1 : 0);
   });
+  if (dv) launch_dot_b(xout, dv, L.N, L.Np, L.nb, *R, st);
 }
 
 static void launch_csr_sor(const LevelView& L, double omega, const double* om, double* x, const double* b, double* r,
