@@ -8,6 +8,8 @@
 // Entries outside the grid, in eliminated Dirichlet columns and structurally
 // absent Q2 couplings are stored as zeros, which lets neighbour indices be
 // clamped to the vector instead of tested.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cstring>
 #include <type_traits>
@@ -31,6 +33,38 @@ struct St {
   static constexpr int NS = D == 1 ? W : (D == 2 ? W * W : W * W * W);
   static constexpr int CENTER = (NS - 1) / 2;
 };
+
+// Programmatic dependent launch: a kernel launched with launch_pdl may start
+// while its predecessor in the stream still runs.  pdl_next lets the
+// successor start; pdl_wait waits until the predecessor has finished and its
+// writes are visible, and comes before the first access to anything that a
+// kernel of the same sequence writes.
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// launches kern after the stream's previous kernel, overlapping its start
+// with that kernel's end when early (kern must call pdl_wait)
+template <typename... KA, typename... A>
+static void launch_pdl(bool early, void (*kern)(KA...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
+                       A... args) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = early ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...);
+}
+
+// copies 8 bytes to shared memory in the background
+__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
 
 template <int D, int P>
 __device__ __forceinline__ long long slot_off(int s, long long M) {
@@ -147,10 +181,13 @@ __device__ __forceinline__ void q2_row(const long long c[3], long long M, F&& f)
 // direction the class's coordinates are d, d+3, d+6, .. (d = coordinate mod 3),
 // or, where the slot restricts the direction to even coordinates, x0(d),
 // x0(d)+6, .. with x0 = 0, 4, 2 for d = 0, 1, 2.  A colour sweep then streams
-// one contiguous block of every slot array.  off[r][colour] is where the
+// one contiguous block of every slot array.  off[colour][r] is where the
 // class's block starts in the arrays of pattern-r slots.
+// (Levels have fewer than 2^31 nodes.  A class's eight offsets sit together:
+// a kernel reads them from its parameters, and each line of those it touches
+// is a miss at the start of every launch.)
 struct Q2Layout {
-  long long off[8][27];
+  int off[27][8];
 };
 
 __host__ __device__ __forceinline__ int q2c_x0(int d) { return d == 0 ? 0 : (d == 1 ? 4 : 2); }
@@ -172,7 +209,7 @@ Q2Layout q2_layout(int D, long long M) {
   for (int r = 0; r < (1 << D); ++r) {
     long long acc = 0;
     for (int col = 0; col < ncol; ++col) {
-      L.off[r][col] = acc;
+      L.off[col][r] = (int)acc;
       long long cnt = 1;
       int t = col;
       for (int k = 0; k < D; ++k) {
@@ -199,7 +236,7 @@ __host__ __device__ __forceinline__ long long q2c_pos(const Q2Layout& L, const l
     p += q2c_j(c[k], d, rk) * mul;
     mul *= q2c_ext(M, d, rk);
   }
-  return L.off[r][col] + p;
+  return L.off[col][r] + p;
 }
 
 // q2_row for the colour-major layout of scalar Q2 levels
@@ -227,8 +264,8 @@ __device__ __forceinline__ void q2c_row(const Q2Layout& L, const long long c[3],
       const int ry = (oy == 2 || oy == -2) ? 1 : 0;
       if (ry && !ev[1]) continue;
       const long long yz = j[1][ry] + e[1][ry] * j[2][rz];
-      const long long b0 = L.off[(ry << 1) | (rz << 2)][col] + j[0][0] + e[0][0] * yz;
-      const long long b1 = L.off[1 | (ry << 1) | (rz << 2)][col] + j[0][1] + e[0][1] * yz;
+      const long long b0 = L.off[col][(ry << 1) | (rz << 2)] + j[0][0] + e[0][0] * yz;
+      const long long b1 = L.off[col][1 | (ry << 1) | (rz << 2)] + j[0][1] + e[0][1] * yz;
       const long long obase = (long long)oy * M + (long long)oz * M * M;
 #pragma unroll
       for (int sx = 0; sx < 5; ++sx) {
@@ -289,7 +326,7 @@ __device__ __forceinline__ void q2_base(const Q2Layout& lay, const long long c[3
     if (!(r & odd)) b.valid |= 1u << r;
     const int rx = r & 1, ry = (r >> 1) & 1, rz = (r >> 2) & 1;
     const int p = j[0][rx] + e[0][rx] * (j[1][ry] + e[1][ry] * j[2][rz]);
-    const int q = COLOUR ? (int)lay.off[r][col] + p : p;
+    const int q = COLOUR ? lay.off[col][r] + p : p;
     b.p[r] = (CLAMP && q >= nmax) ? nmax - 1 : q;
   }
 }
@@ -431,25 +468,33 @@ template <int D>
 constexpr int kQ2MinBlocks = D == 3 ? 4 : 1;
 
 struct Q2Sub {
-  int d[3], j0[3], n[3];  // class digit, first place and row count along each direction
-  long long cnt;          // rows of the (class, parity) subgrid
+  int d[3], j0[3], st[3], n[3];  // class digit, first place, step and row count along each direction
+  long long cnt;                 // rows of the (class, parity) subgrid
 };
 
+// ssc >= 0: only the rows that belong to vertex blocks of that colour of the
+// <geometric-ssc> sweep -- every odd coordinate, and the even ones that are
+// vertices of the colour (coordinate = 2 bit mod 4)
 template <int D>
-__host__ __device__ __forceinline__ void q2_sub(int M, int colour, int pat, Q2Sub& s) {
+__host__ __device__ __forceinline__ void q2_sub(int M, int colour, int pat, Q2Sub& s, int ssc = -1) {
   s.cnt = 1;
   int t = colour;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     if (k < D) {
-      const int d = t % 3, nk = (M - d + 2) / 3, j0 = (((pat >> k) & 1) + d) & 1;
+      const int d = t % 3, nk = (M - d + 2) / 3;
+      const bool quarter = ssc >= 0 && !((pat >> k) & 1);
+      const int j0 = quarter ? ((2 * ((ssc >> k) & 1) - d) * 3) & 3 : (((pat >> k) & 1) + d) & 1;
+      const int st = quarter ? 4 : 2;
       t /= 3;
       s.d[k] = d;
       s.j0[k] = j0;
-      s.n[k] = nk > j0 ? (nk - j0 + 1) / 2 : 0;
+      s.st[k] = st;
+      s.n[k] = nk > j0 ? (nk - j0 + st - 1) / st : 0;
     } else {
       s.d[k] = 0;
       s.j0[k] = 0;
+      s.st[k] = 2;
       s.n[k] = 1;
     }
     s.cnt *= s.n[k];
@@ -458,11 +503,11 @@ __host__ __device__ __forceinline__ void q2_sub(int M, int colour, int pat, Q2Su
 
 // blocks a class takes: its parity subgrids one after another
 template <int D>
-__host__ __device__ __forceinline__ long long q2_class_blocks(int M, int colour) {
+__host__ __device__ __forceinline__ long long q2_class_blocks(int M, int colour, int ssc = -1) {
   long long nb = 0;
   for (int pat = 0; pat < (1 << D); ++pat) {
     Q2Sub s;
-    q2_sub<D>(M, colour, pat, s);
+    q2_sub<D>(M, colour, pat, s, ssc);
     nb += (s.cnt + kQ2T - 1) / kQ2T;
   }
   return nb;
@@ -471,9 +516,10 @@ __host__ __device__ __forceinline__ long long q2_class_blocks(int M, int colour)
 // block blk of a class: its parity pattern, subgrid and this thread's row u
 // in it; false when the thread has no row
 template <int D>
-__device__ __forceinline__ bool q2_block(int M, int colour, long long blk, int& pat, Q2Sub& s, long long& u) {
+__device__ __forceinline__ bool q2_block(int M, int colour, long long blk, int& pat, Q2Sub& s, long long& u,
+                                         int ssc = -1) {
   for (pat = 0; pat < (1 << D); ++pat) {
-    q2_sub<D>(M, colour, pat, s);
+    q2_sub<D>(M, colour, pat, s, ssc);
     const long long nb = (s.cnt + kQ2T - 1) / kQ2T;
     if (blk < nb) {
       u = blk * kQ2T + threadIdx.x;
@@ -497,7 +543,7 @@ __device__ __forceinline__ long long q2_place(const Q2Layout& lay, int M, int co
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     if (k < D) {
-      const int jj = s.j0[k] + 2 * uk[k], d = s.d[k], x0 = q2c_x0(d);
+      const int jj = s.j0[k] + s.st[k] * uk[k], d = s.d[k], x0 = q2c_x0(d);
       c[k] = d + 3 * jj;
       j[k][0] = jj;
       e[k][0] = (M - d + 2) / 3;
@@ -512,7 +558,7 @@ __device__ __forceinline__ long long q2_place(const Q2Layout& lay, int M, int co
 #pragma unroll
   for (int r = 0; r < (1 << D); ++r) {
     const int rx = r & 1, ry = (r >> 1) & 1, rz = (r >> 2) & 1;
-    p[r] = (int)lay.off[r][colour] + j[0][rx] + e[0][rx] * (j[1][ry] + e[1][ry] * j[2][rz]);
+    p[r] = lay.off[colour][r] + j[0][rx] + e[0][rx] * (j[1][ry] + e[1][ry] * j[2][rz]);
   }
   return (long long)c[0] + (long long)M * (c[1] + (long long)M * c[2]);
 }
@@ -579,6 +625,173 @@ __device__ __forceinline__ void q2_pat_dispatch(int pat, F&& f) {
     case 6: if constexpr (D > 2) f(std::integral_constant<int, 6>{}); break;
     default: if constexpr (D > 2) f(std::integral_constant<int, 7>{}); break;
   }
+}
+
+// whether a node lies on a Dirichlet face
+__device__ __forceinline__ bool q2_face(const int c[3], int M, int dmask) {
+  bool on = false;
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    on = on || (c[k] == 0 && ((dmask >> (2 * k)) & 1)) || (c[k] == M - 1 && ((dmask >> (2 * k + 1)) & 1));
+  return on;
+}
+
+// One colour of the multicolour <sor> sweep of a 3D scalar Q2 level of few
+// rows: a tile of 32 rows of one class and parity per block.  A row's sum is
+// one chain of up to 125 fma in slot order (10 cycles each); a thread that
+// also loads its row waits for memory ten times, as its registers hold half a
+// stencil plane, and its unrolled code takes longer to fetch than to run.
+// Here warp w loads the coefficients and unknowns of the (y, z) slot rows
+// 3 w .. 3 w + 2 (the last warp four) of all 32 rows, up to 20 of each at
+// once, into shared memory -- the row's stored slots one after another -- and
+// one warp runs the 32 chains from there.  The colours of a sweep overlap:
+// indices, coefficients, diagonal and damping are fetched while the previous
+// colour still runs, only the unknowns wait for it.
+constexpr int kTileRows = 32, kTileT = 256;
+constexpr size_t kTileSmem = 2 * 125 * kTileRows * sizeof(double);
+// rows of a colour up to which a level takes this form; beyond, the strided
+// reads of x bound it and a thread per row is faster
+constexpr long long kTileMax = 12000;
+#ifndef SSCT
+#define SSCT 100000
+#endif
+constexpr long long kSscTileMax = SSCT;
+
+// SSC: the residuals r = b - A x of the rows of one <geometric-ssc> colour
+// instead (every class, blockIdx.z; b may be r): see k_ssc_solve_q2.
+template <bool SSC>
+__global__ void __launch_bounds__(kTileT, 3)
+k_q2_tile(const double* __restrict__ A, long long Np, int M, int col, int dmask, double damp,
+          const double* __restrict__ omega, double* x, const double* b, double* r,
+          const __grid_constant__ Q2Layout lay) {
+  extern __shared__ double tsm[];
+  pdl_next();
+  const int pat = (int)blockIdx.y, colour = SSC ? (int)blockIdx.z : col;
+  Q2Sub sub;
+  q2_sub<3>(M, colour, pat, sub, SSC ? col : -1);
+  const int u0 = blockIdx.x * kTileRows;
+  if (u0 >= sub.cnt) {
+    pdl_wait();
+    return;
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool live = u0 + lane < sub.cnt;
+  const unsigned u = live ? u0 + lane : (unsigned)sub.cnt - 1;  // spare lanes repeat the last row and store nothing
+  const unsigned q0 = u / (unsigned)sub.n[0];
+  const int uk[3] = {(int)(u - q0 * (unsigned)sub.n[0]), (int)(q0 % (unsigned)sub.n[1]),
+                     (int)(q0 / (unsigned)sub.n[1])};
+  int c[3], j[3][2], e[3][2];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int jj = sub.j0[k] + sub.st[k] * uk[k], d = sub.d[k], x0 = q2c_x0(d);
+    c[k] = d + 3 * jj;
+    j[k][0] = jj;
+    e[k][0] = (M - d + 2) / 3;
+    j[k][1] = (c[k] - x0) / 6;
+    e[k][1] = x0 < M ? (M - x0 + 5) / 6 : 0;
+  }
+  // stored slots per direction (5 or 3) and the first of them
+  const int ox = pat & 1, oy = (pat >> 1) & 1, oz = pat >> 2;
+  const int nx = 5 - 2 * ox, ny = 5 - 2 * oy, nv = nx * ny * (5 - 2 * oz);
+  double* sa = tsm + lane;                    // [stored slot][row] coefficients
+  double* sx = tsm + 125 * kTileRows + lane;  // [stored slot][row] unknowns
+  double v[4][5];
+  bool on[4];
+  int at[4];
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    const int yz = 3 * warp + t, sz = yz / 5, sy = yz - 5 * sz;
+    const bool ry = sy == 0 || sy == 4, rz = sz == 0 || sz == 4;
+    on[t] = (t < 3 || warp == 7) && !(ry && oy) && !(rz && oz);
+    at[t] = ((sz - oz) * ny + sy - oy) * nx - ox;  // where the slot row starts, less its skipped slot
+    if (!on[t]) continue;
+    const int pl = (ry ? j[1][1] : j[1][0]) + (ry ? e[1][1] : e[1][0]) * (rz ? j[2][1] : j[2][0]);
+    const int rr = (ry ? 2 : 0) | (rz ? 4 : 0);
+    const double* a = A + (long long)(5 * yz) * Np;
+    const double* a1 = a + lay.off[colour][rr | 1] + j[0][1] + e[0][1] * pl;
+    a += lay.off[colour][rr] + j[0][0] + e[0][0] * pl;
+    if (!ox) v[t][0] = __ldcg(a1);
+#pragma unroll
+    for (int q = 1; q < 4; ++q) v[t][q] = __ldcg(a + (long long)q * Np);
+    if (!ox) v[t][4] = __ldcg(a1 + 4 * Np);
+  }
+  const long long i = (long long)c[0] + (long long)M * (c[1] + (long long)M * c[2]);
+  double d = 1.0, bi = 0.0, xi = 0.0, w = damp;
+  if (!SSC && warp == 0) {
+    d = __ldcg(A + 62LL * Np + lay.off[colour][0] + j[0][0] + e[0][0] * (j[1][0] + e[1][0] * j[2][0]));
+    if (omega) w = __ldcg(omega + i);
+  }
+#pragma unroll
+  for (int t = 0; t < 4; ++t)
+    if (on[t]) {
+#pragma unroll
+      for (int q = 0; q < 5; ++q)
+        if (!(q == 0 || q == 4) || !ox) sa[(at[t] + q) * kTileRows] = v[t][q];
+    }
+  pdl_wait();
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    if (!on[t]) continue;
+    const int yz = 3 * warp + t, sz = yz / 5, sy = yz - 5 * sz;
+    const double* xl = x + (long long)M * (min(max(c[1] + sy - 2, 0), M - 1) +
+                                           (long long)M * min(max(c[2] + sz - 2, 0), M - 1));
+#pragma unroll
+    for (int q = 0; q < 5; ++q)  // outside the grid the coefficient is a stored zero
+      if (!(q == 0 || q == 4) || !ox) v[t][q] = xl[min(max(c[0] + q - 2, 0), M - 1)];
+  }
+  if (warp == 0) {
+    if (!SSC) xi = x[i];
+    bi = b[i];
+  }
+#pragma unroll
+  for (int t = 0; t < 4; ++t)
+    if (on[t]) {
+#pragma unroll
+      for (int q = 0; q < 5; ++q)
+        if (!(q == 0 || q == 4) || !ox) sx[(at[t] + q) * kTileRows] = v[t][q];
+    }
+  __syncthreads();
+  if (warp) return;
+  double s = 0.0;
+  // nine terms at a time (27, 45 or 75 + 6, 125 + 1: the last ones guarded)
+  int q0v = 0;
+#pragma unroll 1
+  for (; q0v + 9 <= nv; q0v += 9) {
+    double ta[9], tx[9];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) { ta[q] = sa[(q0v + q) * kTileRows]; tx[q] = sx[(q0v + q) * kTileRows]; }
+#pragma unroll
+    for (int q = 0; q < 9; ++q) s = fma(ta[q], tx[q], s);
+  }
+  for (; q0v < nv; ++q0v) s = fma(sa[q0v * kTileRows], sx[q0v * kTileRows], s);
+  if (!live) return;
+  if (SSC) {
+    if (pat == 0 || !q2_face(c, M, dmask)) r[i] = bi - s;
+    return;
+  }
+  const double t = (bi - s) / d;
+  r[i] = t;
+  x[i] = fma(w, t, xi);
+}
+
+// colour `col` by tiles: blockIdx.x the tiles of the largest parity subgrid,
+// .y the parity, .z the class (SSC).  early: the launches of a sweep after the
+// first start early -- the coefficients, diagonal and damping were in place
+// before the sweep began.
+template <bool SSC>
+static void launch_q2_tile(const LevelView& L, int col, bool early, double damp, double* x, const double* b, double* r,
+                           const Q2Layout& lay, cudaStream_t st) {
+  const int M = (int)L.M;
+  long long most = 1;
+  for (int cls = SSC ? 0 : col; cls < (SSC ? 27 : col + 1); ++cls)
+    for (int pat = 0; pat < 8; ++pat) {
+      Q2Sub s;
+      q2_sub<3>(M, cls, pat, s, SSC ? col : -1);
+      most = std::max(most, s.cnt);
+    }
+  if (!early) cudaFuncSetAttribute(k_q2_tile<SSC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmem);
+  launch_pdl(early, k_q2_tile<SSC>, dim3((unsigned)((most + kTileRows - 1) / kTileRows), 8, SSC ? 27 : 1), kTileT,
+             kTileSmem, st, L.A, L.Np, M, col, L.dmask, damp, L.omega, x, b, r, lay);
 }
 
 // the rows of block blk of colour class `colour` in the multicolour <sor>
@@ -740,34 +953,74 @@ __device__ __forceinline__ void ssc_lu_step(double (&a)[NB], int& pos, int lane)
   }
 }
 
-// Column K of the forward substitution with the stored unit lower factor:
-// the row at position K is final, the rows below subtract their multiplier
-// times it (the operations, in order, of carrying the right-hand side
-// through the elimination).
-template <int NB, int K>
-__device__ __forceinline__ void ssc_fwd_step(const double (&a)[NB], double& rr, int pos, int lane) {
-  if constexpr (K < NB) {
-    constexpr unsigned FULL = 0xffffffffu;
-    const unsigned who = __ballot_sync(FULL, lane < NB && pos == K);
-    const double rk = __shfl_sync(FULL, rr, __ffs(who) - 1);
-    if (lane < NB && pos > K) rr = rr - a[K] * rk;
-    ssc_fwd_step<NB, K + 1>(a, rr, pos, lane);
-  }
+// a / u rounded to nearest, given y = 1 / u rounded to nearest: two residual
+// corrections of a y (Markstein, IBM J. Res. Dev. 34, 1990: with y correctly
+// rounded and q within an ulp, q + (a - q u) y rounds to the quotient).  Holds
+// while the residuals are exact, i.e. away from the ends of the exponent
+// range (div_by_ok).  50 cycles in the chain of a substitution instead of the
+// division's 137.
+__device__ __forceinline__ double div_by(double a, double u, double y) {
+  double q = a * y;
+  q = fma(fma(-u, q, a), y, q);
+  return fma(fma(-u, q, a), y, q);
+}
+__device__ __forceinline__ bool div_by_ok(double a, double u, double q) {
+  auto mid = [](double v) { return (((unsigned)__double2hiint(v) >> 20) & 0x7ff) - 300u < 1400u; };
+  return a == 0.0 || (mid(a) && mid(u) && mid(q));
 }
 
-// Column K of the backward substitution: the lane at position K divides,
-// the rows above subtract; the lane of member K keeps the solution.
-template <int NB, int K>
-__device__ __forceinline__ void ssc_back_step(const double (&a)[NB], double& rr, int pos, int lane, double& corr) {
-  if constexpr (K >= 0) {
-    constexpr unsigned FULL = 0xffffffffu;
-    const unsigned who = __ballot_sync(FULL, lane < NB && pos == K);
-    const int kl = __ffs(who) - 1;
-    const double xk = __shfl_sync(FULL, rr / a[K], kl);
-    if (lane < NB && pos < K) rr = rr - xk * a[K];
-    if (lane == K) corr = xk;
-    ssc_back_step<NB, K - 1>(a, rr, pos, lane, corr);
+// A_BB c = r_B of a vertex block with its stored factors: lane t brings member
+// t's residual and gets member t's correction.  f: the factors in shared
+// memory, [column][position]; the rows sit in lanes by their final position,
+// mem is the member of lane's row, u and y its pivot and the pivot's
+// reciprocal.  Forward: the row at position K is final, the rows below
+// subtract their multiplier times it (the operations, in order, of carrying
+// the right-hand side through the elimination).  Backward: the row at
+// position K divides, the rows above subtract; lane K keeps the solution of
+// member K.  The columns run in loops: unrolled, with the factors in
+// registers, the code took longer to fetch than to run.
+template <int NB>
+__device__ __forceinline__ double ssc_block_solve(const double* f, int mem, double u, double y, double rr, int lane) {
+  constexpr unsigned FULL = 0xffffffffu;
+  rr = __shfl_sync(FULL, rr, mem);
+  const int t = lane < NB ? lane : NB - 1;
+#pragma unroll 3
+  for (int K = 0; K < NB; ++K) {
+    const double fk = f[K * NB + t], rk = __shfl_sync(FULL, rr, K);
+    if (lane > K) rr = rr - fk * rk;
   }
+  const double rf = rr;
+  double corr = 0.0;
+#pragma unroll 3
+  for (int K = NB - 1; K >= 0; --K) {
+    const double fk = f[K * NB + t], q = div_by(rr, u, y), xk = __shfl_sync(FULL, q, K);
+    if (lane == K) corr = q;
+    if (lane < K) rr = rr - xk * fk;
+  }
+  // lane K's rr is the numerator of its quotient
+  if (__any_sync(FULL, lane < NB && !div_by_ok(rr, u, corr))) {
+    rr = rf;
+#pragma unroll 1
+    for (int K = NB - 1; K >= 0; --K) {
+      const double fk = f[K * NB + t];
+      if (lane == K) corr = rr / u;
+      const double xk = __shfl_sync(FULL, corr, K);
+      if (lane < K) rr = rr - xk * fk;
+    }
+  }
+  return corr;
+}
+
+// copies a block's factors to shared memory, every load before the first store
+template <int NB>
+__device__ __forceinline__ void ssc_stage(const double* __restrict__ F, double* f, int lane) {
+  constexpr int PER = (NB * NB + 31) / 32;
+  double v[PER];
+#pragma unroll
+  for (int q = 0; q < PER; ++q) v[q] = q * 32 + lane < NB * NB ? __ldcg(F + q * 32 + lane) : 0.0;
+#pragma unroll
+  for (int q = 0; q < PER; ++q)
+    if (q * 32 + lane < NB * NB) f[q * 32 + lane] = v[q];
 }
 
 // Member `lane` of the vertex block of vertex v (2 x vertex index): its node
@@ -806,8 +1059,9 @@ __device__ __forceinline__ SscMember<D> ssc_member(const int v[3], int lane, int
 // the arithmetic of the real rows are those of the compact block), then
 // factored as by gesv! (right-looking, partial pivoting).  The factors depend
 // on the matrix only, so a sweep that reuses them repeats exactly the
-// operations of factoring afresh.  Layout: F[block][k][member], the row's
-// final position in P[block][member]; block = lexicographic vertex index.
+// operations of factoring afresh.  Layout: F[block][k][position], the member
+// whose row ended there in P[block][position]; block = lexicographic vertex
+// index.
 template <int D>
 __global__ void __launch_bounds__(128)
 k_ssc_factor_q2(const double* __restrict__ A, long long Np, long long M, int dmask, double* F, unsigned char* P,
@@ -849,85 +1103,78 @@ k_ssc_factor_q2(const double* __restrict__ A, long long Np, long long M, int dma
   int pos = lane;  // lanes >= NB are never candidates
   ssc_lu_step<NB, 0>(a, pos, lane);
   if (lane < NB) {
-    double* f = F + w * NB * NB + lane;
+    double* f = F + w * NB * NB + pos;
 #pragma unroll
     for (int k = 0; k < NB; ++k) f[k * NB] = a[k];
-    P[w * NB + lane] = (unsigned char)pos;
+    P[w * NB + pos] = (unsigned char)lane;
   }
 }
 
 // One colour of the <geometric-ssc> sweep on a scalar Q2 level
-// (blockit.lisp:118-204 with the vertex-centred blocks of geoblock.lisp:72-158):
-// a warp per vertex block, lane t holding member t of the 3^D box around the
-// vertex (x fastest).  Each member lane forms its row's residual r = b - A x
-// (b may alias r: the alias inside <cg>), then the warp solves A_BB c = r_B
-// with the stored factors (forward in position order, backward column by
-// column) and x_B += omega c.  Blocks of one colour (vertex index mod 2 per
-// direction) share no node and read no unknown another one writes.
+// (blockit.lisp:118-204 with the vertex-centred blocks of geoblock.lisp:72-158)
+// runs in two launches: the residuals r = b - A x (b may alias r: the alias
+// inside <cg>) of the rows of the colour's blocks, in class order as the
+// other row kernels, then a warp per block that solves A_BB c = r_B with the
+// stored factors (forward in position order, backward column by column) and
+// adds x_B += omega c.  Blocks of one colour (vertex index mod 2 per
+// direction) share no node and read no unknown another one writes, so the
+// residuals are those each block would form for itself.  Formed by the block's
+// own lanes, 27 rows of a warp scattered over the classes' arrays, they took
+// most of the colour's time: 65^3 nodes 107 us a colour, SSC65 us so; 17^3
+// 28 us, SSC17 us.
+// A Dirichlet node belongs to no block but its own.
 template <int D>
-__global__ void __launch_bounds__(128, 6)
-k_ssc_q2(const double* __restrict__ A, long long N, long long Np, long long M, int dmask, int colour,
-         double omega, double* x, const double* b, double* r, const double* __restrict__ F,
-         const unsigned char* __restrict__ P, const __grid_constant__ Q2Layout lay) {
+__global__ void __launch_bounds__(kQ2T, kQ2MinBlocks<D>)
+k_ssc_res_q2(const double* __restrict__ A, long long Np, int M, int ssc, int dmask, const double* x, const double* b,
+             double* r, const __grid_constant__ Q2Layout lay) {
+  pdl_next();
+  int pat;
+  Q2Sub sub;
+  long long u;
+  const int colour = (int)blockIdx.y;
+  const bool row = q2_block<D>(M, colour, blockIdx.x, pat, sub, u, ssc);
+  pdl_wait();
+  if (!row) return;
+  int c[3], p[1 << D];
+  const long long i = q2_place<D>(lay, M, colour, sub, u, c, p);
+  const double bi = b[i];
+  double s = 0.0;
+  q2_pat_dispatch<D>(pat, [&](auto P) { s = q2_row_sum<D, decltype(P)::value, 0>(A, Np, x, M, c, p); });
+  if (pat == 0 || !q2_face(c, M, dmask)) r[i] = bi - s;
+}
+
+template <int D>
+__global__ void __launch_bounds__(128, 7)
+k_ssc_solve_q2(int Mi, int dmask, int colour, double omega, double* x, const double* r, const double* __restrict__ F,
+               const unsigned char* __restrict__ P) {
   constexpr int NB = D == 1 ? 3 : (D == 2 ? 9 : 27);
+  __shared__ double fs_all[4][NB * NB];
+  pdl_next();
   const int lane = threadIdx.x & 31;
-  const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // uniform per warp
-  const int Mi = (int)M;
+  const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);  // uniform per warp
   const int nv = (Mi + 1) / 2;  // vertices per direction
   const int bx = colour & 1, by = (colour >> 1) & 1, bz = (colour >> 2) & 1;
   const int ex = (nv - bx + 1) / 2, ey = D > 1 ? (nv - by + 1) / 2 : 1, ez = D > 2 ? (nv - bz + 1) / 2 : 1;
-  if (w >= (long long)ex * ey * ez) return;  // the whole warp leaves together
-  const int wi = (int)w;
-  const int jx = wi % ex, jq = wi / ex, jy = jq % ey, jz = jq / ey;
+  if (w >= ex * ey * ez) {  // the whole warp leaves together
+    pdl_wait();
+    return;
+  }
+  const int jx = w % ex, jq = w / ex, jy = jq % ey, jz = jq / ey;
   const int ax = bx + 2 * jx, ay = D > 1 ? by + 2 * jy : 0, az = D > 2 ? bz + 2 * jz : 0;
   const int v[3] = {2 * ax, 2 * ay, 2 * az};
   const long long blk = ax + (long long)nv * (ay + (long long)nv * az);
+  // the factors do not depend on the previous launch
+  double* fs = fs_all[threadIdx.x >> 5];
+  ssc_stage<NB>(F + blk * NB * NB, fs, lane);
+  const int mem = lane < NB ? P[blk * NB + lane] : lane;
   const SscMember<D> mb = ssc_member<D>(v, lane, Mi, dmask);
-  // the unknowns the block's rows read: the 7^D nodes within 3 of the
-  // vertex, staged in shared memory (0 outside the domain, where the rows'
-  // stored coefficients are 0 as well)
-  constexpr int W7 = D == 1 ? 7 : (D == 2 ? 49 : 343);
-  __shared__ double xs_all[4][W7];
-  double* xs = xs_all[threadIdx.x >> 5];
-  for (int e = lane; e < W7; e += 32) {
-    const int lx = e % 7, ly = (e / 7) % 7, lz = e / 49;
-    const int gx = v[0] + lx - 3, gy = D > 1 ? v[1] + ly - 3 : 0, gz = D > 2 ? v[2] + lz - 3 : 0;
-    const bool inside = gx >= 0 && gx < Mi && (D < 2 || (gy >= 0 && gy < Mi)) && (D < 3 || (gz >= 0 && gz < Mi));
-    xs[e] = inside ? x[gx + M * ((long long)gy + M * (long long)gz)] : 0.0;
-  }
+  const long long i = mb.real ? (long long)mb.c[0] + Mi * ((long long)mb.c[1] + Mi * (long long)mb.c[2]) : 0;
   __syncwarp();
-  const long long i = mb.real ? (long long)mb.c[0] + M * ((long long)mb.c[1] + M * (long long)mb.c[2]) : 0;
-  double rr = 0.0;
-  if (mb.real) {
-    const long long cl[3] = {mb.c[0], mb.c[1], mb.c[2]};
-    Q2Base<D> qb;
-    q2_base<D, true, true>(lay, cl, M, qb);
-    const int lc = (mb.dm[0] + 3) + 7 * (D > 1 ? mb.dm[1] + 3 : 0) + 49 * (D > 2 ? mb.dm[2] + 3 : 0);
-    double s = 0.0;
-    q2_visit<D, true>(qb, M, [&](int k, long long, long long p, bool st) {
-      double av = A[(long long)k * Np + p];
-      av = st ? av : 0.0;
-      const int lo = (k % 5 - 2) + (D > 1 ? 7 * ((k / 5) % 5 - 2) : 0) + (D > 2 ? 49 * (k / 25 - 2) : 0);
-      s = fma(av, xs[lc + lo], s);
-    });
-    rr = b[i] - s;
-    r[i] = rr;
-  }
-  double a[NB];
-  int pos = lane;
-  if (lane < NB) {
-    const double* f = F + blk * NB * NB + lane;
-#pragma unroll
-    for (int k = 0; k < NB; ++k) a[k] = __ldg(f + k * NB);
-    pos = P[blk * NB + lane];
-  } else {
-#pragma unroll
-    for (int k = 0; k < NB; ++k) a[k] = 0.0;
-  }
-  ssc_fwd_step<NB, 0>(a, rr, pos, lane);
-  double corr = 0.0;
-  ssc_back_step<NB, NB - 1>(a, rr, pos, lane, corr);
-  if (mb.real) x[i] = fma(omega, corr, x[i]);
+  const double u = lane < NB ? fs[lane * NB + lane] : 1.0, y = 1.0 / u;
+  pdl_wait();
+  const double rr = mb.real ? r[i] : 0.0, xi = mb.real ? x[i] : 0.0;
+  const double corr = ssc_block_solve<NB>(fs, mem, u, y, rr, lane);
+  if (mb.real) x[i] = fma(omega, corr, xi);
 }
 
 // <geometric-psc> on a scalar Q1 level: one-node blocks, x_i += damp r_i /
@@ -959,21 +1206,14 @@ k_psc_block_q2(long long M, int dmask, const double* __restrict__ r, const doubl
   const int wi = (int)w;
   const int v[3] = {2 * (wi % nv), D > 1 ? 2 * ((wi / nv) % nv) : 0, D > 2 ? 2 * (wi / (nv * nv)) : 0};
   const SscMember<D> mb = ssc_member<D>(v, lane, Mi, dmask);
+  __shared__ double fs_all[4][NB * NB];
+  double* fs = fs_all[threadIdx.x >> 5];
+  ssc_stage<NB>(F + w * NB * NB, fs, lane);
+  const int mem = lane < NB ? P[w * NB + lane] : lane;
+  __syncwarp();
+  const double u = lane < NB ? fs[lane * NB + lane] : 1.0, y = 1.0 / u;
   double rr = mb.real ? r[(long long)mb.c[0] + M * ((long long)mb.c[1] + M * (long long)mb.c[2])] : 0.0;
-  double a[NB];
-  int pos = lane;
-  if (lane < NB) {
-    const double* f = F + w * NB * NB + lane;
-#pragma unroll
-    for (int k = 0; k < NB; ++k) a[k] = __ldg(f + k * NB);
-    pos = P[w * NB + lane];
-  } else {
-#pragma unroll
-    for (int k = 0; k < NB; ++k) a[k] = 0.0;
-  }
-  ssc_fwd_step<NB, 0>(a, rr, pos, lane);
-  double corr = 0.0;
-  ssc_back_step<NB, NB - 1>(a, rr, pos, lane, corr);
+  const double corr = ssc_block_solve<NB>(fs, mem, u, y, rr, lane);
   if (lane < NB) C[w * NB + lane] = corr;
 }
 
@@ -1528,49 +1768,75 @@ __global__ void k_transpose(const double* __restrict__ X, int n, double* __restr
   XT[j * n + i] = X[i * n + j];
 }
 
-// row i of A^-1 r: sum_j (A^-1)^T[j][i] rs[j] in ascending j, sixteen
-// coefficients loaded before their multiply-adds (one memory wait per
-// sixteen terms instead of one per term)
-__device__ __forceinline__ double coarse_row(const double* __restrict__ AinvT, int n, int i, const double* rs) {
-  double acc = 0.0;
-  int j = 0;
-  for (; j + 16 <= n; j += 16) {
-    double a[16];
-#pragma unroll
-    for (int q = 0; q < 16; ++q) a[q] = __ldg(AinvT + (long long)(j + q) * n + i);
-#pragma unroll
-    for (int q = 0; q < 16; ++q) acc = fma(a[q], rs[j + q], acc);
-  }
-  for (; j < n; ++j) acc = fma(__ldg(AinvT + (long long)j * n + i), rs[j], acc);
-  return acc;
-}
+// <lu> coarse-grid iterator: r := A^-1 r, x := x + damp r.  Each row's sum is
+// one chain of fma in ascending j, 10 cycles a term, and the rows' chains run
+// side by side, so that is the time if the coefficients are at hand: eight
+// warps copy them into shared memory (cp.async), 64 terms of a CTA's rows at a
+// time and one group ahead, and a warp per 32 rows does nothing but the sums.
+// The rows are spread over a cluster, whose CTAs all read r before any of
+// them writes it.  One CTA with a thread per row that loaded its own
+// coefficients took SLOWUS.
+constexpr int kCsStep = 64, kCsLoad = 8;  // terms per group, loading warps
 
-// <lu> coarse-grid iterator: r := A^-1 r, x := x + damp r (one block, n <= 1024)
-__global__ void __launch_bounds__(1024)
-k_coarse_solve(const double* __restrict__ AinvT, int n, double damp, double* x, double* r, long long vs = 0) {
-  __shared__ double rs[1024];
-  const long long bq = blockIdx.x;  // one CTA per problem of a batched base level
-  AinvT += bq * n * n;
+template <int R>  // warps of rows per CTA
+__global__ void __launch_bounds__(32 * (R + kCsLoad), 1)
+k_coarse_solve(const double* __restrict__ AinvT, int n, double damp, double* x, double* r, long long vs, int cs) {
+  constexpr int W = 32 * R, PER = kCsStep / kCsLoad;  // rows, terms per loading warp
+  extern __shared__ double csm[];
+  double* ring = csm;                    // [2][term][row]
+  double* rs = csm + 2 * kCsStep * W;    // the residual
+  const long long bq = blockIdx.x / cs;  // a cluster per problem of a batched base level
+  const int rank = (int)(blockIdx.x - bq * cs), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   x += bq * vs;
   r += bq * vs;
-  const int i = threadIdx.x;
-  if (i < n) rs[i] = r[i];
-  __syncthreads();
-  if (i >= n) return;
-  const double acc = coarse_row(AinvT, n, i, rs);
-  r[i] = acc;
-  x[i] = fma(damp, acc, x[i]);
-}
-
-// the same for n > 1024 unknowns (block bases of the vector form): one CTA,
-// rows strided over its threads, the residual staged in shared memory
-__global__ void __launch_bounds__(1024)
-k_coarse_solve_big(const double* __restrict__ AinvT, int n, double damp, double* x, double* r) {
-  extern __shared__ double rsb[];
-  for (int i = threadIdx.x; i < n; i += blockDim.x) rsb[i] = r[i];
-  __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const double acc = coarse_row(AinvT, n, i, rsb);
+  const int row0 = rank * W, ngroup = (n + kCsStep - 1) / kCsStep;
+  const double* src = AinvT + bq * n * n;
+  // loading warp w copies terms w * PER .. of a group, every row of the CTA
+  // (rows and terms beyond n are not read)
+  auto request = [&](int g) {
+    const int t0 = (warp - R) * PER, cnt = min(PER, n - (g * kCsStep + t0));
+    double* d = ring + ((g & 1) * kCsStep + t0) * W + lane;
+    const double* c = src + (long long)(g * kCsStep + t0) * n;
+#pragma unroll
+    for (int h = 0; h < R; ++h) {
+      const double* ch = c + row0 + 32 * h + lane;
+      if (row0 + 32 * h + lane < n) {
+#pragma unroll
+        for (int q = 0; q < PER; ++q, ch += n)
+          if (q < cnt) cp_async8(d + q * W + 32 * h, ch);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  if (warp >= R) request(0);
+  for (int j = threadIdx.x; j < n; j += blockDim.x) rs[j] = r[j];
+  if (cs > 1) cooperative_groups::this_cluster().sync();
+  double acc = 0.0;
+  for (int g = 0; g < ngroup; ++g) {
+    if (warp >= R) asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();  // group g is there, and the sums of group g - 1 are done
+    if (warp >= R) {
+      if (g + 1 < ngroup) request(g + 1);
+    } else {
+      const double* a = ring + (g & 1) * kCsStep * W + threadIdx.x;
+      const double* v = rs + g * kCsStep;
+      const int cnt = n - g * kCsStep;
+      if (cnt >= kCsStep) {
+#pragma unroll 1
+        for (int q0 = 0; q0 < kCsStep; q0 += 16) {
+          double t[16], u[16];
+#pragma unroll
+          for (int q = 0; q < 16; ++q) { t[q] = a[(q0 + q) * W]; u[q] = v[q0 + q]; }
+#pragma unroll
+          for (int q = 0; q < 16; ++q) acc = fma(t[q], u[q], acc);
+        }
+      } else {
+        for (int q = 0; q < cnt; ++q) acc = fma(a[q * W], v[q], acc);
+      }
+    }
+  }
+  const int i = row0 + (int)threadIdx.x;
+  if (warp < R && i < n) {
     r[i] = acc;
     x[i] = fma(damp, acc, x[i]);
   }
@@ -2463,11 +2729,11 @@ static inline unsigned grid1(long long n, int bs = kBlock) { return (unsigned)((
 // the row kernels of scalar Q2 levels over every class: blockIdx.y the class,
 // blockIdx.x the blocks of its parity subgrids (the largest class's count)
 template <int D>
-static dim3 q2_grid(int M) {
+static dim3 q2_grid(int M, int ssc = -1) {
   int ncol = 1;
   for (int k = 0; k < D; ++k) ncol *= 3;
   long long nb = 1;
-  for (int col = 0; col < ncol; ++col) nb = std::max(nb, q2_class_blocks<D>(M, col));
+  for (int col = 0; col < ncol; ++col) nb = std::max(nb, q2_class_blocks<D>(M, col, ssc));
   return dim3((unsigned)nb, (unsigned)ncol);
 }
 
@@ -2589,12 +2855,16 @@ void launch_sor(const LevelView& L, double omega, double* x, const double* b, do
   int Q = L.order + 1, ncol = 1;
   for (int k = 0; k < L.dim; ++k) ncol *= Q;
   g_launches.fetch_add(ncol, std::memory_order_relaxed);
+  const long long most = (L.M + Q - 1) / Q;  // rows of the largest colour along a direction
+  const bool tile = L.order == 2 && L.dim == 3 && most * most * most <= kTileMax;
   for (int col = 0; col < ncol; ++col) {
     const int cx = col % Q, cy = (col / Q) % Q, cz = col / (Q * Q);
     long long cnt = (L.M - cx + Q - 1) / Q;
     if (L.dim > 1) cnt *= (L.M - cy + Q - 1) / Q;
     if (L.dim > 2) cnt *= (L.M - cz + Q - 1) / Q;
-    if (L.order == 2) {
+    if (tile) {
+      launch_q2_tile<false>(L, col, col > 0, omega, x, b, r, lay, st);
+    } else if (L.order == 2) {
       Q2_DISPATCH(L.dim, {
         const unsigned nb = (unsigned)q2_class_blocks<D>((int)L.M, col);
         if (nb) k_sor_q2<D><<<nb, kQ2T, 0, st>>>(L.A, L.Np, (int)L.M, col, omega, L.omega, x, b, r, lay);
@@ -2644,15 +2914,23 @@ void launch_ssc(const LevelView& L, double omega, double* x, const double* b, do
     }
     return;
   }
+  g_launches.fetch_add(ncol, std::memory_order_relaxed);  // two launches a colour
   const Q2Layout lay = q2_layout(L.dim, L.M);
   const long long nv = (L.M + 1) / 2;
+  const bool tile = L.dim == 3 && L.N <= kSscTileMax;
   for (int col = 0; col < ncol; ++col) {
     long long cnt = (nv - (col & 1) + 1) / 2;
     if (L.dim > 1) cnt *= (nv - ((col >> 1) & 1) + 1) / 2;
     if (L.dim > 2) cnt *= (nv - ((col >> 2) & 1) + 1) / 2;
+    if (cnt == 0) continue;
     const unsigned grid = (unsigned)((cnt * 32 + 127) / 128);
     Q2_DISPATCH(L.dim, {
-      k_ssc_q2<D><<<grid, 128, 0, st>>>(L.A, L.N, L.Np, L.M, L.dmask, col, omega, x, b, r, F, P, lay);
+      if (tile)
+        launch_q2_tile<true>(L, col, col > 0, 0.0, x, b, r, lay, st);
+      else
+        launch_pdl(col > 0, k_ssc_res_q2<D>, q2_grid<D>((int)L.M, col), kQ2T, 0, st, L.A, L.Np, (int)L.M, col, L.dmask,
+                   x, b, r, lay);
+      launch_pdl(true, k_ssc_solve_q2<D>, dim3(grid), 128, 0, st, (int)L.M, L.dmask, col, omega, x, r, F, P);
     });
   }
 }
@@ -2720,16 +2998,33 @@ void launch_prolong(const LevelView& Cl, const LevelView& F, const double* xc, d
 void launch_coarse_solve(const double* AinvT, int n, double damp, double* x, double* r, cudaStream_t st, int nb,
                          long long vs) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  if (n <= 1024) {
-    k_coarse_solve<<<(unsigned)nb, 1024, 0, st>>>(AinvT, n, damp, x, r, vs);
-  } else {
-    static bool init = false;
-    if (!init) {
-      cudaFuncSetAttribute(k_coarse_solve_big, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024 * 4);
-      init = true;
-    }
-    k_coarse_solve_big<<<1, 1024, (size_t)n * sizeof(double), st>>>(AinvT, n, damp, x, r);
-  }
+  // one warp of rows per CTA up to 512 unknowns, then two, then four (the
+  // largest block bases, 2,048); clusters beyond 8 CTAs are not portable
+  auto go = [&](auto RT) {
+    constexpr int R = decltype(RT)::value;
+    int cs = 1;
+    while (cs * 32 * R < n) cs *= 2;
+    auto kern = k_coarse_solve<R>;
+    const size_t smem = (size_t)(2 * kCsStep * 32 * R + n) * sizeof(double);
+    // a refusal shows as the launch's error
+    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (cs > 8) cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)cs;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)(nb * cs));
+    cfg.blockDim = dim3(32 * (R + kCsLoad));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, AinvT, n, damp, x, r, vs, cs);
+  };
+  if (n <= 512) go(std::integral_constant<int, 1>{});
+  else if (n <= 1024) go(std::integral_constant<int, 2>{});
+  else go(std::integral_constant<int, 4>{});
 }
 
 void launch_lu(double* A, int n, int* piv, double* X, double* XT, cudaStream_t st) {
