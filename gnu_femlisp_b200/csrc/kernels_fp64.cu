@@ -1380,12 +1380,12 @@ __device__ __forceinline__ bool face_dir(int c, int M, int k, int dmask) {
 // outside the level and Dirichlet nodes are skipped.  (3D Q1, 129^3 coarse
 // nodes: 64 us, 138 us with each load waiting for the previous term; one
 // memory wait per plane on small levels, 12.4 -> 6 us at 33^3.)
-template <int D, int P>
-__device__ __forceinline__ double restrict_node(const int cJ[3], int MC, int MF, int dmask,
-                                                const double* __restrict__ rf) {
+// NC: components per node; rf points at the component summed.
+template <int D, int P, int NC = 1, typename T = double>
+__device__ __forceinline__ T restrict_node(const int cJ[3], int MC, int MF, int dmask, const T* __restrict__ rf) {
 #pragma unroll
   for (int k = 0; k < D; ++k)
-    if (face_dir(cJ[k], MC, k, dmask)) return 0.0;
+    if (face_dir(cJ[k], MC, k, dmask)) return T(0);
   constexpr int R = P == 1 ? 3 : 5;
   // per direction: fine coordinate and weight of each position, and whether it is met
   int f[3][R];
@@ -1404,17 +1404,17 @@ __device__ __forceinline__ double restrict_node(const int cJ[3], int MC, int MF,
       on[k][q] = q < cnt && f[k][q] >= 0 && f[k][q] < MF && !face_dir(f[k][q], MF, k, dmask);
     }
   }
-  double acc = 0.0;
+  T acc = T(0);
 #pragma unroll
   for (int z = 0; z < (D > 2 ? R : 1); ++z) {
-    double v[R * R];
+    T v[R * R];
 #pragma unroll
     for (int y = 0; y < (D > 1 ? R : 1); ++y)
 #pragma unroll
       for (int q = 0; q < R; ++q)
         if (on[0][q] && (D < 2 || on[1][y]) && (D < 3 || on[2][z]))
-          v[y * R + q] = __ldg(rf + f[0][q] + (long long)MF * ((D > 1 ? f[1][y] : 0) +
-                                                               (long long)MF * (D > 2 ? f[2][z] : 0)));
+          v[y * R + q] = __ldg(rf + NC * (f[0][q] + (long long)MF * ((D > 1 ? f[1][y] : 0) +
+                                                                     (long long)MF * (D > 2 ? f[2][z] : 0))));
 #pragma unroll
     for (int y = 0; y < (D > 1 ? R : 1); ++y)
 #pragma unroll
@@ -1423,7 +1423,7 @@ __device__ __forceinline__ double restrict_node(const int cJ[3], int MC, int MF,
           double ww = w[0][q];
           if (D > 1) ww = ww * w[1][y];
           if (D > 2) ww = ww * w[2][z];
-          acc = fma(ww, v[y * R + q], acc);
+          acc = fma((T)ww, v[y * R + q], acc);
         }
   }
   return acc;
@@ -1431,9 +1431,8 @@ __device__ __forceinline__ double restrict_node(const int cJ[3], int MC, int MF,
 
 // (I xc) at fine node fi, not a Dirichlet node (constrained); all loads first
 // (3D Q1, 257^3 fine nodes: 197 us, 469 us with a load per term)
-template <int D, int P>
-__device__ __forceinline__ double prolong_node(const int fi[3], int MF, int MC, int dmask,
-                                               const double* __restrict__ xc) {
+template <int D, int P, int NC = 1, typename T = double>
+__device__ __forceinline__ T prolong_node(const int fi[3], int MF, int MC, int dmask, const T* __restrict__ xc) {
   constexpr int R = P == 1 ? 2 : 3;
   int j[3][R];
   double w[3][R];
@@ -1452,7 +1451,7 @@ __device__ __forceinline__ double prolong_node(const int fi[3], int MF, int MC, 
     }
   }
   constexpr int NY = D > 1 ? R : 1, NZ = D > 2 ? R : 1;
-  double v[NZ * NY * R];
+  T v[NZ * NY * R];
 #pragma unroll
   for (int z = 0; z < NZ; ++z)
 #pragma unroll
@@ -1460,9 +1459,9 @@ __device__ __forceinline__ double prolong_node(const int fi[3], int MF, int MC, 
 #pragma unroll
       for (int q = 0; q < R; ++q)
         if (on[0][q] && (D < 2 || on[1][y]) && (D < 3 || on[2][z]))
-          v[(z * NY + y) * R + q] = __ldg(xc + j[0][q] + (long long)MC * ((D > 1 ? j[1][y] : 0) +
-                                                                          (long long)MC * (D > 2 ? j[2][z] : 0)));
-  double acc = 0.0;
+          v[(z * NY + y) * R + q] = __ldg(xc + NC * (j[0][q] + (long long)MC * ((D > 1 ? j[1][y] : 0) +
+                                                                                (long long)MC * (D > 2 ? j[2][z] : 0))));
+  T acc = T(0);
 #pragma unroll
   for (int z = 0; z < NZ; ++z)
 #pragma unroll
@@ -1473,7 +1472,7 @@ __device__ __forceinline__ double prolong_node(const int fi[3], int MF, int MC, 
           double ww = w[0][q];
           if (D > 1) ww = ww * w[1][y];
           if (D > 2) ww = ww * w[2][z];
-          acc = fma(ww, v[(z * NY + y) * R + q], acc);
+          acc = fma((T)ww, v[(z * NY + y) * R + q], acc);
         }
   return acc;
 }
@@ -1774,8 +1773,10 @@ __global__ void k_transpose(const double* __restrict__ X, int n, double* __restr
 // warps copy them into shared memory (cp.async), 64 terms of a CTA's rows at a
 // time and one group ahead, and a warp per 32 rows does nothing but the sums.
 // The rows are spread over a cluster, whose CTAs all read r before any of
-// them writes it.  One CTA with a thread per row that loaded its own
-// coefficients took SLOWUS.
+// them writes it.  With one CTA and a thread per row that loaded its own
+// coefficients 343 unknowns took 52 us (8 so), 1,029 took 125 us (21 so, near
+// what eight warps can copy).  A cp.async whose lanes repeat an address is many
+// times slower, so rows beyond n are left out and not clamped.
 constexpr int kCsStep = 64, kCsLoad = 8;  // terms per group, loading warps
 
 template <int R>  // warps of rows per CTA
@@ -2204,48 +2205,255 @@ __device__ __forceinline__ void block_solve3(const T* B, const T* r, T* t) {
   }
 }
 
-// the three block-row sums of node i: slots ascending, columns ascending
-template <int P, typename T>
-__device__ __forceinline__ void row_sums3(const T* __restrict__ A, long long N, long long Np, long long M,
-                                          const T* __restrict__ x, long long i, T* s, T* dblk) {
-  constexpr int NS = St<3, P>::NS;
-  constexpr int C = St<3, P>::CENTER;
-  s[0] = s[1] = s[2] = T(0);
-  auto blk = [&](int sl, long long o, long long p, bool) {
-    const long long j = clampi(i + o, N);
-    const T xj[3] = {__ldg(x + 3 * j), __ldg(x + 3 * j + 1), __ldg(x + 3 * j + 2)};
+// The block rows of 64 consecutive nodes, a thread per scalar row (node i,
+// component k): sum over the slots ascending, columns ascending, of
+// A(i, s)[k][m] x(i + off_s)[m].  OP: y = A x, r = b - A x (b may alias r), or
+// compute-residual fused with the following block <jacobi> step: r_i = b_i -
+// (A x)_i, t = B^-1 r_i, y_i = x_i + w t, r_i := t.
+// The stencil's (y, z) slot rows run in a loop (unrolled, the code took longer
+// to fetch than to run on small levels), a slot row's coefficients loaded one
+// turn ahead.  The unknowns come from shared memory: the nodes a slot row
+// meets are consecutive, so each of the (2 P + 1)^2 segments of 64 + 2 P nodes
+// is read once, coalesced, before the loop (nodes outside the level as 0,
+// where the stored coefficients are 0 too).  FP64 Q2 matvec: 49^3 nodes 191 ->
+// 138 us, 25^3 58 -> 25 us, 13^3 41 -> 20 us against a thread per node with
+// the slots unrolled.
+// nodes from which the FP32 form takes a thread per node (97^3 nodes: 443 us so,
+// 814 us a thread per scalar row, 656 us before either; 49^3: 82, 122, 140 us;
+// 25^3: 26 and 24 us); in FP64 the scalar rows are as fast there (921 us, 0.69
+// of the copy peak; a thread per node 1,128 us) and faster below
+constexpr long long kNode3Min = 50000;
+enum Row3Op { ROW3_MUL, ROW3_RES, ROW3_JACOBI };
+constexpr int kRow3Nodes = 64, kRow3T = 3 * kRow3Nodes;
+
+template <int P, typename T, int OP>
+__global__ void __launch_bounds__(kRow3T, sizeof(T) == 8 ? 3 : 4)
+k_row3(const T* __restrict__ A, int N, long long Np, int M, double damp, const double* __restrict__ omega,
+       const T* __restrict__ x, const T* b, T* y, T* r, int write_r) {
+  constexpr int W = 2 * P + 1, Q = W * W, SEG = 3 * (kRow3Nodes + 2 * P);
+  extern __shared__ unsigned char row3_sm[];
+  T* xs = reinterpret_cast<T*>(row3_sm);  // [slot row][node - i0 + P][component]
+  const int node = threadIdx.x % kRow3Nodes, k = threadIdx.x / kRow3Nodes;
+  const int i0 = blockIdx.x * kRow3Nodes, i = min(i0 + node, N - 1);
+  const bool live = i0 + node < N;
+  // the node's place in the slot arrays of every pattern (Q2: sliced storage)
+  const int H = (M + 1) / 2;
+  const unsigned q0 = (unsigned)i / (unsigned)M;
+  const int c0 = i - (int)q0 * M, c1 = (int)(q0 % (unsigned)M), c2 = (int)(q0 / (unsigned)M);
+  const bool ex = P == 1 || !(c0 & 1), ey = !(c1 & 1), ez = !(c2 & 1);
+  const T* Ak = A + (long long)(3 * k) * Np;
+  T cur[W][3], nxt[W][3];
+  auto load = [&](int q, T (&v)[W][3]) {  // slot row q's coefficients, 0 where not stored
+    const int sy = q % W, sz = q / W;
+    const bool ry = P == 2 && (sy == 0 || sy == 4), rz = P == 2 && (sz == 0 || sz == 4);
+    const bool on = q < Q && !(ry && !ey) && !(rz && !ez);
+    int p0 = i, p1 = i;
+    if (P == 2) {
+      const int yz = (ry ? c1 >> 1 : c1) + (ry ? H : M) * (rz ? c2 >> 1 : c2);
+      p0 = c0 + M * yz;
+      p1 = (c0 >> 1) + H * yz;
+    }
+    const T* a = Ak + (long long)(9 * W * q) * Np;
 #pragma unroll
-    for (int k = 0; k < 3; ++k)
+    for (int sx = 0; sx < W; ++sx) {
+      const bool rx = P == 2 && (sx == 0 || sx == 4);
 #pragma unroll
       for (int m = 0; m < 3; ++m) {
-        const T a = __ldg(A + ((long long)(sl * 3 + k) * 3 + m) * Np + p);
-        if (dblk && sl == C) dblk[k * 3 + m] = a;
-        s[k] = fma(a, xj[m], s[k]);
+        v[sx][m] = T(0);
+        if (on && (!rx || ex)) v[sx][m] = __ldg(a + (long long)(9 * sx + m) * Np + (rx ? p1 : p0));
       }
+    }
   };
-  if constexpr (P == 2) {  // sliced storage
-    long long c[3];
-    node_coords32(i, M, 3, c);
-    Q2Base<3> qb;
-    q2_base<3, false>(Q2Layout{}, c, M, qb);
-    q2_visit<3, false>(qb, M, blk);
-  } else {
-#pragma unroll 3
-    for (int sl = 0; sl < NS; ++sl) blk(sl, slot_off<3, P>(sl, M), i, true);
+  load(0, cur);
+  // the unknowns, nine loads at a time
+  constexpr int PER = (Q * SEG + kRow3T - 1) / kRow3T, BATCH = 9;
+#pragma unroll 1
+  for (int f0 = 0; f0 < PER; f0 += BATCH) {
+    T v[BATCH];
+#pragma unroll
+    for (int t = 0; t < BATCH; ++t) {
+      const int f = (f0 + t) * kRow3T + threadIdx.x, q = f / SEG, e = f - q * SEG;
+      const long long g = 3LL * (i0 + (q % W - P) * M + (q / W - P) * M * M - P) + e;
+      v[t] = f < Q * SEG && g >= 0 && g < 3LL * N ? __ldg(x + g) : T(0);
+    }
+#pragma unroll
+    for (int t = 0; t < BATCH; ++t) {
+      const int f = (f0 + t) * kRow3T + threadIdx.x;
+      if (f < Q * SEG) xs[f] = v[t];
+    }
+  }
+  const T bi = OP == ROW3_MUL ? T(0) : b[3LL * i + k];
+  __syncthreads();
+  T s = T(0), dk[3] = {T(0), T(0), T(0)};
+#pragma unroll 1
+  for (int q = 0; q < Q; ++q) {
+    load(q + 1, nxt);
+    const int sy = q % W, sz = q / W;
+    const bool on = P == 1 || (!((sy == 0 || sy == 4) && !ey) && !((sz == 0 || sz == 4) && !ez));
+    const T* xp = xs + q * SEG + 3 * node;
+    if (on) {
+#pragma unroll
+      for (int sx = 0; sx < W; ++sx) {
+        if (P == 2 && (sx == 0 || sx == 4) && !ex) continue;
+#pragma unroll
+        for (int m = 0; m < 3; ++m) s = fma(cur[sx][m], xp[3 * sx + m], s);
+      }
+    }
+    if (OP == ROW3_JACOBI && q == Q / 2) {
+#pragma unroll
+      for (int m = 0; m < 3; ++m) dk[m] = cur[P][m];
+    }
+#pragma unroll
+    for (int sx = 0; sx < W; ++sx)
+#pragma unroll
+      for (int m = 0; m < 3; ++m) cur[sx][m] = nxt[sx][m];
+  }
+  const T res = bi - s;
+  if (OP != ROW3_JACOBI) {
+    if (live) y[3LL * i + k] = OP == ROW3_RES ? res : s;
+    return;
+  }
+  // the node's residual and diagonal block meet in shared memory
+  T* ds = xs + Q * SEG + node;  // [entry][node]: 3 residuals, 9 block entries
+  ds[k * kRow3Nodes] = res;
+#pragma unroll
+  for (int m = 0; m < 3; ++m) ds[(3 + 3 * k + m) * kRow3Nodes] = dk[m];
+  __syncthreads();
+  if (k != 0 || !live) return;
+  T rr[3], B[9], t[3];
+#pragma unroll
+  for (int e = 0; e < 3; ++e) rr[e] = ds[e * kRow3Nodes];
+#pragma unroll
+  for (int e = 0; e < 9; ++e) B[e] = ds[(3 + e) * kRow3Nodes];
+  block_solve3<T>(B, rr, t);
+  const T w = omega ? (T)omega[i] : (T)damp;
+  const T* xi = xs + (Q / 2) * SEG + 3 * (node + P);
+#pragma unroll
+  for (int e = 0; e < 3; ++e) {
+    if (write_r) r[3LL * i + e] = t[e];
+    y[3LL * i + e] = fma(w, t[e], xi[e]);
   }
 }
 
-// y = A x or r = b - A x (b may alias r)
-template <int P, bool RES, typename T = double>
-__global__ void __launch_bounds__(kBlock)
-k_spmv3(const T* __restrict__ A, long long N, long long Np, long long M, const T* __restrict__ x,
-        const T* b, T* y) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  T s[3];
-  row_sums3<P, T>(A, N, Np, M, x, i, s, (T*)nullptr);
+// The same with a thread per node, for large FP32 levels: the loop's loads are
+// then uniform bases plus one 32-bit offset (k is known to the compiler), where
+// the scalar-row form spends most of its issue slots on addresses.  Bound by
+// the memory waits of its 25 slot rows (16 warps an SM, 45 loads each in
+// flight: 4.6 TB/s at 97^3 nodes); requesting a slot row ahead halves the
+// warps and measured slower.
+template <int P, typename T, int OP>
+__global__ void __launch_bounds__(kRow3Nodes, 8)
+k_node3(const T* __restrict__ A, int N, long long Np, int M, double damp, const double* __restrict__ omega,
+        const T* __restrict__ x, const T* b, T* y, T* r, int write_r) {
+  constexpr int W = 2 * P + 1, Q = W * W, SEG = 3 * (kRow3Nodes + 2 * P);
+  extern __shared__ unsigned char row3_sm[];
+  T* xs = reinterpret_cast<T*>(row3_sm);  // [slot row][node - i0 + P][component]
+  const int i0 = blockIdx.x * kRow3Nodes, i = min(i0 + (int)threadIdx.x, N - 1);
+  const bool live = i0 + (int)threadIdx.x < N;
+  const int H = (M + 1) / 2;
+  const unsigned q0 = (unsigned)i / (unsigned)M;
+  const int c0 = i - (int)q0 * M, c1 = (int)(q0 % (unsigned)M), c2 = (int)(q0 / (unsigned)M);
+  const bool ex = P == 1 || !(c0 & 1), ey = !(c1 & 1), ez = !(c2 & 1);
+  constexpr int PER = (Q * SEG + kRow3Nodes - 1) / kRow3Nodes, BATCH = 16;
+#pragma unroll 1
+  for (int f0 = 0; f0 < PER; f0 += BATCH) {
+    T v[BATCH];
 #pragma unroll
-  for (int k = 0; k < 3; ++k) y[3 * i + k] = RES ? b[3 * i + k] - s[k] : s[k];
+    for (int t = 0; t < BATCH; ++t) {
+      const int f = (f0 + t) * kRow3Nodes + threadIdx.x, q = f / SEG, e = f - q * SEG;
+      const long long g = 3LL * (i0 + (q % W - P) * M + (q / W - P) * M * M - P) + e;
+      v[t] = f < Q * SEG && g >= 0 && g < 3LL * N ? __ldg(x + g) : T(0);
+    }
+#pragma unroll
+    for (int t = 0; t < BATCH; ++t) {
+      const int f = (f0 + t) * kRow3Nodes + threadIdx.x;
+      if (f < Q * SEG) xs[f] = v[t];
+    }
+  }
+  T bi[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) bi[k] = OP == ROW3_MUL ? T(0) : b[3LL * i + k];
+  __syncthreads();
+  T s[3] = {T(0), T(0), T(0)}, B[9];
+#pragma unroll 1
+  for (int sz = 0; sz < W; ++sz) {
+    const bool rz = P == 2 && (sz == 0 || sz == 4);
+    if (rz && !ez) continue;
+#pragma unroll 1
+    for (int sy = 0; sy < W; ++sy) {
+      const bool ry = P == 2 && (sy == 0 || sy == 4);
+      if (ry && !ey) continue;
+      const int q = sy + W * sz;
+      unsigned p0 = (unsigned)i, p1 = (unsigned)i;
+      if (P == 2) {
+        const int yz = (ry ? c1 >> 1 : c1) + (ry ? H : M) * (rz ? c2 >> 1 : c2);
+        p0 = (unsigned)(c0 + M * yz);
+        p1 = (unsigned)((c0 >> 1) + H * yz);
+      }
+      const T* a = A + (long long)(9 * W * q) * Np;
+      T v[W][9];
+#pragma unroll
+      for (int sx = 0; sx < W; ++sx) {
+        const bool rx = P == 2 && (sx == 0 || sx == 4);
+#pragma unroll
+        for (int e = 0; e < 9; ++e)
+          if (!rx || ex) v[sx][e] = __ldg(a + (long long)(9 * sx + e) * Np + (rx ? p1 : p0));
+      }
+      const T* xp = xs + q * SEG + 3 * threadIdx.x;
+#pragma unroll
+      for (int sx = 0; sx < W; ++sx) {
+        if (P == 2 && (sx == 0 || sx == 4) && !ex) continue;
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+          for (int m = 0; m < 3; ++m) s[k] = fma(v[sx][3 * k + m], xp[3 * sx + m], s[k]);
+      }
+      if (OP == ROW3_JACOBI && q == Q / 2) {
+#pragma unroll
+        for (int e = 0; e < 9; ++e) B[e] = v[P][e];
+      }
+    }
+  }
+  if (!live) return;
+  T rr[3], t[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) rr[k] = OP == ROW3_MUL ? s[k] : bi[k] - s[k];
+  if (OP != ROW3_JACOBI) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) y[3LL * i + k] = rr[k];
+    return;
+  }
+  block_solve3<T>(B, rr, t);
+  const T w = omega ? (T)omega[i] : (T)damp;
+  const T* xi = xs + (Q / 2) * SEG + 3 * (threadIdx.x + P);
+#pragma unroll
+  for (int e = 0; e < 3; ++e) {
+    if (write_r) r[3LL * i + e] = t[e];
+    y[3LL * i + e] = fma(w, t[e], xi[e]);
+  }
+}
+
+template <typename T, int OP>
+static void launch_row3(int order, const T* A, long long N, long long Np, long long M, double damp,
+                        const double* omega, const T* x, const T* b, T* y, T* r, bool write_r, cudaStream_t st) {
+  auto go = [&](auto PT) {
+    constexpr int P = decltype(PT)::value, W = 2 * P + 1;
+    constexpr size_t smem = (W * W * 3 * (kRow3Nodes + 2 * P) + (OP == ROW3_JACOBI ? 12 * kRow3Nodes : 0)) * sizeof(T);
+    const unsigned grid = (unsigned)((N + kRow3Nodes - 1) / kRow3Nodes);
+    if constexpr (sizeof(T) == 4) {
+      if (N >= kNode3Min) {
+        k_node3<P, T, OP><<<grid, kRow3Nodes, smem, st>>>(A, (int)N, Np, (int)M, damp, omega, x, b, y, r,
+                                                          write_r ? 1 : 0);
+        return;
+      }
+    }
+    if (smem > 48 * 1024)
+      cudaFuncSetAttribute(k_row3<P, T, OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_row3<P, T, OP><<<grid, kRow3T, smem, st>>>(
+        A, (int)N, Np, (int)M, damp, omega, x, b, y, r, write_r ? 1 : 0);
+  };
+  if (order == 2) go(std::integral_constant<int, 2>{});
+  else go(std::integral_constant<int, 1>{});
 }
 
 // <jacobi> on 3 x 3 blocks with an up-to-date residual: t = B^-1 r_i, x_i += w t, r_i := t
@@ -2267,78 +2475,49 @@ k_jacobi3(const double* __restrict__ A, long long N, long long Np, int center, d
   }
 }
 
-// compute-residual fused with the following block <jacobi> step:
-// r_i = b_i - (A x)_i, t = B^-1 r_i, xout_i = x_i + w t, r_i := t
-template <int P, typename T = double>
-__global__ void __launch_bounds__(kBlock)
-k_jacobi_res3(const T* __restrict__ A, long long N, long long Np, long long M, double damp,
-              const double* __restrict__ omega, const T* __restrict__ x, const T* b,
-              T* __restrict__ xout, T* r, int write_r) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  T s[3], B[9], t[3];
-  row_sums3<P, T>(A, N, Np, M, x, i, s, B);
-  const T rr[3] = {b[3 * i] - s[0], b[3 * i + 1] - s[1], b[3 * i + 2] - s[2]};
-  block_solve3<T>(B, rr, t);
-  const T w = omega ? (T)omega[i] : (T)damp;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    if (write_r) r[3 * i + k] = t[k];
-    xout[3 * i + k] = fma(w, t[k], x[3 * i + k]);
-  }
-}
+// The transfer sums of a node's three components with the terms in loops, for
+// large levels: a thread per scalar unknown repeats the node's indices and
+// weights three times and is bound by them there (Q2, 49^3 coarse nodes:
+// restriction 150 us, 74 so; prolongation to 97^3 105 and 57 us; the other
+// way round on small levels, where memory waits are the time: 19 and 31 us
+// at 13^3).
+constexpr long long kXferLoopMin = 30000;
 
-// rc := I^T rf per component (constrained), rhs_c := rc, sol_c := 0
-template <int P, typename T = double>
-__global__ void __launch_bounds__(kBlock)
-k_restrict3(int MC, int MF, int dmask, const T* __restrict__ rf, T* __restrict__ rc,
-            T* __restrict__ rhsc, T* __restrict__ solc) {
-  const int cJ[3] = {(int)(blockIdx.x * 32 + threadIdx.x), (int)(blockIdx.y * 8 + threadIdx.y), (int)blockIdx.z};
-  if (cJ[0] >= MC || cJ[1] >= MC) return;
-  const long long J = cJ[0] + (long long)MC * (cJ[1] + (long long)MC * cJ[2]);
-  bool dj = false;
-  for (int k = 0; k < 3; ++k) dj = dj || face_dir(cJ[k], MC, k, dmask);
-  T acc[3] = {T(0), T(0), T(0)};
-  if (!dj) {
-    long long off[3][5] = {{0}, {0}, {0}};
-    double w[3][5] = {{1.0}, {1.0}, {1.0}};
-    int cnt[3];
-    for (int k = 0; k < 3; ++k) cnt[k] = restrict_1d<P>(cJ[k], off[k], w[k]);
-    for (int z = 0; z < cnt[2]; ++z)
-      for (int y = 0; y < cnt[1]; ++y)
-        for (int xx = 0; xx < cnt[0]; ++xx) {
-          const int fi[3] = {2 * cJ[0] + (int)off[0][xx], 2 * cJ[1] + (int)off[1][y], 2 * cJ[2] + (int)off[2][z]};
-          bool skip = false;
-          for (int k = 0; k < 3; ++k) skip = skip || fi[k] < 0 || fi[k] >= MF || face_dir(fi[k], MF, k, dmask);
-          if (skip) continue;
-          const T ww = (T)(w[0][xx] * w[1][y] * w[2][z]);
-          const long long f = fi[0] + (long long)MF * (fi[1] + (long long)MF * fi[2]);
+template <int P, typename T>
+__device__ __forceinline__ void restrict3_loop(const int cJ[3], int MC, int MF, int dmask, const T* __restrict__ rf,
+                                              T (&acc)[3]) {
 #pragma unroll
-          for (int c = 0; c < 3; ++c) acc[c] = fma(ww, rf[3 * f + c], acc[c]);
-        }
-  }
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    rc[3 * J + c] = acc[c];
-    rhsc[3 * J + c] = acc[c];
-    solc[3 * J + c] = T(0);
-  }
-}
-
-// xf := xf + I xc per component (constrained)
-template <int P, typename T = double>
-__global__ void __launch_bounds__(kBlock)
-k_prolong3(int MF, int MC, int dmask, const T* __restrict__ xc, T* __restrict__ xf) {
-  const int fi[3] = {(int)(blockIdx.x * 32 + threadIdx.x), (int)(blockIdx.y * 8 + threadIdx.y), (int)blockIdx.z};
-  if (fi[0] >= MF || fi[1] >= MF) return;
+  for (int c = 0; c < 3; ++c) acc[c] = T(0);
   for (int k = 0; k < 3; ++k)
-    if (face_dir(fi[k], MF, k, dmask)) return;
-  const long long i = fi[0] + (long long)MF * (fi[1] + (long long)MF * fi[2]);
+    if (face_dir(cJ[k], MC, k, dmask)) return;
+  long long off[3][5] = {{0}, {0}, {0}};
+  double w[3][5] = {{1.0}, {1.0}, {1.0}};
+  int cnt[3] = {1, 1, 1};
+  for (int k = 0; k < 3; ++k) cnt[k] = restrict_1d<P>(cJ[k], off[k], w[k]);
+  for (int z = 0; z < cnt[2]; ++z)
+    for (int y = 0; y < cnt[1]; ++y)
+      for (int xx = 0; xx < cnt[0]; ++xx) {
+        const int fi[3] = {2 * cJ[0] + (int)off[0][xx], 2 * cJ[1] + (int)off[1][y], 2 * cJ[2] + (int)off[2][z]};
+        bool skip = false;
+        for (int k = 0; k < 3; ++k) skip = skip || fi[k] < 0 || fi[k] >= MF || face_dir(fi[k], MF, k, dmask);
+        if (skip) continue;
+        double ww = w[0][xx];
+        ww = ww * w[1][y] * w[2][z];
+        const long long f = fi[0] + (long long)MF * (fi[1] + (long long)MF * fi[2]);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) acc[c] = fma((T)ww, rf[3 * f + c], acc[c]);
+      }
+}
+
+template <int P, typename T>
+__device__ __forceinline__ void prolong3_loop(const int fi[3], int MC, int dmask, const T* __restrict__ xc,
+                                             T (&acc)[3]) {
+#pragma unroll
+  for (int c = 0; c < 3; ++c) acc[c] = T(0);
   long long J[3][3] = {{0}, {0}, {0}};
   double w[3][3] = {{1.0}, {1.0}, {1.0}};
-  int cnt[3];
+  int cnt[3] = {1, 1, 1};
   for (int k = 0; k < 3; ++k) cnt[k] = prolong_1d<P>(fi[k], J[k], w[k]);
-  T acc[3] = {T(0), T(0), T(0)};
   for (int z = 0; z < cnt[2]; ++z)
     for (int y = 0; y < cnt[1]; ++y)
       for (int xx = 0; xx < cnt[0]; ++xx) {
@@ -2346,13 +2525,77 @@ k_prolong3(int MF, int MC, int dmask, const T* __restrict__ xc, T* __restrict__ 
         bool dj = false;
         for (int k = 0; k < 3; ++k) dj = dj || face_dir(cj[k], MC, k, dmask);
         if (dj) continue;
-        const T ww = (T)(w[0][xx] * w[1][y] * w[2][z]);
+        double ww = w[0][xx];
+        ww = ww * w[1][y] * w[2][z];
         const long long j = cj[0] + (long long)MC * (cj[1] + (long long)MC * cj[2]);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) acc[c] = fma(ww, xc[3 * j + c], acc[c]);
+        for (int c = 0; c < 3; ++c) acc[c] = fma((T)ww, xc[3 * j + c], acc[c]);
       }
+}
+
+// rc := I^T rf per component (constrained), rhs_c := rc, sol_c := 0.  LOOP: a
+// thread per node, its three components in the loop form; otherwise a thread
+// per scalar unknown (x: node and component)
+template <int P, bool LOOP, typename T = double>
+__global__ void __launch_bounds__(kBlock)
+k_restrict3(int MC, int MF, int dmask, const T* __restrict__ rf, T* __restrict__ rc,
+            T* __restrict__ rhsc, T* __restrict__ solc) {
+  constexpr int CT = LOOP ? 3 : 1;
+  const int xs = blockIdx.x * 32 + threadIdx.x, c0 = LOOP ? 0 : xs % 3;
+  const int cJ[3] = {LOOP ? xs : xs / 3, (int)(blockIdx.y * 8 + threadIdx.y), (int)blockIdx.z};
+  if (cJ[0] >= MC || cJ[1] >= MC) return;
+  const long long J = 3 * (cJ[0] + (long long)MC * (cJ[1] + (long long)MC * cJ[2])) + c0;
+  T acc[CT];
+  if constexpr (LOOP) restrict3_loop<P, T>(cJ, MC, MF, dmask, rf, acc);
+  else acc[0] = restrict_node<3, P, 3, T>(cJ, MC, MF, dmask, rf + c0);
 #pragma unroll
-  for (int c = 0; c < 3; ++c) xf[3 * i + c] = xf[3 * i + c] + acc[c];
+  for (int c = 0; c < CT; ++c) {
+    rc[J + c] = acc[c];
+    rhsc[J + c] = acc[c];
+    solc[J + c] = T(0);
+  }
+}
+
+// xf := xf + I xc per component (constrained)
+template <int P, bool LOOP, typename T = double>
+__global__ void __launch_bounds__(kBlock)
+k_prolong3(int MF, int MC, int dmask, const T* __restrict__ xc, T* __restrict__ xf) {
+  constexpr int CT = LOOP ? 3 : 1;
+  const int xs = blockIdx.x * 32 + threadIdx.x, c0 = LOOP ? 0 : xs % 3;
+  const int fi[3] = {LOOP ? xs : xs / 3, (int)(blockIdx.y * 8 + threadIdx.y), (int)blockIdx.z};
+  if (fi[0] >= MF || fi[1] >= MF) return;
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    if (face_dir(fi[k], MF, k, dmask)) return;
+  const long long i = 3 * (fi[0] + (long long)MF * (fi[1] + (long long)MF * fi[2])) + c0;
+  T acc[CT];
+  if constexpr (LOOP) prolong3_loop<P, T>(fi, MC, dmask, xc, acc);
+  else acc[0] = prolong_node<3, P, 3, T>(fi, MF, MC, dmask, xc + c0);
+#pragma unroll
+  for (int c = 0; c < CT; ++c) xf[i + c] = xf[i + c] + acc[c];
+}
+
+template <typename T>
+static void launch_restrict3(int order, long long MC, long long MF, int dmask, const T* rf, T* rc, T* rhsc, T* solc,
+                             cudaStream_t st) {
+  const bool big = MC * MC * MC >= kXferLoopMin;
+  const dim3 g((unsigned)(((big ? 1 : 3) * MC + 31) / 32), (unsigned)((MC + 7) / 8), (unsigned)MC), t(32, 8);
+  const int mc = (int)MC, mf = (int)MF;
+  if (order == 2 && big) k_restrict3<2, true, T><<<g, t, 0, st>>>(mc, mf, dmask, rf, rc, rhsc, solc);
+  else if (order == 2) k_restrict3<2, false, T><<<g, t, 0, st>>>(mc, mf, dmask, rf, rc, rhsc, solc);
+  else if (big) k_restrict3<1, true, T><<<g, t, 0, st>>>(mc, mf, dmask, rf, rc, rhsc, solc);
+  else k_restrict3<1, false, T><<<g, t, 0, st>>>(mc, mf, dmask, rf, rc, rhsc, solc);
+}
+
+template <typename T>
+static void launch_prolong3(int order, long long MF, long long MC, int dmask, const T* xc, T* xf, cudaStream_t st) {
+  const bool big = MF * MF * MF >= kXferLoopMin;
+  const dim3 g((unsigned)(((big ? 1 : 3) * MF + 31) / 32), (unsigned)((MF + 7) / 8), (unsigned)MF), t(32, 8);
+  const int mc = (int)MC, mf = (int)MF;
+  if (order == 2 && big) k_prolong3<2, true, T><<<g, t, 0, st>>>(mf, mc, dmask, xc, xf);
+  else if (order == 2) k_prolong3<2, false, T><<<g, t, 0, st>>>(mf, mc, dmask, xc, xf);
+  else if (big) k_prolong3<1, true, T><<<g, t, 0, st>>>(mf, mc, dmask, xc, xf);
+  else k_prolong3<1, false, T><<<g, t, 0, st>>>(mf, mc, dmask, xc, xf);
 }
 
 // Elasticity stiffness by gather (the vector form of k_assemble): for node i,
@@ -2747,13 +2990,8 @@ void launch_spmv(const LevelView& L, const double* x, const double* b, double* y
   }
   if (L.nc == 3) {  // 3 x 3 blocks: the reduction, if any, as a separate DR4096 pass
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    if (L.order == 2) {
-      if (b) k_spmv3<2, true><<<grid1(L.N), kBlock, 0, st>>>(L.A, L.N, L.Np, L.M, x, b, y);
-      else k_spmv3<2, false><<<grid1(L.N), kBlock, 0, st>>>(L.A, L.N, L.Np, L.M, x, b, y);
-    } else {
-      if (b) k_spmv3<1, true><<<grid1(L.N), kBlock, 0, st>>>(L.A, L.N, L.Np, L.M, x, b, y);
-      else k_spmv3<1, false><<<grid1(L.N), kBlock, 0, st>>>(L.A, L.N, L.Np, L.M, x, b, y);
-    }
+    if (b) launch_row3<double, ROW3_RES>(L.order, L.A, L.N, L.Np, L.M, 0.0, nullptr, x, b, y, nullptr, false, st);
+    else launch_row3<double, ROW3_MUL>(L.order, L.A, L.N, L.Np, L.M, 0.0, nullptr, x, b, y, nullptr, false, st);
     if (dv) launch_dot(y, dv, 3 * L.N, *R, st);
     return;
   }
@@ -2810,12 +3048,7 @@ void launch_jacobi_res(const LevelView& L, double damp, const double* x, const d
     return;
   }
   if (L.nc == 3) {
-    if (L.order == 2)
-      k_jacobi_res3<2><<<grid1(L.N), kBlock, 0, st>>>(L.A, L.N, L.Np, L.M, damp, L.omega, x, b, xout, r,
-                                                        write_r ? 1 : 0);
-    else
-      k_jacobi_res3<1><<<grid1(L.N), kBlock, 0, st>>>(L.A, L.N, L.Np, L.M, damp, L.omega, x, b, xout, r,
-                                                        write_r ? 1 : 0);
+    launch_row3<double, ROW3_JACOBI>(L.order, L.A, L.N, L.Np, L.M, damp, L.omega, x, b, xout, r, write_r, st);
     if (dv) launch_dot(xout, dv, 3 * L.N, *R, st);
     return;
   }
@@ -2962,10 +3195,7 @@ void launch_restrict(const LevelView& F, const LevelView& Cl, const double* rf, 
     return;
   }
   if (F.nc == 3) {
-    if (F.order == 2)
-      k_restrict3<2><<<xfer_grid(Cl.M, 3), dim3(32, 8), 0, st>>>((int)Cl.M, (int)F.M, F.dmask, rf, rc, rhsc, solc);
-    else
-      k_restrict3<1><<<xfer_grid(Cl.M, 3), dim3(32, 8), 0, st>>>((int)Cl.M, (int)F.M, F.dmask, rf, rc, rhsc, solc);
+    launch_restrict3<double>(F.order, Cl.M, F.M, F.dmask, rf, rc, rhsc, solc, st);
     return;
   }
   FMG_DISPATCH(F.dim, F.order, {
@@ -2982,10 +3212,7 @@ void launch_prolong(const LevelView& Cl, const LevelView& F, const double* xc, d
     return;
   }
   if (F.nc == 3) {
-    if (F.order == 2)
-      k_prolong3<2><<<xfer_grid(F.M, 3), dim3(32, 8), 0, st>>>((int)F.M, (int)Cl.M, F.dmask, xc, xf);
-    else
-      k_prolong3<1><<<xfer_grid(F.M, 3), dim3(32, 8), 0, st>>>((int)F.M, (int)Cl.M, F.dmask, xc, xf);
+    launch_prolong3<double>(F.order, F.M, Cl.M, F.dmask, xc, xf, st);
     return;
   }
   FMG_DISPATCH(F.dim, F.order, {
@@ -3211,8 +3438,7 @@ void launch_acc_prod3(double* acc, const double* a, const double* b, long long N
 void vec32_spmv(int order, const float* A, long long N, long long Np, long long M, const float* x, const float* b,
                 float* y, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  if (order == 2) k_spmv3<2, true, float><<<grid1(N), kBlock, 0, st>>>(A, N, Np, M, x, b, y);
-  else k_spmv3<1, true, float><<<grid1(N), kBlock, 0, st>>>(A, N, Np, M, x, b, y);
+  launch_row3<float, ROW3_RES>(order, A, N, Np, M, 0.0, nullptr, x, b, y, nullptr, false, st);
 }
 void vec32_jacobi0(const float* A, long long N, long long Np, int center, float damp, const double* omega,
                    const float* b, float* x, cudaStream_t st) {
@@ -3222,23 +3448,16 @@ void vec32_jacobi0(const float* A, long long N, long long Np, int center, float 
 void vec32_jacobi_res(int order, const float* A, long long N, long long Np, long long M, double damp,
                       const double* omega, const float* x, const float* b, float* xout, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  if (order == 2)
-    k_jacobi_res3<2, float><<<grid1(N), kBlock, 0, st>>>(A, N, Np, M, damp, omega, x, b, xout, (float*)nullptr, 0);
-  else
-    k_jacobi_res3<1, float><<<grid1(N), kBlock, 0, st>>>(A, N, Np, M, damp, omega, x, b, xout, (float*)nullptr, 0);
+  launch_row3<float, ROW3_JACOBI>(order, A, N, Np, M, damp, omega, x, b, xout, (float*)nullptr, false, st);
 }
 void vec32_restrict(int order, long long MC, long long MF, int dmask, const float* rf, float* bc, float* xc,
                     cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  if (order == 2)
-    k_restrict3<2, float><<<xfer_grid(MC, 3), dim3(32, 8), 0, st>>>((int)MC, (int)MF, dmask, rf, bc, bc, xc);
-  else
-    k_restrict3<1, float><<<xfer_grid(MC, 3), dim3(32, 8), 0, st>>>((int)MC, (int)MF, dmask, rf, bc, bc, xc);
+  launch_restrict3<float>(order, MC, MF, dmask, rf, bc, bc, xc, st);
 }
 void vec32_prolong(int order, long long MF, long long MC, int dmask, const float* xc, float* xf, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  if (order == 2) k_prolong3<2, float><<<xfer_grid(MF, 3), dim3(32, 8), 0, st>>>((int)MF, (int)MC, dmask, xc, xf);
-  else k_prolong3<1, float><<<xfer_grid(MF, 3), dim3(32, 8), 0, st>>>((int)MF, (int)MC, dmask, xc, xf);
+  launch_prolong3<float>(order, MF, MC, dmask, xc, xf, st);
 }
 void vec_to32(const double* x, const double* sc, int slot, int mode, float* y, long long n, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
