@@ -217,6 +217,7 @@ int cuda_err(fmg_ctx* c, cudaError_t e, const char* what) {
   } while (0)
 
 int launched(fmg_ctx* c, const char* what) {
+  pdl_break();  // what was queued may have written what later launches fetch early
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_err(c, e, what);
   return FMG_OK;
@@ -2275,6 +2276,7 @@ int run_step_graph(fmg_grid* g, const fmg_solve_cfg& c, const double* x, Body bo
     const long long l0 = g_launches.load(std::memory_order_relaxed);
     cudaGraph_t gr = nullptr;
     cudaGraphExec_t ex = nullptr;
+    pdl_break();  // a graph's first launch has no predecessor to overlap
     bool ok = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
     if (ok) {
       body();

@@ -112,6 +112,63 @@ __device__ __forceinline__ void dr_finish(double lane_sum, const Reduce& R, doub
   }
 }
 
+// Programmatic dependent launch: a kernel launched with launch_early or
+// launch_pdl (on a small grid) may start while its predecessor in the stream
+// still runs.  pdl_next lets the successor start; pdl_wait waits until the
+// predecessor has finished and its writes are visible.  Every kernel launched
+// so calls both, pdl_wait before its first access to anything that a kernel
+// of the same sequence writes; before it, only what was in place when the
+// sequence began (matrices, damping, factors, indices) is read.  At least one
+// thread of every launch passes pdl_wait, so a launch never ends before its
+// predecessor and waiting for one kernel is waiting for all before it.
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// The stream this thread's last such launch went to.  A sequence begins with a
+// launch that waits for everything before it (the first one on a stream, and
+// the first after launched(), which follows whatever writes a matrix, damping
+// or factors); the launches after it overlap their starts (2-4 us a launch on
+// small levels instead of 4-6).
+extern thread_local cudaStream_t t_pdl_stream;
+inline void pdl_break() { t_pdl_stream = nullptr; }
+
+// Which launches overlap was measured kernel by kernel: kernels that fetch
+// before they wait and light streaming ones gain at every size (launch_early);
+// register- and cache-heavy ones that only wait gain on small grids and lose
+// on large ones (launch_pdl: Q2 residual among the SOR sweeps of 129^3 nodes,
+// 31.9 -> 34.9 ms a solve with all launches early; FCG update of 97^3 nodes,
+// 3.83 -> 4.07 ms), and the elasticity rows lose always (launch_late).
+constexpr long long kPdlBlocks = 148;
+
+template <typename... KA, typename... A>
+inline void launch_after(bool early, void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                         A... args) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = early && t_pdl_stream == st ? 1 : 0;
+  t_pdl_stream = st;
+  cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...);
+}
+template <typename... KA, typename... A>
+inline void launch_early(void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  launch_after(true, kern, grid, block, smem, st, args...);
+}
+template <typename... KA, typename... A>
+inline void launch_pdl(void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  launch_after((long long)grid.x * grid.y * grid.z <= kPdlBlocks, kern, grid, block, smem, st, args...);
+}
+template <typename... KA, typename... A>
+inline void launch_late(void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  launch_after(false, kern, grid, block, smem, st, args...);
+}
+
 inline unsigned nchunks(long long n) { return (unsigned)((n + kChunk - 1) / kChunk); }
 
 }  // namespace fmg

@@ -18,6 +18,7 @@
 namespace fmg {
 
 std::atomic<long long> g_launches{0};
+thread_local cudaStream_t t_pdl_stream = nullptr;
 
 // The Q1 row kernels: 128 threads, four blocks per SM.  The bound matters for
 // its effect on register allocation: without it ptxas keeps the 3D kernels at
@@ -33,32 +34,6 @@ struct St {
   static constexpr int NS = D == 1 ? W : (D == 2 ? W * W : W * W * W);
   static constexpr int CENTER = (NS - 1) / 2;
 };
-
-// Programmatic dependent launch: a kernel launched with launch_pdl may start
-// while its predecessor in the stream still runs.  pdl_next lets the
-// successor start; pdl_wait waits until the predecessor has finished and its
-// writes are visible, and comes before the first access to anything that a
-// kernel of the same sequence writes.
-__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
-// launches kern after the stream's previous kernel, overlapping its start
-// with that kernel's end when early (kern must call pdl_wait)
-template <typename... KA, typename... A>
-static void launch_pdl(bool early, void (*kern)(KA...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
-                       A... args) {
-  cudaLaunchConfig_t cfg{};
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cfg.attrs = &at;
-  cfg.numAttrs = early ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...);
-}
 
 // copies 8 bytes to shared memory in the background
 __device__ __forceinline__ void cp_async8(double* dst, const double* src) {
@@ -383,6 +358,7 @@ __device__ __forceinline__ double q1_row_sum(const double* __restrict__ A, long 
   const double* a = A + i;
 #pragma unroll
   for (int s = 0; s < NS; ++s) av[s] = __ldg(a + s * Np);
+  pdl_wait();  // the coefficients do not depend on the previous launch, the unknowns do
 #pragma unroll
   for (int s = 0; s < NS; ++s) {
     const int o = (s % 3 - 1) + (D > 1 ? M * ((s / 3) % 3 - 1) : 0) + (D > 2 ? M * M * (s / 9 - 1) : 0);
@@ -401,16 +377,16 @@ template <int D, bool RES>
 __global__ void __launch_bounds__(kRowT, kRowMinBlocks)
 k_row_q1(const double* __restrict__ A, int N, long long Np, int M, const double* __restrict__ x, const double* b,
          double* y) {
+  pdl_next();
   const int i = blockIdx.x * kRowT + threadIdx.x;
   if (i >= N) return;
   const long long bq = blockIdx.y;  // problem of a batched level
   A += bq * St<D, 1>::NS * Np;
   x += bq * Np;
   y += bq * Np;
-  const double bi = RES ? b[bq * Np + i] : 0.0;
   double dg;
   const double s = q1_row_sum<D>(A, Np, N, M, x, i, dg);
-  y[i] = RES ? bi - s : s;
+  y[i] = RES ? b[bq * Np + i] - s : s;
 }
 
 // compute-residual fused with the following <jacobi> step on a Q1 level:
@@ -420,17 +396,18 @@ __global__ void __launch_bounds__(kRowT, kRowMinBlocks)
 k_row_jacobi_q1(const double* __restrict__ A, int N, long long Np, int M, double damp,
                 const double* __restrict__ omega, const double* __restrict__ x, const double* b,
                 double* __restrict__ xout, double* r, int write_r) {
+  pdl_next();
   const int i = blockIdx.x * kRowT + threadIdx.x;
   if (i >= N) return;
   const long long bq = blockIdx.y;  // problem of a batched level
   A += bq * St<D, 1>::NS * Np;
   x += bq * Np;
-  const double bi = b[bq * Np + i], xi = __ldg(x + i), w = omega ? __ldg(omega + bq * Np + i) : damp;
+  const double w = omega ? __ldg(omega + bq * Np + i) : damp;
   double dg;
   const double s = q1_row_sum<D>(A, Np, N, M, x, i, dg);
-  const double t = (bi - s) / dg;
+  const double t = (b[bq * Np + i] - s) / dg;
   if (write_r) r[bq * Np + i] = t;
-  xout[bq * Np + i] = fma(w, t, xi);
+  xout[bq * Np + i] = fma(w, t, __ldg(x + i));
 }
 
 // k_jacobi on a scalar Q2 level (the diagonal sits at the node's colour-major place)
@@ -438,6 +415,8 @@ template <int D>
 __global__ void __launch_bounds__(kBlock)
 k_jacobi_q2(const double* __restrict__ A, long long N, long long Np, long long M, double damp,
             const double* __restrict__ omega, double* x, double* r, int write_r, const __grid_constant__ Q2Layout lay) {
+  pdl_next();
+  pdl_wait();
   constexpr int C = St<D, 2>::CENTER;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
@@ -775,11 +754,9 @@ k_q2_tile(const double* __restrict__ A, long long Np, int M, int col, int dmask,
 }
 
 // colour `col` by tiles: blockIdx.x the tiles of the largest parity subgrid,
-// .y the parity, .z the class (SSC).  early: the launches of a sweep after the
-// first start early -- the coefficients, diagonal and damping were in place
-// before the sweep began.
+// .y the parity, .z the class (SSC)
 template <bool SSC>
-static void launch_q2_tile(const LevelView& L, int col, bool early, double damp, double* x, const double* b, double* r,
+static void launch_q2_tile(const LevelView& L, int col, double damp, double* x, const double* b, double* r,
                            const Q2Layout& lay, cudaStream_t st) {
   const int M = (int)L.M;
   long long most = 1;
@@ -789,8 +766,8 @@ static void launch_q2_tile(const LevelView& L, int col, bool early, double damp,
       q2_sub<3>(M, cls, pat, s, SSC ? col : -1);
       most = std::max(most, s.cnt);
     }
-  if (!early) cudaFuncSetAttribute(k_q2_tile<SSC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmem);
-  launch_pdl(early, k_q2_tile<SSC>, dim3((unsigned)((most + kTileRows - 1) / kTileRows), 8, SSC ? 27 : 1), kTileT,
+  if (col == 0) cudaFuncSetAttribute(k_q2_tile<SSC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmem);
+  launch_early(k_q2_tile<SSC>, dim3((unsigned)((most + kTileRows - 1) / kTileRows), 8, SSC ? 27 : 1), kTileT,
              kTileSmem, st, L.A, L.Np, M, col, L.dmask, damp, L.omega, x, b, r, lay);
 }
 
@@ -823,6 +800,8 @@ __global__ void __launch_bounds__(kQ2T)
 k_sor_q2(const double* __restrict__ A, long long Np, int M, int colour, double omega_s,
          const double* __restrict__ omega, double* x, const double* b, double* r,
          const __grid_constant__ Q2Layout lay) {
+  pdl_next();
+  pdl_wait();
   sor_q2_block<D, 0>(A, Np, M, colour, blockIdx.x, omega_s, omega, x, b, r, lay);
 }
 
@@ -831,6 +810,8 @@ template <int D, bool RES>
 __global__ void __launch_bounds__(kQ2T, kQ2MinBlocks<D>)
 k_spmv_q2c(const double* __restrict__ A, long long Np, int M, const double* __restrict__ x, const double* b,
            double* y, const __grid_constant__ Q2Layout lay) {
+  pdl_next();
+  pdl_wait();
   int pat;
   Q2Sub sub;
   long long u;
@@ -849,6 +830,8 @@ __global__ void __launch_bounds__(kQ2T, kQ2MinBlocks<D>)
 k_jacobi_res_q2c(const double* __restrict__ A, long long Np, int M, double damp, const double* __restrict__ omega,
                  const double* __restrict__ x, const double* b, double* __restrict__ xout, double* r, int write_r,
                  const __grid_constant__ Q2Layout lay) {
+  pdl_next();
+  pdl_wait();
   int pat;
   Q2Sub sub;
   long long u;
@@ -869,7 +852,9 @@ k_jacobi_res_q2c(const double* __restrict__ A, long long Np, int M, double damp,
 // <jacobi> step with an up-to-date residual: t = r/d, x += w t, r := t
 __global__ void __launch_bounds__(kBlock)
 k_jacobi(const double* __restrict__ Dg, long long N, double damp, const double* __restrict__ omega,
-         double* x, double* r, int write_r, long long vs = 0, long long as = 0) {
+         double* x, double* r, int write_r, long long vs, long long as) {
+  pdl_next();
+  pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   const long long bq = blockIdx.y;  // problem of a batched level: vector stride vs, matrix stride as
@@ -889,9 +874,10 @@ k_jacobi(const double* __restrict__ Dg, long long N, double damp, const double* 
 // node -- the same update, with r keeping the unscaled residual
 // (blockit.lisp:131-138) instead of the <sor> correction (linit.lisp:312-322)
 template <int D, int P, bool SSC = false>
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kRowT, kRowMinBlocks)
 k_sor_colour(const double* __restrict__ A, long long N, long long Np, long long M, int colour,
              double omega_s, const double* __restrict__ omega, double* x, const double* b, double* r) {
+  pdl_next();
   constexpr int NS = St<D, P>::NS;
   constexpr int C = St<D, P>::CENTER;
   constexpr int Q = P + 1;
@@ -905,18 +891,22 @@ k_sor_colour(const double* __restrict__ A, long long N, long long Np, long long 
   const unsigned tq = tu / nxu;
   const long long jx = tu - tq * nxu, jy = tq % nyu, jz = tq / nyu;
   const long long i = (cx + Q * jx) + M * ((D > 1 ? cy + Q * jy : 0) + M * (D > 2 ? cz + Q * jz : 0));
-  double s = 0.0, d = 1.0;
+  // coefficients and damping do not depend on the previous launch
+  double av[NS], xv[NS];
 #pragma unroll
-  for (int k = 0; k < NS; ++k) {
-    const long long o = slot_off<D, P>(k, M);
-    const double a = A[(long long)k * Np + i];
-    if (k == C) d = a;
-    s = fma(a, x[clampi(i + o, N)], s);
-  }
+  for (int k = 0; k < NS; ++k) av[k] = __ldg(A + (long long)k * Np + i);
+  const double w = omega ? __ldg(omega + i) : omega_s;
+  pdl_wait();
+#pragma unroll
+  for (int k = 0; k < NS; ++k) xv[k] = x[clampi(i + slot_off<D, P>(k, M), N)];
+  double s = 0.0;
+  const double d = av[C];
+#pragma unroll
+  for (int k = 0; k < NS; ++k) s = fma(av[k], xv[k], s);
   const double rr = b[i] - s;
   const double tt = rr / d;
   r[i] = SSC ? rr : tt;
-  x[i] = fma(omega ? omega[i] : omega_s, tt, x[i]);
+  x[i] = fma(w, tt, xv[C]);
 }
 
 // Step K of the warp's LU factorisation of a vertex block (rows in lanes):
@@ -1182,6 +1172,8 @@ k_ssc_solve_q2(int Mi, int dmask, int colour, double omega, double* x, const dou
 template <int D>
 __global__ void __launch_bounds__(kBlock)
 k_psc_q1(const double* __restrict__ A, long long N, long long Np, double damp, double* x, const double* r) {
+  pdl_next();
+  pdl_wait();
   constexpr int C = St<D, 1>::CENTER;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
@@ -1196,6 +1188,8 @@ template <int D>
 __global__ void __launch_bounds__(128, 6)
 k_psc_block_q2(long long M, int dmask, const double* __restrict__ r, const double* __restrict__ F,
                const unsigned char* __restrict__ P, double* __restrict__ C) {
+  pdl_next();
+  pdl_wait();
   constexpr int NB = D == 1 ? 3 : (D == 2 ? 9 : 27);
   const int lane = threadIdx.x & 31;
   const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // uniform per warp
@@ -1223,6 +1217,8 @@ k_psc_block_q2(long long M, int dmask, const double* __restrict__ r, const doubl
 template <int D>
 __global__ void __launch_bounds__(kBlock)
 k_psc_gather_q2(long long N, long long M, int dmask, double damp, const double* __restrict__ C, double* x) {
+  pdl_next();
+  pdl_wait();
   constexpr int NB = D == 1 ? 3 : (D == 2 ? 9 : 27);
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
@@ -1270,28 +1266,68 @@ k_psc_gather_q2(long long N, long long M, int dmask, double damp, const double* 
 // order in which the stencil forms sum their slots, so a structured level
 // given as compressed rows yields the structured results bit for bit.
 
+// The row sums fetch eight entries at a time -- indices and values, then the
+// unknowns -- so a row of up to eight entries waits for memory twice (entry by
+// entry it was twice per few entries), and the first eight are fetched while
+// the previous launch still runs.  ROX: x by the read-only path (a sweep that
+// updates x in place reads it plainly).  Every caller's thread passes pdl_wait
+// here.
+template <bool ROX>
+__device__ __forceinline__ double csr_row_sum(const CsrView& a, long long i, const double* x) {
+  constexpr int K = 8;
+  const long long e1 = a.start[i + 1];
+  long long e = a.start[i];
+  int ix[K];
+  double v[K];
+  auto fetch = [&]() {
+#pragma unroll
+    for (int q = 0; q < K; ++q)
+      if (e + q < e1) {
+        ix[q] = __ldg(a.index + e + q);
+        v[q] = __ldg(a.value + e + q);
+      }
+  };
+  fetch();
+  pdl_wait();
+  double s = 0.0;
+  while (e < e1) {
+    double xv[K];
+#pragma unroll
+    for (int q = 0; q < K; ++q)
+      if (e + q < e1) xv[q] = ROX ? __ldg(x + ix[q]) : x[ix[q]];
+#pragma unroll
+    for (int q = 0; q < K; ++q)
+      if (e + q < e1) s = fma(v[q], xv[q], s);
+    e += K;
+    if (e < e1) fetch();
+  }
+  return s;
+}
+constexpr int kCsrT = 64;  // threads per block of the compressed-row kernels: small levels spread over more SMs
+
 // y = A x, or r = b - A x (b may alias r)
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kCsrT, 8)
 k_csr_spmv(long long N, CsrView a, const double* __restrict__ x, const double* b, double* y, int res) {
+  pdl_next();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  double s = 0.0;
-  for (long long e = a.start[i]; e < a.start[i + 1]; ++e) s = fma(a.value[e], __ldg(x + a.index[e]), s);
+  const double s = csr_row_sum<true>(a, i, x);
   y[i] = res ? b[i] - s : s;
 }
 
-// compute-residual fused with the following <jacobi> step (as k_jacobi_res)
-__global__ void __launch_bounds__(kBlock)
+// compute-residual fused with the following <jacobi> step (as k_row_jacobi_q1)
+__global__ void __launch_bounds__(kCsrT, 8)
 k_csr_jacobi_res(long long N, CsrView a, const double* __restrict__ diag, double damp,
                  const double* __restrict__ omega, const double* __restrict__ x, const double* b,
                  double* __restrict__ xout, double* r, int write_r) {
+  pdl_next();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  double s = 0.0;
-  for (long long e = a.start[i]; e < a.start[i + 1]; ++e) s = fma(a.value[e], __ldg(x + a.index[e]), s);
-  const double t = (b[i] - s) / diag[i];
+  const double d = __ldg(diag + i), w = omega ? __ldg(omega + i) : damp;
+  const double s = csr_row_sum<true>(a, i, x);
+  const double t = (b[i] - s) / d;
   if (write_r) r[i] = t;
-  xout[i] = fma(omega ? omega[i] : damp, t, x[i]);
+  xout[i] = fma(w, t, x[i]);
 }
 
 // one colour of the SOR (SSC = false: r := the scaled correction, the
@@ -1299,40 +1335,44 @@ k_csr_jacobi_res(long long N, CsrView a, const double* __restrict__ diag, double
 // blockit.lisp:131-138) of an algebraic level: rows of the colour in any
 // order (they couple to none of each other), the row sum over the stored
 // entries, columns ascending
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kCsrT, 8)
 k_csr_sor(const int* __restrict__ rows, long long cnt, CsrView a, const double* __restrict__ diag, double omega_s,
           const double* __restrict__ omega, double* x, const double* b, double* r, int ssc) {
+  pdl_next();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= cnt) return;
-  const long long i = rows[t];
-  double s = 0.0;
-  for (long long e = a.start[i]; e < a.start[i + 1]; ++e) s = fma(a.value[e], x[a.index[e]], s);
+  const long long i = __ldg(rows + t);
+  const double d = __ldg(diag + i), w = omega ? __ldg(omega + i) : omega_s;
+  const double s = csr_row_sum<false>(a, i, x);
   const double rr = b[i] - s;
-  const double tt = rr / diag[i];
+  const double tt = rr / d;
   r[i] = ssc ? rr : tt;
-  x[i] = fma(omega ? omega[i] : omega_s, tt, x[i]);
+  x[i] = fma(w, tt, x[i]);
 }
 
 // rc = I^T rf row by row of I^T (fine entries ascending); the coarse rhs
 // takes rc, the coarse solution 0 (the :after methods of restrict)
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kCsrT, 8)
 k_csr_restrict(long long NC, CsrView pt, const double* __restrict__ rf, double* rc, double* rhsc, double* solc) {
+  pdl_next();
   const long long J = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (J >= NC) return;
-  double s = 0.0;
-  for (long long e = pt.start[J]; e < pt.start[J + 1]; ++e) s = fma(pt.value[e], __ldg(rf + pt.index[e]), s);
+  const double s = csr_row_sum<true>(pt, J, rf);
   rc[J] = s;
   if (rhsc) rhsc[J] = s;
   if (solc) solc[J] = 0.0;
 }
 
 // xf += I xc (coarse entries ascending)
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kCsrT, 8)
 k_csr_prolong(long long NF, CsrView p, const double* __restrict__ xc, double* xf) {
+  pdl_next();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= NF || p.start[i] == p.start[i + 1]) return;  // constrained rows keep their value
-  double s = 0.0;
-  for (long long e = p.start[i]; e < p.start[i + 1]; ++e) s = fma(p.value[e], __ldg(xc + p.index[e]), s);
+  if (i >= NF || p.start[i] == p.start[i + 1]) {  // constrained rows keep their value
+    pdl_wait();  // (were all rows empty, the launch would otherwise end before its predecessor)
+    return;
+  }
+  const double s = csr_row_sum<true>(p, i, xc);
   xf[i] = xf[i] + s;
 }
 
@@ -1482,7 +1522,9 @@ __device__ __forceinline__ T prolong_node(const int fi[3], int MF, int MC, int d
 template <int D, int P>
 __global__ void __launch_bounds__(kBlock)
 k_restrict(int MC, int MF, int dmask, const double* __restrict__ rf, double* __restrict__ rc,
-           double* __restrict__ rhsc, double* __restrict__ solc, long long fs = 0, long long cs = 0) {
+           double* __restrict__ rhsc, double* __restrict__ solc, long long fs, long long cs) {
+  pdl_next();
+  pdl_wait();
   if (D == 1 && threadIdx.y != 0) return;
   if (D < 3) {  // problem of a batched level: fine stride fs, coarse stride cs
     const long long bq = blockIdx.z;
@@ -1504,8 +1546,10 @@ k_restrict(int MC, int MF, int dmask, const double* __restrict__ rf, double* __r
 // xf := xf + I xc (constrained) (prolongate, multigrid.lisp:237-239)
 template <int D, int P>
 __global__ void __launch_bounds__(kBlock)
-k_prolong(int MF, int MC, int dmask, const double* __restrict__ xc, double* __restrict__ xf, long long fs = 0,
-          long long cs = 0) {
+k_prolong(int MF, int MC, int dmask, const double* __restrict__ xc, double* __restrict__ xf, long long fs,
+          long long cs) {
+  pdl_next();
+  pdl_wait();
   if (D == 1 && threadIdx.y != 0) return;
   if (D < 3) {  // problem of a batched level
     const long long bq = blockIdx.z;
@@ -1809,7 +1853,9 @@ k_coarse_solve(const double* __restrict__ AinvT, int n, double damp, double* x, 
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
+  pdl_next();
   if (warp >= R) request(0);
+  pdl_wait();
   for (int j = threadIdx.x; j < n; j += blockDim.x) rs[j] = r[j];
   if (cs > 1) cooperative_groups::this_cluster().sync();
   double acc = 0.0;
@@ -1845,11 +1891,15 @@ k_coarse_solve(const double* __restrict__ AinvT, int n, double damp, double* x, 
 
 // ------------------------------------------------------------ vector ops
 __global__ void k_fill(double* x, long long n, double v) {
+  pdl_next();
+  pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) x[i] = v;
 }
 
 __global__ void k_copy(const double* __restrict__ x, double* __restrict__ y, long long n) {
+  pdl_next();
+  pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) y[i] = x[i];
 }
@@ -1857,6 +1907,8 @@ __global__ void k_copy(const double* __restrict__ x, double* __restrict__ y, lon
 // axpy!: y := y + alpha x (alpha from a device slot when aslot >= 0)
 __global__ void k_axpy(double alpha, const double* __restrict__ sc, int aslot, const double* __restrict__ x,
                        double* y, long long n) {
+  pdl_next();
+  pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double a = aslot >= 0 ? sc[aslot] : alpha;
@@ -1865,7 +1917,9 @@ __global__ void k_axpy(double alpha, const double* __restrict__ sc, int aslot, c
 
 // DR4096 dot product (x, y)
 __global__ void __launch_bounds__(kBlock)
-k_dot(const double* __restrict__ x, const double* __restrict__ y, long long n, Reduce R, long long vs = 0) {
+k_dot(const double* __restrict__ x, const double* __restrict__ y, long long n, Reduce R, long long vs) {
+  pdl_next();
+  pdl_wait();
   __shared__ double smem[8];
   const long long bq = blockIdx.y;  // problem of a batched vector (stride vs)
   x += bq * vs;
@@ -1887,8 +1941,10 @@ k_dot(const double* __restrict__ x, const double* __restrict__ y, long long n, R
 __global__ void __launch_bounds__(kBlock)
 k_cg_update(const double* __restrict__ sc, double* __restrict__ x, const double* __restrict__ p,
             double* __restrict__ r, const double* __restrict__ a, double* __restrict__ w,
-            double* __restrict__ w2, double* __restrict__ q, long long n, Reduce R, long long vs = 0,
-            const double* __restrict__ frozen = nullptr) {
+            double* __restrict__ w2, double* __restrict__ q, long long n, Reduce R, long long vs,
+            const double* __restrict__ frozen) {
+  pdl_next();
+  pdl_wait();
   __shared__ double smem[8];
   const long long bq = blockIdx.y;  // problem of a batched vector (stride vs); frozen: it has converged
   sc += bq * S_COUNT;
@@ -1927,7 +1983,9 @@ k_cg_update(const double* __restrict__ sc, double* __restrict__ x, const double*
 
 // p := (new_alpha/alpha) p (scal!), then p := p + q (m+!)
 __global__ void k_p_update(const double* __restrict__ sc, double* __restrict__ p, const double* __restrict__ q,
-                           long long n, long long vs = 0, const double* __restrict__ frozen = nullptr) {
+                           long long n, long long vs, const double* __restrict__ frozen) {
+  pdl_next();
+  pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const long long bq = blockIdx.y;  // problem of a batched vector; frozen problems keep p
@@ -2230,6 +2288,7 @@ template <int P, typename T, int OP>
 __global__ void __launch_bounds__(kRow3T, sizeof(T) == 8 ? 3 : 4)
 k_row3(const T* __restrict__ A, int N, long long Np, int M, double damp, const double* __restrict__ omega,
        const T* __restrict__ x, const T* b, T* y, T* r, int write_r) {
+  pdl_next();
   constexpr int W = 2 * P + 1, Q = W * W, SEG = 3 * (kRow3Nodes + 2 * P);
   extern __shared__ unsigned char row3_sm[];
   T* xs = reinterpret_cast<T*>(row3_sm);  // [slot row][node - i0 + P][component]
@@ -2265,6 +2324,7 @@ k_row3(const T* __restrict__ A, int N, long long Np, int M, double damp, const d
     }
   };
   load(0, cur);
+  pdl_wait();
   // the unknowns, nine loads at a time
   constexpr int PER = (Q * SEG + kRow3T - 1) / kRow3T, BATCH = 9;
 #pragma unroll 1
@@ -2345,6 +2405,8 @@ template <int P, typename T, int OP>
 __global__ void __launch_bounds__(kRow3Nodes, 8)
 k_node3(const T* __restrict__ A, int N, long long Np, int M, double damp, const double* __restrict__ omega,
         const T* __restrict__ x, const T* b, T* y, T* r, int write_r) {
+  pdl_next();
+  pdl_wait();
   constexpr int W = 2 * P + 1, Q = W * W, SEG = 3 * (kRow3Nodes + 2 * P);
   extern __shared__ unsigned char row3_sm[];
   T* xs = reinterpret_cast<T*>(row3_sm);  // [slot row][node - i0 + P][component]
@@ -2442,15 +2504,14 @@ static void launch_row3(int order, const T* A, long long N, long long Np, long l
     const unsigned grid = (unsigned)((N + kRow3Nodes - 1) / kRow3Nodes);
     if constexpr (sizeof(T) == 4) {
       if (N >= kNode3Min) {
-        k_node3<P, T, OP><<<grid, kRow3Nodes, smem, st>>>(A, (int)N, Np, (int)M, damp, omega, x, b, y, r,
+        launch_late(k_node3<P, T, OP>, grid, kRow3Nodes, smem, st, A, (int)N, Np, (int)M, damp, omega, x, b, y, r,
                                                           write_r ? 1 : 0);
         return;
       }
     }
     if (smem > 48 * 1024)
       cudaFuncSetAttribute(k_row3<P, T, OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_row3<P, T, OP><<<grid, kRow3T, smem, st>>>(
-        A, (int)N, Np, (int)M, damp, omega, x, b, y, r, write_r ? 1 : 0);
+    launch_late(k_row3<P, T, OP>, grid, kRow3T, smem, st, A, (int)N, Np, (int)M, damp, omega, x, b, y, r, write_r ? 1 : 0);
   };
   if (order == 2) go(std::integral_constant<int, 2>{});
   else go(std::integral_constant<int, 1>{});
@@ -2460,6 +2521,8 @@ static void launch_row3(int order, const T* A, long long N, long long Np, long l
 __global__ void __launch_bounds__(kBlock)
 k_jacobi3(const double* __restrict__ A, long long N, long long Np, int center, double damp,
           const double* __restrict__ omega, double* x, double* r, int write_r) {
+  pdl_next();
+  pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   double B[9], t[3];
@@ -2540,6 +2603,8 @@ template <int P, bool LOOP, typename T = double>
 __global__ void __launch_bounds__(kBlock)
 k_restrict3(int MC, int MF, int dmask, const T* __restrict__ rf, T* __restrict__ rc,
             T* __restrict__ rhsc, T* __restrict__ solc) {
+  pdl_next();
+  pdl_wait();
   constexpr int CT = LOOP ? 3 : 1;
   const int xs = blockIdx.x * 32 + threadIdx.x, c0 = LOOP ? 0 : xs % 3;
   const int cJ[3] = {LOOP ? xs : xs / 3, (int)(blockIdx.y * 8 + threadIdx.y), (int)blockIdx.z};
@@ -2560,6 +2625,8 @@ k_restrict3(int MC, int MF, int dmask, const T* __restrict__ rf, T* __restrict__
 template <int P, bool LOOP, typename T = double>
 __global__ void __launch_bounds__(kBlock)
 k_prolong3(int MF, int MC, int dmask, const T* __restrict__ xc, T* __restrict__ xf) {
+  pdl_next();
+  pdl_wait();
   constexpr int CT = LOOP ? 3 : 1;
   const int xs = blockIdx.x * 32 + threadIdx.x, c0 = LOOP ? 0 : xs % 3;
   const int fi[3] = {LOOP ? xs : xs / 3, (int)(blockIdx.y * 8 + threadIdx.y), (int)blockIdx.z};
@@ -2581,10 +2648,10 @@ static void launch_restrict3(int order, long long MC, long long MF, int dmask, c
   const bool big = MC * MC * MC >= kXferLoopMin;
   const dim3 g((unsigned)(((big ? 1 : 3) * MC + 31) / 32), (unsigned)((MC + 7) / 8), (unsigned)MC), t(32, 8);
   const int mc = (int)MC, mf = (int)MF;
-  if (order == 2 && big) k_restrict3<2, true, T><<<g, t, 0, st>>>(mc, mf, dmask, rf, rc, rhsc, solc);
-  else if (order == 2) k_restrict3<2, false, T><<<g, t, 0, st>>>(mc, mf, dmask, rf, rc, rhsc, solc);
-  else if (big) k_restrict3<1, true, T><<<g, t, 0, st>>>(mc, mf, dmask, rf, rc, rhsc, solc);
-  else k_restrict3<1, false, T><<<g, t, 0, st>>>(mc, mf, dmask, rf, rc, rhsc, solc);
+  if (order == 2 && big) launch_pdl(k_restrict3<2, true, T>, g, t, 0, st, mc, mf, dmask, rf, rc, rhsc, solc);
+  else if (order == 2) launch_pdl(k_restrict3<2, false, T>, g, t, 0, st, mc, mf, dmask, rf, rc, rhsc, solc);
+  else if (big) launch_pdl(k_restrict3<1, true, T>, g, t, 0, st, mc, mf, dmask, rf, rc, rhsc, solc);
+  else launch_pdl(k_restrict3<1, false, T>, g, t, 0, st, mc, mf, dmask, rf, rc, rhsc, solc);
 }
 
 template <typename T>
@@ -2592,10 +2659,10 @@ static void launch_prolong3(int order, long long MF, long long MC, int dmask, co
   const bool big = MF * MF * MF >= kXferLoopMin;
   const dim3 g((unsigned)(((big ? 1 : 3) * MF + 31) / 32), (unsigned)((MF + 7) / 8), (unsigned)MF), t(32, 8);
   const int mc = (int)MC, mf = (int)MF;
-  if (order == 2 && big) k_prolong3<2, true, T><<<g, t, 0, st>>>(mf, mc, dmask, xc, xf);
-  else if (order == 2) k_prolong3<2, false, T><<<g, t, 0, st>>>(mf, mc, dmask, xc, xf);
-  else if (big) k_prolong3<1, true, T><<<g, t, 0, st>>>(mf, mc, dmask, xc, xf);
-  else k_prolong3<1, false, T><<<g, t, 0, st>>>(mf, mc, dmask, xc, xf);
+  if (order == 2 && big) launch_pdl(k_prolong3<2, true, T>, g, t, 0, st, mf, mc, dmask, xc, xf);
+  else if (order == 2) launch_pdl(k_prolong3<2, false, T>, g, t, 0, st, mf, mc, dmask, xc, xf);
+  else if (big) launch_pdl(k_prolong3<1, true, T>, g, t, 0, st, mf, mc, dmask, xc, xf);
+  else launch_pdl(k_prolong3<1, false, T>, g, t, 0, st, mf, mc, dmask, xc, xf);
 }
 
 // Elasticity stiffness by gather (the vector form of k_assemble): for node i,
@@ -2876,6 +2943,8 @@ k_galerkin(const double* __restrict__ AF, long long NpF, int MF, double* __restr
 __global__ void __launch_bounds__(kBlock)
 k_bdiag3(const double* __restrict__ A, long long N, long long Np, int center, int mode,
          const double* __restrict__ w, const double* __restrict__ x, double* __restrict__ y) {
+  pdl_next();
+  pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   double B[9], t[3];
@@ -2894,6 +2963,8 @@ k_bdiag3(const double* __restrict__ A, long long N, long long Np, int center, in
 // y = x + w .* v with w per node (y may be x)
 __global__ void k_xpwv3(const double* x, const double* __restrict__ w, const double* __restrict__ v, double* y,
                         long long N) {
+  pdl_next();
+  pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
 #pragma unroll
@@ -2903,6 +2974,8 @@ __global__ void k_xpwv3(const double* x, const double* __restrict__ w, const dou
 // acc_i += sum_k a_ik b_ik (per-node dot of two vectors)
 __global__ void k_acc_prod3(double* __restrict__ acc, const double* __restrict__ a, const double* __restrict__ b,
                             long long N) {
+  pdl_next();
+  pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   double s = a[3 * i] * b[3 * i];
@@ -2917,6 +2990,8 @@ template <typename T>
 __global__ void __launch_bounds__(kBlock)
 k_jacobi0_3(const T* __restrict__ A, long long N, long long Np, int center, float damp,
             const double* __restrict__ omega, const T* __restrict__ b, T* __restrict__ x) {
+  pdl_next();
+  pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   T B[9], t[3];
@@ -2933,6 +3008,8 @@ k_jacobi0_3(const T* __restrict__ A, long long N, long long Np, int center, floa
 template <typename TI, typename TO>
 __global__ void k_vscale(const TI* __restrict__ x, const double* __restrict__ sc, int slot, int mode,
                          TO* __restrict__ y, long long n) {
+  pdl_next();
+  pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double f = 1.0;
@@ -2945,6 +3022,8 @@ __global__ void k_vscale(const TI* __restrict__ x, const double* __restrict__ sc
 
 // the FCG(1) coefficient beta = -(z, a) / (p, a) of the previous step (0 on a restart)
 __global__ void k_fcg_beta(double* sc, int first) {
+  pdl_next();
+  pdl_wait();
   sc[S_RATIO] = first ? 0.0 : -sc[S_TMP] / sc[S_BETA];
 }
 
@@ -2984,7 +3063,7 @@ void launch_spmv(const LevelView& L, const double* x, const double* b, double* y
                  const Reduce* R, cudaStream_t st) {
   if (L.csr) {  // the reduction as a separate DR4096 pass
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    k_csr_spmv<<<grid1(L.N), kBlock, 0, st>>>(L.N, L.a, x, b, y, b ? 1 : 0);
+    launch_early(k_csr_spmv, grid1(L.N, kCsrT), kCsrT, 0, st, L.N, L.a, x, b, y, b ? 1 : 0);
     if (dv) launch_dot(y, dv, L.N, *R, st);
     return;
   }
@@ -3000,16 +3079,16 @@ void launch_spmv(const LevelView& L, const double* x, const double* b, double* y
     const Q2Layout lay = q2_layout(L.dim, L.M);
     Q2_DISPATCH(L.dim, {
       const dim3 g = q2_grid<D>((int)L.M);
-      if (b) k_spmv_q2c<D, true><<<g, kQ2T, 0, st>>>(L.A, L.Np, (int)L.M, x, b, y, lay);
-      else k_spmv_q2c<D, false><<<g, kQ2T, 0, st>>>(L.A, L.Np, (int)L.M, x, b, y, lay);
+      if (b) launch_pdl(k_spmv_q2c<D, true>, g, kQ2T, 0, st, L.A, L.Np, (int)L.M, x, b, y, lay);
+      else launch_pdl(k_spmv_q2c<D, false>, g, kQ2T, 0, st, L.A, L.Np, (int)L.M, x, b, y, lay);
     });
     if (dv) launch_dot(y, dv, L.N, *R, st);
     return;
   }
   const dim3 g(grid1(L.N, kRowT), (unsigned)L.nb);
   Q1_DISPATCH(L.dim, {
-    if (b) k_row_q1<D, true><<<g, kRowT, 0, st>>>(L.A, (int)L.N, L.Np, (int)L.M, x, b, y);
-    else k_row_q1<D, false><<<g, kRowT, 0, st>>>(L.A, (int)L.N, L.Np, (int)L.M, x, b, y);
+    if (b) launch_early(k_row_q1<D, true>, g, kRowT, 0, st, L.A, (int)L.N, L.Np, (int)L.M, x, b, y);
+    else launch_early(k_row_q1<D, false>, g, kRowT, 0, st, L.A, (int)L.N, L.Np, (int)L.M, x, b, y);
   });
   if (dv) launch_dot_b(y, dv, L.N, L.Np, L.nb, *R, st);
 }
@@ -3017,24 +3096,24 @@ void launch_spmv(const LevelView& L, const double* x, const double* b, double* y
 void launch_jacobi(const LevelView& L, double damp, double* x, double* r, bool write_r, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
   if (L.csr) {
-    k_jacobi<<<grid1(L.N), kBlock, 0, st>>>(L.diag, L.N, damp, L.omega, x, r, write_r ? 1 : 0);
+    launch_early(k_jacobi, grid1(L.N), kBlock, 0, st, L.diag, L.N, damp, L.omega, x, r, write_r ? 1 : 0, 0, 0);
     return;
   }
   if (L.nc == 3) {
-    k_jacobi3<<<grid1(L.N), kBlock, 0, st>>>(L.A, L.N, L.Np, L.center, damp, L.omega, x, r, write_r ? 1 : 0);
+    launch_early(k_jacobi3, grid1(L.N), kBlock, 0, st, L.A, L.N, L.Np, L.center, damp, L.omega, x, r, write_r ? 1 : 0);
     return;
   }
   if (L.order == 2) {  // colour-major sliced storage
     const Q2Layout lay = q2_layout(L.dim, L.M);
     Q2_DISPATCH(L.dim, {
-      k_jacobi_q2<D><<<grid1(L.N), kBlock, 0, st>>>(L.A, L.N, L.Np, L.M, damp, L.omega, x, r, write_r ? 1 : 0, lay);
+      launch_early(k_jacobi_q2<D>, grid1(L.N), kBlock, 0, st, L.A, L.N, L.Np, L.M, damp, L.omega, x, r, write_r ? 1 : 0, lay);
     });
     return;
   }
   const double* Dg = L.A + (long long)L.center * L.Np;
   long long ns = 1;
   for (int k = 0; k < L.dim; ++k) ns *= 3;
-  k_jacobi<<<dim3(grid1(L.N), (unsigned)L.nb), kBlock, 0, st>>>(Dg, L.N, damp, L.omega, x, r, write_r ? 1 : 0,
+  launch_early(k_jacobi, dim3(grid1(L.N), (unsigned)L.nb), kBlock, 0, st, Dg, L.N, damp, L.omega, x, r, write_r ? 1 : 0,
                                                                 L.Np, ns * L.Np);
 }
 
@@ -3042,7 +3121,7 @@ void launch_jacobi_res(const LevelView& L, double damp, const double* x, const d
                        double* r, bool write_r, const double* dv, const Reduce* R, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
   if (L.csr) {
-    k_csr_jacobi_res<<<grid1(L.N), kBlock, 0, st>>>(L.N, L.a, L.diag, damp, L.omega, x, b, xout, r,
+    launch_early(k_csr_jacobi_res, grid1(L.N, kCsrT), kCsrT, 0, st, L.N, L.a, L.diag, damp, L.omega, x, b, xout, r,
                                                       write_r ? 1 : 0);
     if (dv) launch_dot(xout, dv, L.N, *R, st);
     return;
@@ -3055,7 +3134,7 @@ void launch_jacobi_res(const LevelView& L, double damp, const double* x, const d
   if (L.order == 2) {  // rows by colour class and parity
     const Q2Layout lay = q2_layout(L.dim, L.M);
     Q2_DISPATCH(L.dim, {
-      k_jacobi_res_q2c<D><<<q2_grid<D>((int)L.M), kQ2T, 0, st>>>(L.A, L.Np, (int)L.M, damp, L.omega, x, b, xout, r,
+      launch_pdl(k_jacobi_res_q2c<D>, q2_grid<D>((int)L.M), kQ2T, 0, st, L.A, L.Np, (int)L.M, damp, L.omega, x, b, xout, r,
                                                                  write_r ? 1 : 0, lay);
     });
     if (dv) launch_dot(xout, dv, L.N, *R, st);
@@ -3063,7 +3142,7 @@ void launch_jacobi_res(const LevelView& L, double damp, const double* x, const d
   }
   const dim3 g(grid1(L.N, kRowT), (unsigned)L.nb);
   Q1_DISPATCH(L.dim, {
-    k_row_jacobi_q1<D><<<g, kRowT, 0, st>>>(L.A, (int)L.N, L.Np, (int)L.M, damp, L.omega, x, b, xout, r,
+    launch_early(k_row_jacobi_q1<D>, g, kRowT, 0, st, L.A, (int)L.N, L.Np, (int)L.M, damp, L.omega, x, b, xout, r,
                                             write_r ? 1 : 0);
   });
   if (dv) launch_dot_b(xout, dv, L.N, L.Np, L.nb, *R, st);
@@ -3075,7 +3154,7 @@ static void launch_csr_sor(const LevelView& L, double omega, const double* om, d
   for (int c = 0; c < L.ncol; ++c) {
     const long long cnt = L.coff[c + 1] - L.coff[c];
     if (cnt > 0)
-      k_csr_sor<<<grid1(cnt), kBlock, 0, st>>>(L.crow + L.coff[c], cnt, L.a, L.diag, omega, om, x, b, r, ssc ? 1 : 0);
+      launch_early(k_csr_sor, grid1(cnt, kCsrT), kCsrT, 0, st, L.crow + L.coff[c], cnt, L.a, L.diag, omega, om, x, b, r, ssc ? 1 : 0);
   }
 }
 
@@ -3096,15 +3175,15 @@ void launch_sor(const LevelView& L, double omega, double* x, const double* b, do
     if (L.dim > 1) cnt *= (L.M - cy + Q - 1) / Q;
     if (L.dim > 2) cnt *= (L.M - cz + Q - 1) / Q;
     if (tile) {
-      launch_q2_tile<false>(L, col, col > 0, omega, x, b, r, lay, st);
+      launch_q2_tile<false>(L, col, omega, x, b, r, lay, st);
     } else if (L.order == 2) {
       Q2_DISPATCH(L.dim, {
         const unsigned nb = (unsigned)q2_class_blocks<D>((int)L.M, col);
-        if (nb) k_sor_q2<D><<<nb, kQ2T, 0, st>>>(L.A, L.Np, (int)L.M, col, omega, L.omega, x, b, r, lay);
+        if (nb) launch_pdl(k_sor_q2<D>, nb, kQ2T, 0, st, L.A, L.Np, (int)L.M, col, omega, L.omega, x, b, r, lay);
       });
     } else {
       Q1_DISPATCH(L.dim, {
-        k_sor_colour<D, 1><<<grid1(cnt), kBlock, 0, st>>>(L.A, L.N, L.Np, L.M, col, omega, L.omega, x, b, r);
+        launch_early(k_sor_colour<D, 1>, grid1(cnt, kRowT), kRowT, 0, st, L.A, L.N, L.Np, L.M, col, omega, L.omega, x, b, r);
       });
     }
   }
@@ -3142,7 +3221,7 @@ void launch_ssc(const LevelView& L, double omega, double* x, const double* b, do
       if (L.dim > 1) cnt *= (L.M - cy + 1) / 2;
       if (L.dim > 2) cnt *= (L.M - cz + 1) / 2;
       Q1_DISPATCH(L.dim, {
-        k_sor_colour<D, 1, true><<<grid1(cnt), kBlock, 0, st>>>(L.A, L.N, L.Np, L.M, col, omega, nullptr, x, b, r);
+        launch_early(k_sor_colour<D, 1, true>, grid1(cnt, kRowT), kRowT, 0, st, L.A, L.N, L.Np, L.M, col, omega, nullptr, x, b, r);
       });
     }
     return;
@@ -3159,11 +3238,11 @@ void launch_ssc(const LevelView& L, double omega, double* x, const double* b, do
     const unsigned grid = (unsigned)((cnt * 32 + 127) / 128);
     Q2_DISPATCH(L.dim, {
       if (tile)
-        launch_q2_tile<true>(L, col, col > 0, 0.0, x, b, r, lay, st);
+        launch_q2_tile<true>(L, col, 0.0, x, b, r, lay, st);
       else
-        launch_pdl(col > 0, k_ssc_res_q2<D>, q2_grid<D>((int)L.M, col), kQ2T, 0, st, L.A, L.Np, (int)L.M, col, L.dmask,
+        launch_pdl(k_ssc_res_q2<D>, q2_grid<D>((int)L.M, col), kQ2T, 0, st, L.A, L.Np, (int)L.M, col, L.dmask,
                    x, b, r, lay);
-      launch_pdl(true, k_ssc_solve_q2<D>, dim3(grid), 128, 0, st, (int)L.M, L.dmask, col, omega, x, r, F, P);
+      launch_early(k_ssc_solve_q2<D>, dim3(grid), 128, 0, st, (int)L.M, L.dmask, col, omega, x, r, F, P);
     });
   }
 }
@@ -3172,14 +3251,14 @@ void launch_psc(const LevelView& L, double damp, double* x, const double* r, con
                 const unsigned char* P, double* C, cudaStream_t st) {
   if (L.order == 1) {  // one-node blocks: x_i += damp r_i / a_ii, r unchanged
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    Q1_DISPATCH(L.dim, { k_psc_q1<D><<<grid1(L.N), kBlock, 0, st>>>(L.A, L.N, L.Np, damp, x, r); });
+    Q1_DISPATCH(L.dim, { launch_pdl(k_psc_q1<D>, grid1(L.N), kBlock, 0, st, L.A, L.N, L.Np, damp, x, r); });
     return;
   }
   g_launches.fetch_add(2, std::memory_order_relaxed);
   const unsigned grid = (unsigned)((ssc_blocks(L) * 32 + 127) / 128);
   Q2_DISPATCH(L.dim, {
-    k_psc_block_q2<D><<<grid, 128, 0, st>>>(L.M, L.dmask, r, F, P, C);
-    k_psc_gather_q2<D><<<grid1(L.N), kBlock, 0, st>>>(L.N, L.M, L.dmask, damp, C, x);
+    launch_pdl(k_psc_block_q2<D>, grid, 128, 0, st, L.M, L.dmask, r, F, P, C);
+    launch_pdl(k_psc_gather_q2<D>, grid1(L.N), kBlock, 0, st, L.N, L.M, L.dmask, damp, C, x);
   });
 }
 
@@ -3191,7 +3270,7 @@ void launch_restrict(const LevelView& F, const LevelView& Cl, const double* rf, 
                      double* solc, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
   if (F.csr) {
-    k_csr_restrict<<<grid1(Cl.N), kBlock, 0, st>>>(Cl.N, F.pt, rf, rc, rhsc, solc);
+    launch_early(k_csr_restrict, grid1(Cl.N, kCsrT), kCsrT, 0, st, Cl.N, F.pt, rf, rc, rhsc, solc);
     return;
   }
   if (F.nc == 3) {
@@ -3201,14 +3280,14 @@ void launch_restrict(const LevelView& F, const LevelView& Cl, const double* rf, 
   FMG_DISPATCH(F.dim, F.order, {
     dim3 gr = xfer_grid(Cl.M, D);
     if (D < 3) gr.z = (unsigned)F.nb;  // the problems of a batched level
-    k_restrict<D, P><<<gr, dim3(32, 8), 0, st>>>((int)Cl.M, (int)F.M, F.dmask, rf, rc, rhsc, solc, F.Np, Cl.Np);
+    launch_early(k_restrict<D, P>, gr, dim3(32, 8), 0, st, (int)Cl.M, (int)F.M, F.dmask, rf, rc, rhsc, solc, F.Np, Cl.Np);
   });
 }
 
 void launch_prolong(const LevelView& Cl, const LevelView& F, const double* xc, double* xf, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
   if (F.csr) {
-    k_csr_prolong<<<grid1(F.N), kBlock, 0, st>>>(F.N, F.p, xc, xf);
+    launch_early(k_csr_prolong, grid1(F.N, kCsrT), kCsrT, 0, st, F.N, F.p, xc, xf);
     return;
   }
   if (F.nc == 3) {
@@ -3218,7 +3297,7 @@ void launch_prolong(const LevelView& Cl, const LevelView& F, const double* xc, d
   FMG_DISPATCH(F.dim, F.order, {
     dim3 gr = xfer_grid(F.M, D);
     if (D < 3) gr.z = (unsigned)F.nb;
-    k_prolong<D, P><<<gr, dim3(32, 8), 0, st>>>((int)F.M, (int)Cl.M, F.dmask, xc, xf, F.Np, Cl.Np);
+    launch_early(k_prolong<D, P>, gr, dim3(32, 8), 0, st, (int)F.M, (int)Cl.M, F.dmask, xc, xf, F.Np, Cl.Np);
   });
 }
 
@@ -3237,16 +3316,19 @@ void launch_coarse_solve(const double* AinvT, int n, double damp, double* x, dou
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (cs > 8) cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = (unsigned)cs;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchAttribute at[2]{};
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)cs;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_pdl
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.gridDim = dim3((unsigned)(nb * cs));
     cfg.blockDim = dim3(32 * (R + kCsLoad));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = t_pdl_stream == st ? 2 : 1;
+    t_pdl_stream = st;
     cudaLaunchKernelEx(&cfg, kern, AinvT, n, damp, x, r, vs, cs);
   };
   if (n <= 512) go(std::integral_constant<int, 1>{});
@@ -3290,45 +3372,45 @@ void launch_lu(double* A, int n, int* piv, double* X, double* XT, cudaStream_t s
 
 void launch_fill(double* x, long long n, double v, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  if (n > 0) k_fill<<<grid1(n), kBlock, 0, st>>>(x, n, v);
+  if (n > 0) launch_early(k_fill, grid1(n), kBlock, 0, st, x, n, v);
 }
 void launch_copy(const double* x, double* y, long long n, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  if (n > 0) k_copy<<<grid1(n), kBlock, 0, st>>>(x, y, n);
+  if (n > 0) launch_early(k_copy, grid1(n), kBlock, 0, st, x, y, n);
 }
 void launch_axpy(double alpha, const double* sc, int aslot, const double* x, double* y, long long n,
                  cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  if (n > 0) k_axpy<<<grid1(n), kBlock, 0, st>>>(alpha, sc, aslot, x, y, n);
+  if (n > 0) launch_early(k_axpy, grid1(n), kBlock, 0, st, alpha, sc, aslot, x, y, n);
 }
 void launch_dot(const double* x, const double* y, long long n, const Reduce& R, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_dot<<<nchunks(n), kBlock, 0, st>>>(x, y, n, R);
+  launch_early(k_dot, nchunks(n), kBlock, 0, st, x, y, n, R, 0);
 }
 void launch_dot_b(const double* x, const double* y, long long n, long long vs, int nb, const Reduce& R,
                   cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_dot<<<dim3(nchunks(n), (unsigned)nb), kBlock, 0, st>>>(x, y, n, R, vs);
+  launch_early(k_dot, dim3(nchunks(n), (unsigned)nb), kBlock, 0, st, x, y, n, R, vs);
 }
 void launch_cg_update(const double* sc, double* x, const double* p, double* r, const double* a, double* w,
                       double* w2, double* q, long long n, const Reduce& R, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_cg_update<<<nchunks(n), kBlock, 0, st>>>(sc, x, p, r, a, w, w2, q, n, R);
+  launch_early(k_cg_update, nchunks(n), kBlock, 0, st, sc, x, p, r, a, w, w2, q, n, R, 0, nullptr);
 }
 void launch_p_update(const double* sc, double* p, const double* q, long long n, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_p_update<<<grid1(n), kBlock, 0, st>>>(sc, p, q, n);
+  launch_early(k_p_update, grid1(n), kBlock, 0, st, sc, p, q, n, 0, nullptr);
 }
 void launch_cg_update_b(const double* sc, double* x, const double* p, double* r, const double* a, double* w,
                         double* w2, double* q, long long n, long long vs, int nb, const double* frozen,
                         const Reduce& R, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_cg_update<<<dim3(nchunks(n), (unsigned)nb), kBlock, 0, st>>>(sc, x, p, r, a, w, w2, q, n, R, vs, frozen);
+  launch_early(k_cg_update, dim3(nchunks(n), (unsigned)nb), kBlock, 0, st, sc, x, p, r, a, w, w2, q, n, R, vs, frozen);
 }
 void launch_p_update_b(const double* sc, double* p, const double* q, long long n, long long vs, int nb,
                        const double* frozen, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_p_update<<<dim3(grid1(n), (unsigned)nb), kBlock, 0, st>>>(sc, p, q, n, vs, frozen);
+  launch_early(k_p_update, dim3(grid1(n), (unsigned)nb), kBlock, 0, st, sc, p, q, n, vs, frozen);
 }
 
 void launch_sample_kq(int dim, long long ncells_l, long long n_l, long long n_top, double ratio, int np,
@@ -3424,15 +3506,15 @@ void launch_galerkin(const LevelView& F, const LevelView& Cl, double* AC, cudaSt
 
 void launch_bdiag3(const LevelView& L, int mode, const double* w, const double* x, double* y, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_bdiag3<<<grid1(L.N), kBlock, 0, st>>>(L.A, L.N, L.Np, L.center, mode, w, x, y);
+  launch_early(k_bdiag3, grid1(L.N), kBlock, 0, st, L.A, L.N, L.Np, L.center, mode, w, x, y);
 }
 void launch_xpwv3(const double* x, const double* w, const double* v, double* y, long long N, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_xpwv3<<<grid1(N), kBlock, 0, st>>>(x, w, v, y, N);
+  launch_early(k_xpwv3, grid1(N), kBlock, 0, st, x, w, v, y, N);
 }
 void launch_acc_prod3(double* acc, const double* a, const double* b, long long N, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_acc_prod3<<<grid1(N), kBlock, 0, st>>>(acc, a, b, N);
+  launch_early(k_acc_prod3, grid1(N), kBlock, 0, st, acc, a, b, N);
 }
 
 void vec32_spmv(int order, const float* A, long long N, long long Np, long long M, const float* x, const float* b,
@@ -3443,7 +3525,7 @@ void vec32_spmv(int order, const float* A, long long N, long long Np, long long 
 void vec32_jacobi0(const float* A, long long N, long long Np, int center, float damp, const double* omega,
                    const float* b, float* x, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_jacobi0_3<float><<<grid1(N), kBlock, 0, st>>>(A, N, Np, center, damp, omega, b, x);
+  launch_pdl(k_jacobi0_3<float>, grid1(N), kBlock, 0, st, A, N, Np, center, damp, omega, b, x);
 }
 void vec32_jacobi_res(int order, const float* A, long long N, long long Np, long long M, double damp,
                       const double* omega, const float* x, const float* b, float* xout, cudaStream_t st) {
@@ -3461,19 +3543,19 @@ void vec32_prolong(int order, long long MF, long long MC, int dmask, const float
 }
 void vec_to32(const double* x, const double* sc, int slot, int mode, float* y, long long n, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_vscale<double, float><<<grid1(n), kBlock, 0, st>>>(x, sc, slot, mode, y, n);
+  launch_pdl(k_vscale<double, float>, grid1(n), kBlock, 0, st, x, sc, slot, mode, y, n);
 }
 void vec_to64(const float* x, const double* sc, int slot, int mode, double* y, long long n, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_vscale<float, double><<<grid1(n), kBlock, 0, st>>>(x, sc, slot, mode, y, n);
+  launch_pdl(k_vscale<float, double>, grid1(n), kBlock, 0, st, x, sc, slot, mode, y, n);
 }
 void vec_f64_to_f32(const double* x, float* y, long long n, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_vscale<double, float><<<grid1(n), kBlock, 0, st>>>(x, nullptr, 0, 0, y, n);
+  launch_pdl(k_vscale<double, float>, grid1(n), kBlock, 0, st, x, nullptr, 0, 0, y, n);
 }
 void launch_fcg_beta(double* sc, bool first, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_fcg_beta<<<1, 1, 0, st>>>(sc, first ? 1 : 0);
+  launch_early(k_fcg_beta, 1, 1, 0, st, sc, first ? 1 : 0);
 }
 
 long long q2_slot_pos(int dim, long long M, long long i, int s, bool colour_major) {

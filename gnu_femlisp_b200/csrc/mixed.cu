@@ -350,6 +350,8 @@ k_mfc(MFArgsT<T> g, const __grid_constant__ CUtensorMap tk_cells, const __grid_c
   constexpr bool DIFF = sizeof(T) == 8;  // the FP64 operator in difference form
   constexpr bool HX = L::HX, HB = L::HB, HO = L::HO;
   constexpr bool OM = HO && (OPT & 1), V2 = RED && (OPT & 2), UWD = HO && (OPT & 4);
+  pdl_next();
+  pdl_wait();
   extern __shared__ __align__(128) unsigned char sm_dyn[];
   __shared__ double red[8];
   unsigned char* sm = sm_dyn + ((128u - (umma::smem_u32(sm_dyn) & 127u)) & 127u);
@@ -589,6 +591,8 @@ __global__ void __launch_bounds__(kBlock)
 k_st32(const float* __restrict__ A, long long N, long long Np, long long M, float w, const float* __restrict__ om,
        const float* __restrict__ x, const TB* __restrict__ b, TY* __restrict__ y, const double* __restrict__ v,
        const double* __restrict__ v2, Reduce2 R) {
+  pdl_next();
+  pdl_wait();
   constexpr int NS = St32<D, P>::NS;
   constexpr int C = St32<D, P>::CENTER;
   static_assert(RPT == 1 || RPT == 4, "one or four rows per thread");
@@ -710,6 +714,8 @@ template <int D, typename TR>
 __global__ void __launch_bounds__(kBlock)
 k_restrict_q1(int MC, int MF, int dmask, const TR* __restrict__ rf, __nv_bfloat16* __restrict__ bc,
               float* __restrict__ xc) {
+  pdl_next();
+  pdl_wait();
   if (D == 1 && threadIdx.y != 0) return;
   const int c0 = (int)(blockIdx.x * 32 + threadIdx.x), c1 = D > 1 ? (int)(blockIdx.y * 8 + threadIdx.y) : 0;
   if (c0 >= MC || c1 >= MC) return;
@@ -726,6 +732,8 @@ template <typename TR>
 __global__ void __launch_bounds__(kBlock)
 k_restrict_q1b(int MC, int MF, int dmask, const TR* __restrict__ rf, __nv_bfloat16* __restrict__ bc,
                float* __restrict__ xc) {
+  pdl_next();
+  pdl_wait();
   const int I = blockIdx.x * 32 + threadIdx.x, J0 = 2 * (blockIdx.y * 8 + threadIdx.y), K0 = 2 * blockIdx.z;
   if (I >= MC || J0 >= MC) return;
   if (I >= 1 && I <= MC - 2 && J0 >= 1 && J0 + 1 <= MC - 2 && K0 >= 1 && K0 + 1 <= MC - 2) {
@@ -768,6 +776,8 @@ template <int D, int P, typename TR>
 __global__ void __launch_bounds__(kBlock)
 k_restrict_mx(int MC, int MF, int dmask, const TR* __restrict__ rf, __nv_bfloat16* __restrict__ bc,
               float* __restrict__ xc) {
+  pdl_next();
+  pdl_wait();
   if (D == 1 && threadIdx.y != 0) return;
   const int cJ[3] = {(int)(blockIdx.x * 32 + threadIdx.x), D > 1 ? (int)(blockIdx.y * 8 + threadIdx.y) : 0,
                      D > 2 ? (int)blockIdx.z : 0};
@@ -813,6 +823,8 @@ k_restrict_mx(int MC, int MF, int dmask, const TR* __restrict__ rf, __nv_bfloat1
 template <int D>
 __global__ void __launch_bounds__(kBlock)
 k_prolong_q1(int MF, int MC, int dmask, const float* __restrict__ xc, float* __restrict__ xf) {
+  pdl_next();
+  pdl_wait();
   if (D == 1 && threadIdx.y != 0) return;
   const int fi[3] = {(int)(blockIdx.x * 32 + threadIdx.x), D > 1 ? (int)(blockIdx.y * 8 + threadIdx.y) : 0,
                      D > 2 ? (int)blockIdx.z : 0};
@@ -855,6 +867,8 @@ k_prolong_q1(int MF, int MC, int dmask, const float* __restrict__ xc, float* __r
 // fine node with the weights and in the order of k_prolong_q1.
 __global__ void __launch_bounds__(kBlock)
 k_prolong_q1c(int MF, int MC, int dmask, const float* __restrict__ xc, float* __restrict__ xf, VLay fl) {
+  pdl_next();
+  pdl_wait();
   const int I = blockIdx.x * 32 + threadIdx.x, J = blockIdx.y * 8 + threadIdx.y, K = blockIdx.z;
   if (I >= MC || J >= MC) return;
   const long long MC2 = (long long)MC * MC;
@@ -965,6 +979,8 @@ k_prolong_q1c(int MF, int MC, int dmask, const float* __restrict__ xc, float* __
 // Dirichlet values read as zero).
 __global__ void __launch_bounds__(kBlock)
 k_prolong_q1v(int MF, int MC, int dmask, const float* __restrict__ xc, float* __restrict__ xf, VLay fl) {
+  pdl_next();
+  pdl_wait();
   const unsigned q = (unsigned)fl.py >> 2;
   const unsigned idx = blockIdx.x * kBlock + threadIdx.x;
   if (idx >= q * (unsigned)MC) return;
@@ -1042,6 +1058,8 @@ k_prolong_q1v(int MF, int MC, int dmask, const float* __restrict__ xc, float* __
 template <int D, int P>
 __global__ void __launch_bounds__(kBlock)
 k_prolong_mx(int MF, int MC, int dmask, const float* __restrict__ xc, float* __restrict__ xf) {
+  pdl_next();
+  pdl_wait();
   if (D == 1 && threadIdx.y != 0) return;
   const int fi[3] = {(int)(blockIdx.x * 32 + threadIdx.x), D > 1 ? (int)(blockIdx.y * 8 + threadIdx.y) : 0,
                      D > 2 ? (int)blockIdx.z : 0};
@@ -1083,6 +1101,8 @@ k_prolong_mx(int MF, int MC, int dmask, const float* __restrict__ xc, float* __r
 // are in flight together
 __global__ void __launch_bounds__(1024)
 k_coarse_mx(const double* __restrict__ AinvT, int n, const __nv_bfloat16* __restrict__ b, float* __restrict__ x) {
+  pdl_next();
+  pdl_wait();
   __shared__ double rs[1024];
   for (int i = threadIdx.x; i < n; i += 1024) rs[i] = (double)__bfloat162float(b[i]);
   __syncthreads();
@@ -1103,6 +1123,8 @@ k_coarse_mx(const double* __restrict__ AinvT, int n, const __nv_bfloat16* __rest
 
 // ------------------------------------------------------------ vector ops
 __global__ void k_f64_to_f32(const double* __restrict__ a, float* __restrict__ b, long long n) {
+  pdl_next();
+  pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) b[i] = (float)a[i];
 }
@@ -1136,6 +1158,8 @@ constexpr int kUpdBlocks = 1184;  // eight per SM of a B200
 __global__ void __launch_bounds__(kBlock)
 k_fcg64_update(double* sc, double* __restrict__ x, const float* __restrict__ p, double* __restrict__ r,
                const double* __restrict__ a, float* __restrict__ r32, long long n, Reduce2 R) {
+  pdl_next();
+  pdl_wait();
   __shared__ double smem[8];
   const double lam = sc[M_LAM], s = sc[M_SCALE];
   double acc = 0.0;
@@ -1163,6 +1187,8 @@ k_fcg64_update(double* sc, double* __restrict__ x, const float* __restrict__ p, 
 // the same vector in a = A p and in x += lam p, which it is
 __global__ void k_fcg64_p(const double* __restrict__ sc, float* __restrict__ p, const float* __restrict__ q,
                           long long n, int first) {
+  pdl_next();
+  pdl_wait();
   const long long i0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i0 >= n) return;
   const double inv = sc[M_SINV], beta = sc[M_BETA];  // 1 / scale of the FP32 residual
@@ -1184,6 +1210,8 @@ __global__ void k_fcg64_p(const double* __restrict__ sc, float* __restrict__ p, 
 }
 
 __global__ void k_f32_to_f64(const float* __restrict__ a, double* __restrict__ b, long long n) {
+  pdl_next();
+  pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) b[i] = (double)a[i];
 }
@@ -1191,6 +1219,8 @@ __global__ void k_f32_to_f64(const float* __restrict__ a, double* __restrict__ b
 // r32 = r * sc[slot]
 __global__ void k_scale_to32(const double* __restrict__ r, const double* __restrict__ sc, int slot,
                              float* __restrict__ r32, long long n) {
+  pdl_next();
+  pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) r32[i] = (float)(r[i] * sc[slot]);
 }
@@ -1199,6 +1229,8 @@ __global__ void k_scale_to32(const double* __restrict__ r, const double* __restr
 __global__ void __launch_bounds__(kBlock)
 k_dot2_64(const double* __restrict__ xv, const float* __restrict__ yv, const double* __restrict__ y2,
           long long n, Reduce2 R) {
+  pdl_next();
+  pdl_wait();
   __shared__ double smem[8];
   const long long i = (long long)blockIdx.x * kBlock + threadIdx.x;
   double a0 = 0.0, a1 = 0.0;
@@ -1369,7 +1401,7 @@ static void mft_launch(const MFArgsT<T>& g, const TX* x, const T* b, T* y, const
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
       attr |= 1u << dev;
     }
-    kern<<<mft_blocks(q), kFThreads, smem, st>>>(g, tk, tx, tb, to, tv, tv2, q, x, b, y, v, v2, R);
+    launch_pdl(kern, mft_blocks(q), kFThreads, smem, st, g, tk, tx, tb, to, tv, tv2, q, x, b, y, v, v2, R);
   };
   switch (opt) {
     case 1: if constexpr (HO) go(std::integral_constant<int, 1>{}); break;
@@ -1410,6 +1442,8 @@ static void mf_launch(int mode, const MFArgsT<T>& g, const TX* x, const T* b, T*
 // four nodes per thread (16-byte accesses when all three vectors allow them)
 __global__ void __launch_bounds__(kBlock) k_wd_scale(const float* __restrict__ wd, const float* __restrict__ b,
                                                      float* __restrict__ y, long long n) {
+  pdl_next();
+  pdl_wait();
   const long long i0 = ((long long)blockIdx.x * kBlock + threadIdx.x) * 4;
   if (i0 >= n) return;
   if (i0 + 4 <= n && (((uintptr_t)wd | (uintptr_t)b | (uintptr_t)y) & 15) == 0) {
@@ -1439,6 +1473,8 @@ __device__ __forceinline__ bool plane_node(int M, int& ix, int& iy, int& iz, lon
 // in the same order; cells outside the grid count zero); Dirichlet nodes
 // (identity rows) get the damping itself
 __global__ void __launch_bounds__(kBlock) k_mf_wd(MFArgs g, float* __restrict__ wd) {
+  pdl_next();
+  pdl_wait();
   const int M = g.M, n = g.n, dm = g.dmask;
   int ix, iy, iz;
   long long i;
@@ -1481,7 +1517,7 @@ __global__ void __launch_bounds__(kBlock) k_mf_wd(MFArgs g, float* __restrict__ 
 
 void mx_top_wd(const MFArgs& g, float* wd, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_mf_wd<<<dim3(g1((long long)g.M * g.M), (unsigned)g.M), kBlock, 0, st>>>(g, wd);
+  launch_pdl(k_mf_wd, dim3(g1((long long)g.M * g.M), (unsigned)g.M), kBlock, 0, st, g, wd);
 }
 
 void mx_top_apply(int mode, const MFArgs& g, const float* x, const float* b, float* y, const double* v,
@@ -1489,7 +1525,7 @@ void mx_top_apply(int mode, const MFArgs& g, const float* x, const float* b, flo
   if (mode == 3 && g.wd && !R) {  // a stream of two reads and a write over the arrays (padding included)
     g_launches.fetch_add(1, std::memory_order_relaxed);
     const long long n = g.ol.total;
-    k_wd_scale<<<g1((n + 3) / 4), kBlock, 0, st>>>(g.wd, b, y, n);
+    launch_pdl(k_wd_scale, g1((n + 3) / 4), kBlock, 0, st, g.wd, b, y, n);
     return;
   }
   mf_launch<float, double, float>(mode, g, x, b, y, v, v2, R, st);
@@ -1518,10 +1554,9 @@ void st32_launch(const Lev32& L, const float* x, const void* b, void* y, const d
                  const Reduce2& r0, cudaStream_t st) {
   constexpr int W = (D == 3 && P == 2) ? 1 : 4;
   if (W == 4 && L.N >= kSt32Wide)
-    k_st32<D, P, MODE, TB, TY, RED, W><<<g1((L.N + W - 1) / W), kBlock, 0, st>>>(
-        L.A, L.N, L.Np, L.M, L.w, L.om, x, (const TB*)b, (TY*)y, v, v2, r0);
+    launch_pdl(k_st32<D, P, MODE, TB, TY, RED, W>, g1((L.N + W - 1) / W), kBlock, 0, st, L.A, L.N, L.Np, L.M, L.w, L.om, x, (const TB*)b, (TY*)y, v, v2, r0);
   else
-    k_st32<D, P, MODE, TB, TY, RED, 1><<<g1(L.N), kBlock, 0, st>>>(L.A, L.N, L.Np, L.M, L.w, L.om, x,
+    launch_pdl(k_st32<D, P, MODE, TB, TY, RED, 1>, g1(L.N), kBlock, 0, st, L.A, L.N, L.Np, L.M, L.w, L.om, x,
                                                                     (const TB*)b, (TY*)y, v, v2, r0);
 }
 
@@ -1564,23 +1599,23 @@ void mx_restrict(const Lev32& F, const Lev32& C, const void* rf, bool rf_bf16, _
     typedef __nv_bfloat16 bf;
     if (F.dim == 3 && C.N >= (1ll << 20)) {  // large levels: 2 x 2 coarse nodes per thread
       const dim3 g2((unsigned)((C.M + 31) / 32), (unsigned)((C.M + 15) / 16), (unsigned)((C.M + 1) / 2));
-      if (rf_bf16) k_restrict_q1b<bf><<<g2, bl, 0, st>>>((int)C.M, (int)F.M, F.dmask, (const bf*)rf, bc, xc);
-      else k_restrict_q1b<float><<<g2, bl, 0, st>>>((int)C.M, (int)F.M, F.dmask, (const float*)rf, bc, xc);
+      if (rf_bf16) launch_pdl(k_restrict_q1b<bf>, g2, bl, 0, st, (int)C.M, (int)F.M, F.dmask, (const bf*)rf, bc, xc);
+      else launch_pdl(k_restrict_q1b<float>, g2, bl, 0, st, (int)C.M, (int)F.M, F.dmask, (const float*)rf, bc, xc);
     } else if (F.dim == 3) {  // small levels are latency-bound: one coarse node per thread
-      if (rf_bf16) k_restrict_q1<3, bf><<<gr, bl, 0, st>>>((int)C.M, (int)F.M, F.dmask, (const bf*)rf, bc, xc);
-      else k_restrict_q1<3, float><<<gr, bl, 0, st>>>((int)C.M, (int)F.M, F.dmask, (const float*)rf, bc, xc);
+      if (rf_bf16) launch_pdl(k_restrict_q1<3, bf>, gr, bl, 0, st, (int)C.M, (int)F.M, F.dmask, (const bf*)rf, bc, xc);
+      else launch_pdl(k_restrict_q1<3, float>, gr, bl, 0, st, (int)C.M, (int)F.M, F.dmask, (const float*)rf, bc, xc);
     } else if (F.dim == 2) {
-      if (rf_bf16) k_restrict_q1<2, bf><<<gr, bl, 0, st>>>((int)C.M, (int)F.M, F.dmask, (const bf*)rf, bc, xc);
-      else k_restrict_q1<2, float><<<gr, bl, 0, st>>>((int)C.M, (int)F.M, F.dmask, (const float*)rf, bc, xc);
+      if (rf_bf16) launch_pdl(k_restrict_q1<2, bf>, gr, bl, 0, st, (int)C.M, (int)F.M, F.dmask, (const bf*)rf, bc, xc);
+      else launch_pdl(k_restrict_q1<2, float>, gr, bl, 0, st, (int)C.M, (int)F.M, F.dmask, (const float*)rf, bc, xc);
     } else {
-      if (rf_bf16) k_restrict_q1<1, bf><<<gr, bl, 0, st>>>((int)C.M, (int)F.M, F.dmask, (const bf*)rf, bc, xc);
-      else k_restrict_q1<1, float><<<gr, bl, 0, st>>>((int)C.M, (int)F.M, F.dmask, (const float*)rf, bc, xc);
+      if (rf_bf16) launch_pdl(k_restrict_q1<1, bf>, gr, bl, 0, st, (int)C.M, (int)F.M, F.dmask, (const bf*)rf, bc, xc);
+      else launch_pdl(k_restrict_q1<1, float>, gr, bl, 0, st, (int)C.M, (int)F.M, F.dmask, (const float*)rf, bc, xc);
     }
     return;
   }
   MX_DISPATCH(F.dim, F.order, {
-    if (rf_bf16) k_restrict_mx<D, P, __nv_bfloat16><<<gr, bl, 0, st>>>((int)C.M, (int)F.M, F.dmask, (const __nv_bfloat16*)rf, bc, xc);
-    else k_restrict_mx<D, P, float><<<gr, bl, 0, st>>>((int)C.M, (int)F.M, F.dmask, (const float*)rf, bc, xc);
+    if (rf_bf16) launch_pdl(k_restrict_mx<D, P, __nv_bfloat16>, gr, bl, 0, st, (int)C.M, (int)F.M, F.dmask, (const __nv_bfloat16*)rf, bc, xc);
+    else launch_pdl(k_restrict_mx<D, P, float>, gr, bl, 0, st, (int)C.M, (int)F.M, F.dmask, (const float*)rf, bc, xc);
   });
 }
 
@@ -1589,39 +1624,39 @@ void mx_prolong(const Lev32& C, const Lev32& F, const float* xc, float* xf, cuda
   const dim3 gr = xgrid(F.M, F.dim), bl(32, 8);
   if (F.order == 1) {
     if (F.dim == 3 && xfl && xfl->py % 4 == 0 && xfl->pz % 4 == 0 && ((uintptr_t)xf & 15) == 0)
-      k_prolong_q1v<<<dim3((unsigned)((xfl->py / 4 * C.M + kBlock - 1) / kBlock), (unsigned)C.M), kBlock, 0, st>>>(
-          (int)F.M, (int)C.M, F.dmask, xc, xf, *xfl);
+      launch_pdl(k_prolong_q1v, dim3((unsigned)((xfl->py / 4 * C.M + kBlock - 1) / kBlock), (unsigned)C.M), kBlock, 0, st, (int)F.M, (int)C.M, F.dmask, xc, xf, *xfl);
     else if (F.dim == 3)
-      k_prolong_q1c<<<dim3((unsigned)((C.M + 31) / 32), (unsigned)((C.M + 7) / 8), (unsigned)C.M), bl, 0, st>>>(
-          (int)F.M, (int)C.M, F.dmask, xc, xf, xfl ? *xfl : natural_lay((int)F.M, 3));
-    else if (F.dim == 2) k_prolong_q1<2><<<gr, bl, 0, st>>>((int)F.M, (int)C.M, F.dmask, xc, xf);
-    else k_prolong_q1<1><<<gr, bl, 0, st>>>((int)F.M, (int)C.M, F.dmask, xc, xf);
+      launch_pdl(k_prolong_q1c, dim3((unsigned)((C.M + 31) / 32), (unsigned)((C.M + 7) / 8), (unsigned)C.M), bl, 0, st, (int)F.M, (int)C.M, F.dmask, xc, xf, xfl ? *xfl : natural_lay((int)F.M, 3));
+    else if (F.dim == 2) launch_pdl(k_prolong_q1<2>, gr, bl, 0, st, (int)F.M, (int)C.M, F.dmask, xc, xf);
+    else launch_pdl(k_prolong_q1<1>, gr, bl, 0, st, (int)F.M, (int)C.M, F.dmask, xc, xf);
     return;
   }
-  MX_DISPATCH(F.dim, F.order, { k_prolong_mx<D, P><<<gr, bl, 0, st>>>((int)F.M, (int)C.M, F.dmask, xc, xf); });
+  MX_DISPATCH(F.dim, F.order, { launch_pdl(k_prolong_mx<D, P>, gr, bl, 0, st, (int)F.M, (int)C.M, F.dmask, xc, xf); });
 }
 
 void mx_coarse(const double* AinvT, int n, const __nv_bfloat16* b, float* x, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_coarse_mx<<<1, 1024, 0, st>>>(AinvT, n, b, x);
+  launch_pdl(k_coarse_mx, 1, 1024, 0, st, AinvT, n, b, x);
 }
 
 void mx_f64_to_f32(const double* a, float* b, long long n, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_f64_to_f32<<<g1(n), kBlock, 0, st>>>(a, b, n);
+  launch_pdl(k_f64_to_f32, g1(n), kBlock, 0, st, a, b, n);
 }
 
 void mx_fcg64_update(double* sc, double* x, const float* p, double* r, const double* a, float* r32, long long np,
                      const Reduce2& R, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
   const long long nb = std::min<long long>(g1(np / 2), kUpdBlocks);
-  k_fcg64_update<<<(unsigned)std::max<long long>(nb, 1), kBlock, 0, st>>>(sc, x, p, r, a, r32, np, R);
+  launch_pdl(k_fcg64_update, (unsigned)std::max<long long>(nb, 1), kBlock, 0, st, sc, x, p, r, a, r32, np, R);
 }
 
 // b (layout bl) = a (natural), 3D, M nodes a side: FP64 to FP32, and FP64
 // copied (grids of plane_node)
 
 __global__ void k_f64_to_f32_lay(const double* __restrict__ a, float* __restrict__ b, VLay bl, int M) {
+  pdl_next();
+  pdl_wait();
   int ix, iy, iz;
   long long i;
   if (!plane_node(M, ix, iy, iz, i)) return;
@@ -1629,6 +1664,8 @@ __global__ void k_f64_to_f32_lay(const double* __restrict__ a, float* __restrict
 }
 
 __global__ void k_f64_copy_lay(const double* __restrict__ a, double* __restrict__ b, VLay bl, int M) {
+  pdl_next();
+  pdl_wait();
   int ix, iy, iz;
   long long i;
   if (!plane_node(M, ix, iy, iz, i)) return;
@@ -1637,6 +1674,8 @@ __global__ void k_f64_copy_lay(const double* __restrict__ a, double* __restrict_
 
 // b (natural) = a (layout al), FP64, 3D
 __global__ void k_f64_from_lay(const double* __restrict__ a, VLay al, double* __restrict__ b, int M) {
+  pdl_next();
+  pdl_wait();
   int ix, iy, iz;
   long long i;
   if (!plane_node(M, ix, iy, iz, i)) return;
@@ -1645,37 +1684,37 @@ __global__ void k_f64_from_lay(const double* __restrict__ a, VLay al, double* __
 
 void mx_f64_from_lay(const double* a, const VLay& al, double* b, int M, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_f64_from_lay<<<dim3(g1((long long)M * M), (unsigned)M), kBlock, 0, st>>>(a, al, b, M);
+  launch_pdl(k_f64_from_lay, dim3(g1((long long)M * M), (unsigned)M), kBlock, 0, st, a, al, b, M);
 }
 
 void mx_f64_to_f32_lay(const double* a, float* b, const VLay& bl, int M, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_f64_to_f32_lay<<<dim3(g1((long long)M * M), (unsigned)M), kBlock, 0, st>>>(a, b, bl, M);
+  launch_pdl(k_f64_to_f32_lay, dim3(g1((long long)M * M), (unsigned)M), kBlock, 0, st, a, b, bl, M);
 }
 
 void mx_f64_copy_lay(const double* a, double* b, const VLay& bl, int M, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_f64_copy_lay<<<dim3(g1((long long)M * M), (unsigned)M), kBlock, 0, st>>>(a, b, bl, M);
+  launch_pdl(k_f64_copy_lay, dim3(g1((long long)M * M), (unsigned)M), kBlock, 0, st, a, b, bl, M);
 }
 
 void mx_f32_to_f64(const float* a, double* b, long long n, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_f32_to_f64<<<g1(n), kBlock, 0, st>>>(a, b, n);
+  launch_pdl(k_f32_to_f64, g1(n), kBlock, 0, st, a, b, n);
 }
 
 void mx_fcg64_p(const double* sc, float* p, const float* q, long long n, bool first, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_fcg64_p<<<g1((n + 3) / 4), kBlock, 0, st>>>(sc, p, q, n, first ? 1 : 0);
+  launch_pdl(k_fcg64_p, g1((n + 3) / 4), kBlock, 0, st, sc, p, q, n, first ? 1 : 0);
 }
 
 void mx_scale_to32(const double* r, const double* sc, int slot, float* r32, long long n, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_scale_to32<<<g1(n), kBlock, 0, st>>>(r, sc, slot, r32, n);
+  launch_pdl(k_scale_to32, g1(n), kBlock, 0, st, r, sc, slot, r32, n);
 }
 
 void mx_dot2_64(const double* x, const float* y, const double* y2, long long n, const Reduce2& R, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_dot2_64<<<g1(n), kBlock, 0, st>>>(x, y, y2, n, R);
+  launch_pdl(k_dot2_64, g1(n), kBlock, 0, st, x, y, y2, n, R);
 }
 
 }  // namespace fmg
