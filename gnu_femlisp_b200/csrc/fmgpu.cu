@@ -421,10 +421,36 @@ struct MG {
   const fmg_solve_cfg& c;
   bool literal;          // keep every residual write (fmg_vcycle on user vectors)
   cudaStream_t st;
+  Tail tail{};           // the steps on small levels, run in one launch when the cycle leaves them
+  int tail_top = -2;     // the highest such level (-2: not yet known)
+
+  // level l's steps are collected; otherwise what was collected runs now
+  bool small(int l) {
+    if (tail_top == -2) {
+      tail_top = -1;
+      long long need = 0;
+      const bool q1 = g->nc == 1 && (g->algebraic || g->order == 1);
+      for (int k = g->base; q1 && k <= g->top && k < g->base + Tail::kLev - 1; ++k) {
+        need += tail_need(view(g, k));
+        if (need > tail_room(g->algebraic ? 1 : g->dim, g->nb)) break;
+        tail_top = k;
+      }
+      if (tail_top <= g->base) tail_top = -1;  // the base level alone: one launch either way
+    }
+    if (l <= tail_top) return true;
+    tail_flush(tail, st, true);
+    return false;
+  }
 
   bool alias(int l) const { return g->rhsp[l] == g->resp[l]; }
 
   void residual(int l) {
+    if (small(l)) {
+      TailStep s{TAIL_RES};
+      s.x = g->solp[l]; s.b = g->rhsp[l]; s.r = g->resp[l];
+      tail_add(tail, l, view(g, l), s, st);
+      return;
+    }
     launch_spmv(view(g, l), g->solp[l], g->rhsp[l], g->resp[l], nullptr, nullptr, st);
   }
   void ensure_res() {  // ensure-mg-residual (multigrid.lisp:173-177)
@@ -434,6 +460,13 @@ struct MG {
   // one <jacobi> step; with need_res the preceding compute-residual is fused in
   void jacobi_step(int l, bool need_res) {
     const bool write_r = literal || alias(l);
+    if (small(l)) {
+      TailStep s{need_res ? TAIL_JACOBI_RES : TAIL_JACOBI, write_r, c.damp};
+      s.x = g->solp[l]; s.y = g->sparep[l]; s.b = g->rhsp[l]; s.r = g->resp[l];
+      tail_add(tail, l, view(g, l), s, st);
+      if (need_res) std::swap(g->solp[l], g->sparep[l]);
+      return;
+    }
     if (need_res) {
       launch_jacobi_res(view(g, l), c.damp, g->solp[l], g->rhsp[l], g->sparep[l], g->resp[l], write_r,
                         nullptr, nullptr, st);
@@ -462,7 +495,8 @@ struct MG {
       if (!ready) { g->ssc_unprepared = true; g->rp[l] = 0; return; }
       if (keep) ensure_res();
       for (int s = 0; s < steps; ++s) {
-        launch_ssc(view(g, l), c.damp, g->solp[l], g->rhsp[l], g->resp[l], g->order == 2 ? g->sscF[l] : nullptr,
+        if (small(l)) tail_sweep(tail, l, view(g, l), true, c.damp, g->solp[l], g->rhsp[l], g->resp[l], st);
+        else launch_ssc(view(g, l), c.damp, g->solp[l], g->rhsp[l], g->resp[l], g->order == 2 ? g->sscF[l] : nullptr,
                    g->order == 2 ? g->sscP[l] : nullptr, st);
         if (steps > 1 && keep) residual(l);
       }
@@ -474,33 +508,58 @@ struct MG {
       bool need = !g->rp[l];
       for (int s = 0; s < steps; ++s) {
         if (need) residual(l);
+        tail_flush(tail, st, false);
         launch_psc(view(g, l), c.damp, g->solp[l], g->resp[l], g->order == 2 ? g->sscF[l] : nullptr,
                    g->order == 2 ? g->sscP[l] : nullptr, g->order == 2 ? g->sscC[l] : nullptr, st);
         need = true;
       }
       if (steps > 1 && (literal || alias(l))) residual(l);
     } else {
-      for (int s = 0; s < steps; ++s) launch_sor(view(g, l), c.damp, g->solp[l], g->rhsp[l], g->resp[l], st);
+      for (int s = 0; s < steps; ++s) {
+        if (small(l)) tail_sweep(tail, l, view(g, l), false, c.damp, g->solp[l], g->rhsp[l], g->resp[l], st);
+        else launch_sor(view(g, l), c.damp, g->solp[l], g->rhsp[l], g->resp[l], st);
+      }
     }
     g->rp[l] = 0;
   }
   void restrict_() {  // restrict + :after methods (multigrid.lisp:202-224)
     const int l = g->cur;
     ensure_res();
-    launch_restrict(view(g, l), view(g, l - 1), g->resp[l], g->resp[l - 1], g->rhsp[l - 1], g->solp[l - 1], st);
+    if (small(l)) {
+      TailStep s{TAIL_RESTRICT};
+      s.x = g->resp[l]; s.r = g->resp[l - 1]; s.b = g->rhsp[l - 1]; s.y = g->solp[l - 1];
+      const LevelView C = view(g, l - 1);
+      tail_add(tail, l, view(g, l), s, st, &C);
+    } else launch_restrict(view(g, l), view(g, l - 1), g->resp[l], g->resp[l - 1], g->rhsp[l - 1], g->solp[l - 1], st);
     g->cur = l - 1;
     g->rp[l - 1] = 1;
   }
   void prolongate() {  // multigrid.lisp:237-252
     const int l = g->cur;
-    launch_prolong(view(g, l), view(g, l + 1), g->solp[l], g->solp[l + 1], st);
+    if (small(l + 1)) {
+      TailStep s{TAIL_PROLONG};
+      s.x = g->solp[l]; s.y = g->solp[l + 1];
+      const LevelView C = view(g, l);
+      tail_add(tail, l + 1, view(g, l + 1), s, st, &C);
+    } else {
+      launch_prolong(view(g, l), view(g, l + 1), g->solp[l], g->solp[l + 1], st);
+    }
     g->cur = l + 1;
     g->rp[l + 1] = 0;
   }
   void lmgc() {  // multigrid.lisp:254-288
     const int l = g->cur;
     if (l == g->base) {
-      launch_coarse_solve(g->ainvT, g->nbase, c.coarse_damp, g->solp[l], g->resp[l], st, g->nb, g->lev[l].Np);
+      if (g->nbase <= 128 && small(l)) {
+        TailStep s{TAIL_COARSE, true, c.coarse_damp};
+        s.x = g->solp[l]; s.r = g->resp[l];
+        tail.nbase = g->nbase;
+        tail.ainv = g->ainvT;
+        tail_add(tail, l, view(g, l), s, st);
+      } else {
+        tail_flush(tail, st, false);
+        launch_coarse_solve(g->ainvT, g->nbase, c.coarse_damp, g->solp[l], g->resp[l], st, g->nb, g->lev[l].Np);
+      }
       g->rp[l] = 0;
       return;
     }
@@ -549,6 +608,7 @@ struct MG {
     g->cur = top;
     if (c.fmg) fcycle();
     else lmgc();
+    tail_flush(tail, st, true);
     *x = g->solp[top];
     *spare = g->sparep[top];
   }
@@ -2853,6 +2913,7 @@ void coarse_apply(fmg_grid* g, const fmg_solve_cfg& cf, const double* y, cudaStr
   g->rp[t - 1] = 1;
   MG mg{g, cf, false, st};
   mg.lmgc();
+  tail_flush(mg.tail, st, true);
   g->cur = t;
 }
 

@@ -110,6 +110,64 @@ void launch_prolong(const LevelView& C, const LevelView& F, const double* xc, do
 // nb problems of a batched base level: inverses n x n apart, vectors vs apart
 void launch_coarse_solve(const double* AinvT, int n, double damp, double* x, double* r, cudaStream_t st,
                          int nb = 1, long long vs = 0);
+// Small levels in one launch: the steps a cycle takes on the levels whose data
+// fit in one SM's shared memory (scalar Q1, structured or algebraic) are
+// collected and run by one CTA (one per problem of a batch), a block barrier
+// between consecutive steps.  Each step does, row by row, the operations of
+// its own kernel.
+struct TailLevel {
+  const double* A;      // structured: slot arrays (copied to aoff)
+  const double* omega;
+  long long Np;
+  int N, M, aoff;
+  CsrView a, p, pt;     // algebraic
+  const double* diag;
+};
+struct TailVec {        // a level vector: where it lives, its place in shared memory
+  double* g;
+  int off, lev;
+  bool in, out;         // read before the steps write it; written
+};
+enum TailKind { TAIL_RES, TAIL_JACOBI, TAIL_JACOBI_RES, TAIL_SOR, TAIL_SSC, TAIL_RESTRICT, TAIL_PROLONG, TAIL_COARSE };
+struct TailOp {
+  short kind, lev, clev;  // level (RESTRICT, PROLONG: the fine one) and coarse level, as table entries
+  short flag;             // write_r, or the colour
+  int x, y, r, b;         // vectors (places in shared memory): solution (RESTRICT: fine residual; PROLONG: coarse
+                          // solution), output (RESTRICT: coarse solution), residual, rhs
+  int n;                  // items (rows) of the step
+  double w;               // damping
+  const int* rows;        // algebraic colour
+};
+struct Tail {
+  static constexpr int kOps = 160, kLev = 10, kVec = 48;
+  int dim = 0, dmask = 0, nb = 1, nbase = 0;
+  const double* ainv = nullptr;
+  bool csr = false;
+  int nops = 0, nlev = 0, nvec = 0, used = 0;  // used: doubles of shared memory
+  int levid[kLev];      // grid level of each table entry
+  TailLevel lev[kLev];
+  TailVec vec[kVec];
+  TailOp ops[kOps];
+};
+// doubles of shared memory a level's steps take, and those one CTA has when nb
+// of them run
+long long tail_need(const LevelView& L);
+long long tail_room(int dim, int nb);
+struct TailStep {       // a step as the cycle names it
+  TailKind kind;
+  bool write_r = false;
+  double w = 0.0;
+  double *x = nullptr, *y = nullptr, *r = nullptr, *b = nullptr;
+};
+// appends a step on level l (view L); RESTRICT and PROLONG: l, L the fine
+// level, *C the coarse one
+void tail_add(Tail& t, int l, const LevelView& L, const TailStep& s, cudaStream_t st, const LevelView* C = nullptr);
+// the colours of one SOR (or one-unknown SSC) sweep
+void tail_sweep(Tail& t, int l, const LevelView& L, bool ssc, double omega, double* x, double* b, double* r,
+                cudaStream_t st);
+// runs what was collected.  leaving: the cycle goes on above these levels, so
+// only the vectors of the highest one are read again before they are written
+void tail_flush(Tail& t, cudaStream_t st, bool leaving);
 void launch_lu(double* A, int n, int* piv, double* X, double* XT, cudaStream_t st);
 void launch_fill(double* x, long long n, double v, cudaStream_t st);
 void launch_copy(const double* x, double* y, long long n, cudaStream_t st);

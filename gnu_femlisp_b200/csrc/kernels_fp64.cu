@@ -41,6 +41,14 @@ __device__ __forceinline__ void cp_async8(double* dst, const double* src) {
                : "memory");
 }
 
+// an input vector's element: in global memory and read-only, or (OWN) in
+// shared memory
+template <bool OWN, typename T>
+__device__ __forceinline__ T load_in(const T* p) {
+  if constexpr (OWN) return *p;
+  else return __ldg(p);
+}
+
 template <int D, int P>
 __device__ __forceinline__ long long slot_off(int s, long long M) {
   constexpr int W = 2 * P + 1;
@@ -1420,8 +1428,8 @@ __device__ __forceinline__ bool face_dir(int c, int M, int k, int dmask) {
 // outside the level and Dirichlet nodes are skipped.  (3D Q1, 129^3 coarse
 // nodes: 64 us, 138 us with each load waiting for the previous term; one
 // memory wait per plane on small levels, 12.4 -> 6 us at 33^3.)
-// NC: components per node; rf points at the component summed.
-template <int D, int P, int NC = 1, typename T = double>
+// NC: components per node; rf points at the component summed; CG: see load_in.
+template <int D, int P, int NC = 1, typename T = double, bool OWN = false>
 __device__ __forceinline__ T restrict_node(const int cJ[3], int MC, int MF, int dmask, const T* __restrict__ rf) {
 #pragma unroll
   for (int k = 0; k < D; ++k)
@@ -1453,7 +1461,7 @@ __device__ __forceinline__ T restrict_node(const int cJ[3], int MC, int MF, int 
 #pragma unroll
       for (int q = 0; q < R; ++q)
         if (on[0][q] && (D < 2 || on[1][y]) && (D < 3 || on[2][z]))
-          v[y * R + q] = __ldg(rf + NC * (f[0][q] + (long long)MF * ((D > 1 ? f[1][y] : 0) +
+          v[y * R + q] = load_in<OWN>(rf + NC * (f[0][q] + (long long)MF * ((D > 1 ? f[1][y] : 0) +
                                                                      (long long)MF * (D > 2 ? f[2][z] : 0))));
 #pragma unroll
     for (int y = 0; y < (D > 1 ? R : 1); ++y)
@@ -1471,7 +1479,7 @@ __device__ __forceinline__ T restrict_node(const int cJ[3], int MC, int MF, int 
 
 // (I xc) at fine node fi, not a Dirichlet node (constrained); all loads first
 // (3D Q1, 257^3 fine nodes: 197 us, 469 us with a load per term)
-template <int D, int P, int NC = 1, typename T = double>
+template <int D, int P, int NC = 1, typename T = double, bool OWN = false>
 __device__ __forceinline__ T prolong_node(const int fi[3], int MF, int MC, int dmask, const T* __restrict__ xc) {
   constexpr int R = P == 1 ? 2 : 3;
   int j[3][R];
@@ -1499,7 +1507,7 @@ __device__ __forceinline__ T prolong_node(const int fi[3], int MF, int MC, int d
 #pragma unroll
       for (int q = 0; q < R; ++q)
         if (on[0][q] && (D < 2 || on[1][y]) && (D < 3 || on[2][z]))
-          v[(z * NY + y) * R + q] = __ldg(xc + NC * (j[0][q] + (long long)MC * ((D > 1 ? j[1][y] : 0) +
+          v[(z * NY + y) * R + q] = load_in<OWN>(xc + NC * (j[0][q] + (long long)MC * ((D > 1 ? j[1][y] : 0) +
                                                                                 (long long)MC * (D > 2 ? j[2][z] : 0))));
   T acc = T(0);
 #pragma unroll
@@ -3027,6 +3035,241 @@ __global__ void k_fcg_beta(double* sc, int first) {
   sc[S_RATIO] = first ? 0.0 : -sc[S_TMP] / sc[S_BETA];
 }
 
+// ------------------------------------------------------------ small levels
+// The collected steps of a cycle on small levels (see Tail).  A launch costs a
+// small level 2-3 us whatever it does, and a step that goes to L2 for its
+// operands 1,400 cycles and more (so measured with the levels' data in global
+// memory, one CTA or a cluster of eight: no faster than the launches).  Here
+// the structured matrices come into shared memory while the previous launch
+// ends, the vectors the steps read first follow, and a step costs its barrier,
+// its chain and its division: 600-1,300 cycles on up to 300 nodes.  The 26
+// steps of a V(1,1) cycle on 33^2 nodes and below take 25 us in place of some
+// 60; 64^2 Poisson solve 1.09 -> 0.81 ms, adaptive 2D solve 2.38 -> 2.16 ms.
+constexpr int kTailT = 512;
+
+// the launch's parameters; CAP: room for the steps (the parameters are copied
+// at every launch, and most cycles' tails have fewer than 48 steps)
+template <int CAP>
+struct TailArgs {
+  int dmask, nbase, nops, nlev, nvec;
+  const double* ainv;
+  TailLevel lev[Tail::kLev];
+  TailVec vec[Tail::kVec];
+  TailOp ops[CAP];
+};
+
+// row sum, the unknowns (and a structured matrix) in shared memory
+template <int D, bool CSR>
+__device__ __forceinline__ double tail_row(const TailLevel& L, const double* sm, const double* x, int i, double& dg) {
+  double s = 0.0;
+  if constexpr (CSR) {
+    dg = __ldg(L.diag + i);
+    constexpr int K = 8;
+    const int e1 = (int)L.a.start[i + 1];
+    for (int e = (int)L.a.start[i]; e < e1; e += K) {
+      int ix[K];
+      double v[K];
+#pragma unroll
+      for (int q = 0; q < K; ++q)
+        if (e + q < e1) { ix[q] = __ldg(L.a.index + e + q); v[q] = __ldg(L.a.value + e + q); }
+#pragma unroll
+      for (int q = 0; q < K; ++q)
+        if (e + q < e1) s = fma(v[q], x[ix[q]], s);
+    }
+  } else {
+    const int M = L.M, N = L.N;
+    const double* a = sm + L.aoff + i;
+    dg = a[St<D, 1>::CENTER * N];
+#pragma unroll
+    for (int oz = (D > 2 ? -1 : 0); oz <= (D > 2 ? 1 : 0); ++oz)
+#pragma unroll
+      for (int oy = (D > 1 ? -1 : 0); oy <= (D > 1 ? 1 : 0); ++oy)
+#pragma unroll
+        for (int ox = -1; ox <= 1; ++ox) {
+          s = fma(*a, x[min(max(i + ox + M * (oy + M * oz), 0), N - 1)], s);
+          a += N;
+        }
+  }
+  return s;
+}
+
+// row sum of a transfer matrix, the vector in shared memory
+__device__ __forceinline__ double tail_csr_sum(const CsrView& a, const double* x, int i) {
+  double s = 0.0;
+  for (long long e = a.start[i]; e < a.start[i + 1]; ++e) s = fma(__ldg(a.value + e), x[__ldg(a.index + e)], s);
+  return s;
+}
+
+template <int D, bool CSR, int CAP>
+__global__ void __launch_bounds__(kTailT, 1)
+k_tail(const __grid_constant__ TailArgs<CAP> g) {
+  extern __shared__ double sm[];
+  __shared__ TailOp ops[CAP];
+  __shared__ TailLevel lv[Tail::kLev];
+  __shared__ TailVec vc[Tail::kVec];
+  const int tid = threadIdx.x;
+  const long long bq = blockIdx.x;  // problem of a batch
+  pdl_next();
+  {
+    auto copy = [&](void* dst, const void* src, int bytes) {
+      for (int k = tid; k < bytes / 4; k += kTailT) static_cast<int*>(dst)[k] = static_cast<const int*>(src)[k];
+    };
+    copy(ops, g.ops, g.nops * (int)sizeof(TailOp));
+    copy(lv, g.lev, g.nlev * (int)sizeof(TailLevel));
+    copy(vc, g.vec, g.nvec * (int)sizeof(TailVec));
+  }
+  __syncthreads();
+  // background copies (cp.async): every level's matrix and every vector in flight
+  if constexpr (!CSR) {
+    constexpr int NS = St<D, 1>::NS;
+    for (int l = 0; l < g.nlev; ++l) {
+      const int N = lv[l].N;
+      const long long Np = lv[l].Np;
+      const double* A = lv[l].A + bq * NS * Np;
+      double* d = sm + lv[l].aoff;
+      for (int i = tid; i < N; i += kTailT)
+#pragma unroll
+        for (int s = 0; s < NS; ++s) cp_async8(d + s * N + i, A + s * Np + i);
+    }
+  }
+  pdl_wait();
+  for (int k = 0; k < g.nvec; ++k)
+    if (vc[k].in) {
+      const TailLevel& L = lv[vc[k].lev];
+      for (int i = tid; i < L.N; i += kTailT) cp_async8(sm + vc[k].off + i, vc[k].g + bq * L.Np + i);
+    }
+  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+  const int dmask = g.dmask;
+#pragma unroll 1
+  for (int o = 0; o < g.nops; ++o) {
+    __syncthreads();
+    const TailOp& op = ops[o];
+    // a warp without work goes straight to the next barrier: on the smallest
+    // levels the idle warps' decoding would be the step's time
+    const int n = op.n;
+    if ((tid & ~31) >= n) continue;
+    const TailLevel& L = lv[op.lev];
+    const int N = L.N;
+    double *x = sm + op.x, *y = sm + op.y, *r = sm + op.r, *b = sm + op.b;
+    const double* om = L.omega ? L.omega + bq * L.Np : nullptr;
+    switch (op.kind) {
+      case TAIL_RES:
+        for (int i = tid; i < n; i += kTailT) {
+          double dg;
+          const double s = tail_row<D, CSR>(L, sm, x, i, dg);
+          r[i] = b[i] - s;
+        }
+        break;
+      case TAIL_JACOBI:
+        for (int i = tid; i < n; i += kTailT) {
+          const double w = om ? __ldg(om + i) : op.w;
+          const double d = CSR ? __ldg(L.diag + i) : sm[L.aoff + St<D, 1>::CENTER * N + i];
+          const double t = r[i] / d;
+          if (op.flag) r[i] = t;
+          x[i] = fma(w, t, x[i]);
+        }
+        break;
+      case TAIL_JACOBI_RES:
+        for (int i = tid; i < n; i += kTailT) {
+          const double w = om ? __ldg(om + i) : op.w;
+          double dg;
+          const double s = tail_row<D, CSR>(L, sm, x, i, dg);
+          const double t = (b[i] - s) / dg;
+          if (op.flag) r[i] = t;
+          y[i] = fma(w, t, x[i]);
+        }
+        break;
+      case TAIL_SOR:
+      case TAIL_SSC: {
+        int nx = 1, ny = 1;
+        const int cx = op.flag & 1, cy = (op.flag >> 1) & 1, cz = (op.flag >> 2) & 1;
+        if (!CSR) {
+          nx = (L.M - cx + 1) / 2;
+          ny = D > 1 ? (L.M - cy + 1) / 2 : 1;
+        }
+        for (int u = tid; u < n; u += kTailT) {
+          int i;
+          if (CSR) {
+            i = __ldg(op.rows + u);
+          } else {
+            const int q = u / nx, jx = u - q * nx, jy = D > 1 ? q % ny : 0, jz = D > 2 ? q / ny : 0;
+            i = cx + 2 * jx + L.M * ((D > 1 ? cy + 2 * jy : 0) + L.M * (D > 2 ? cz + 2 * jz : 0));
+          }
+          const double w = op.kind == TAIL_SOR && om ? __ldg(om + i) : op.w;
+          double dg;
+          const double s = tail_row<D, CSR>(L, sm, x, i, dg);
+          const double rr = b[i] - s, tt = rr / dg;
+          r[i] = op.kind == TAIL_SSC ? rr : tt;
+          x[i] = fma(w, tt, x[i]);
+        }
+        break;
+      }
+      case TAIL_RESTRICT: {
+        const TailLevel& C = lv[op.clev];
+        for (int j = tid; j < n; j += kTailT) {
+          double acc;
+          if constexpr (CSR) {
+            acc = tail_csr_sum(L.pt, x, j);
+          } else {
+            const int q = j / C.M;
+            const int c[3] = {j - q * C.M, D > 1 ? q % C.M : 0, D > 2 ? q / C.M : 0};
+            acc = restrict_node<D, 1, 1, double, true>(c, C.M, L.M, dmask, x);
+          }
+          r[j] = acc;
+          b[j] = acc;
+          y[j] = 0.0;
+        }
+        break;
+      }
+      case TAIL_PROLONG: {
+        const TailLevel& C = lv[op.clev];
+        for (int i = tid; i < n; i += kTailT) {
+          if constexpr (CSR) {
+            if (L.p.start[i] == L.p.start[i + 1]) continue;  // constrained rows keep their value
+            y[i] = y[i] + tail_csr_sum(L.p, x, i);
+          } else {
+            const int q = i / L.M;
+            const int c[3] = {i - q * L.M, D > 1 ? q % L.M : 0, D > 2 ? q / L.M : 0};
+            bool dir = false;
+#pragma unroll
+            for (int k = 0; k < D; ++k) dir = dir || face_dir(c[k], L.M, k, dmask);
+            if (dir) continue;
+            y[i] = y[i] + prolong_node<D, 1, 1, double, true>(c, L.M, C.M, dmask, x);
+          }
+        }
+        break;
+      }
+      default: {  // TAIL_COARSE: at most 128 unknowns, four warps; r is read before it is written
+        const int nb = g.nbase;
+        double acc = 0.0;
+        if (tid < nb) {
+          const double* a = g.ainv + bq * nb * nb + tid;
+          int j = 0;
+          for (; j + 16 <= nb; j += 16) {
+            double c[16];
+#pragma unroll
+            for (int q = 0; q < 16; ++q) c[q] = __ldg(a + (j + q) * nb);
+#pragma unroll
+            for (int q = 0; q < 16; ++q) acc = fma(c[q], r[j + q], acc);
+          }
+          for (; j < nb; ++j) acc = fma(__ldg(a + j * nb), r[j], acc);
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (tid < nb) {
+          r[tid] = acc;
+          x[tid] = fma(op.w, acc, x[tid]);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  for (int k = 0; k < g.nvec; ++k)
+    if (vc[k].out) {
+      const TailLevel& L = lv[vc[k].lev];
+      for (int i = tid; i < L.N; i += kTailT) vc[k].g[bq * L.Np + i] = sm[vc[k].off + i];
+    }
+}
+
 // ---------------------------------------------------------- dispatchers
 #define FMG_DISPATCH(D_, P_, ...)                                             \
   do {                                                                        \
@@ -3609,6 +3852,143 @@ void launch_densify(const LevelView& L, double* Dm, cudaStream_t st) {
     constexpr int NS = St<D, P>::NS;
     k_densify<D, P><<<grid1(L.N * NS), kBlock, 0, st>>>(L.A, L.N, L.Np, L.M, Dm, lay);
   });
+}
+
+// ------------------------------------------------------------ small levels
+long long tail_need(const LevelView& L) {  // the matrix and four vectors
+  long long ns = 0;
+  if (!L.csr) {
+    ns = 1;
+    for (int k = 0; k < L.dim; ++k) ns *= 3;
+  }
+  return (ns + 4) * L.N;
+}
+
+// One CTA has 208 KB for the levels, half of it used in 3D: there a cycle takes
+// few steps for the matrix it brings in (9^3 and 5^3 nodes, 183 KB and seven
+// Jacobi steps: a 128^3-cell solve 8.0 -> 8.3 ms; 7^3 and 4^3 with their colours:
+// a cycle on 48^3 273 -> 258 us).  The problems of a batch share an SM where
+// there are more of them than SMs (a second wave would double the time).
+long long tail_room(int dim, int nb) { return (dim == 3 ? 104 : 208) * 1024 / 8 / ((nb + 147) / 148); }
+
+template <int CAP>
+static void tail_launch(const Tail& t, cudaStream_t st) {
+  TailArgs<CAP> a;
+  a.dmask = t.dmask; a.nbase = t.nbase; a.nops = t.nops; a.nlev = t.nlev; a.nvec = t.nvec;
+  a.ainv = t.ainv;
+  std::memcpy(a.lev, t.lev, t.nlev * sizeof(TailLevel));
+  std::memcpy(a.vec, t.vec, t.nvec * sizeof(TailVec));
+  std::memcpy(a.ops, t.ops, t.nops * sizeof(TailOp));
+  const size_t smem = t.used * sizeof(double);
+  auto go = [&](auto kern) {
+    if (smem > 32 * 1024)
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(tail_room(2, 1) * sizeof(double)));
+    launch_early(kern, (unsigned)t.nb, kTailT, smem, st, a);
+  };
+  if (t.csr) go(k_tail<1, true, CAP>);
+  else if (t.dim == 1) go(k_tail<1, false, CAP>);
+  else if (t.dim == 2) go(k_tail<2, false, CAP>);
+  else go(k_tail<3, false, CAP>);
+}
+
+void tail_flush(Tail& t, cudaStream_t st, bool leaving) {
+  if (!t.nops) return;
+  if (leaving) {
+    int high = 0;
+    for (int k = 1; k < t.nlev; ++k)
+      if (t.levid[k] > t.levid[high]) high = k;
+    for (int q = 0; q < t.nvec; ++q) t.vec[q].out = t.vec[q].out && t.vec[q].lev == high;
+  }
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  if (t.nops <= 48) tail_launch<48>(t, st);
+  else tail_launch<Tail::kOps>(t, st);
+  t.nops = t.nlev = t.nvec = t.used = 0;
+}
+
+// the table entry of grid level l
+static int tail_entry(Tail& t, int l, const LevelView& L) {
+  for (int k = 0; k < t.nlev; ++k)
+    if (t.levid[k] == l) return k;
+  const int k = t.nlev++;
+  t.levid[k] = l;
+  TailLevel& e = t.lev[k];
+  e.A = L.A; e.omega = L.omega; e.Np = L.Np; e.N = (int)L.N; e.M = (int)L.M;
+  e.a = L.a; e.p = L.p; e.pt = L.pt; e.diag = L.diag;
+  e.aoff = t.used;
+  if (!L.csr) t.used += (int)(tail_need(L) - 4 * L.N);
+  t.dim = L.dim; t.dmask = L.dmask; t.nb = L.nb; t.csr = L.csr;
+  return k;
+}
+
+// the place of vector v of table level k; read, written: what the step does
+// with it (a step that writes a vector without reading it writes all of it)
+static int tail_vec(Tail& t, int k, double* v, bool read, bool written) {
+  if (!v) return 0;
+  int q = 0;
+  while (q < t.nvec && t.vec[q].g != v) ++q;
+  if (q == t.nvec) {
+    t.vec[t.nvec++] = TailVec{v, t.used, k, read, false};
+    t.used += t.lev[k].N;
+  }
+  t.vec[q].out = t.vec[q].out || written;
+  return t.vec[q].off;
+}
+
+static bool tail_full(const Tail& t) {  // a step adds one operation, two levels and four vectors at most
+  return t.nops == Tail::kOps || t.nlev + 2 > Tail::kLev || t.nvec + 4 > Tail::kVec;
+}
+
+void tail_add(Tail& t, int l, const LevelView& L, const TailStep& s, cudaStream_t st, const LevelView* C) {
+  if (tail_full(t)) tail_flush(t, st, false);
+  TailOp op{};
+  op.kind = (short)s.kind;
+  op.flag = s.write_r ? 1 : 0;
+  op.w = s.w;
+  const int k = tail_entry(t, l, L), c = C ? tail_entry(t, l - 1, *C) : k;
+  op.lev = (short)k;
+  op.clev = (short)c;
+  // what each step reads (in) and writes (out) of x, y, r, b
+  bool xi = true, xo = false, yi = false, yo = false, ri = false, ro = false, bi = false, bo = false;
+  int kx = k, ky = k, kr = k, kb = k;
+  switch (s.kind) {
+    case TAIL_RES: bi = true; ro = true; break;
+    case TAIL_JACOBI: xo = true; ri = true; ro = s.write_r; break;
+    case TAIL_JACOBI_RES: bi = true; yo = true; ro = s.write_r; break;
+    case TAIL_RESTRICT: ky = kr = kb = c; yo = ro = bo = true; break;
+    case TAIL_PROLONG: kx = c; yi = yo = true; break;
+    default: xo = true; ri = ro = true;  // TAIL_COARSE
+  }
+  op.b = tail_vec(t, kb, bi || bo ? s.b : nullptr, bi, bo);
+  op.x = tail_vec(t, kx, s.x, xi, xo);
+  op.y = tail_vec(t, ky, yi || yo ? s.y : nullptr, yi, yo);
+  op.r = tail_vec(t, kr, ri || ro ? s.r : nullptr, ri, ro);
+  op.n = s.kind == TAIL_COARSE ? 128 : (int)(s.kind == TAIL_RESTRICT ? C->N : L.N);
+  t.ops[t.nops++] = op;
+}
+
+void tail_sweep(Tail& t, int l, const LevelView& L, bool ssc, double omega, double* x, double* b, double* r,
+                cudaStream_t st) {
+  const int ncol = L.csr ? L.ncol : 1 << L.dim;
+  for (int c = 0; c < ncol; ++c) {
+    if (L.csr && L.coff[c + 1] == L.coff[c]) continue;
+    if (tail_full(t)) tail_flush(t, st, false);
+    TailOp op{};
+    op.kind = ssc ? TAIL_SSC : TAIL_SOR;
+    op.flag = (short)c;
+    op.w = omega;
+    op.lev = (short)tail_entry(t, l, L);
+    op.b = tail_vec(t, op.lev, b, true, false);
+    op.x = tail_vec(t, op.lev, x, true, true);
+    op.r = tail_vec(t, op.lev, r, true, true);  // a colour writes its own rows only
+    if (L.csr) {
+      op.n = (int)(L.coff[c + 1] - L.coff[c]);
+      op.rows = L.crow + L.coff[c];
+    } else {
+      op.n = 1;
+      for (int k = 0; k < L.dim; ++k) op.n *= ((int)L.M - ((c >> k) & 1) + 1) / 2;
+    }
+    t.ops[t.nops++] = op;
+  }
 }
 
 }  // namespace fmg
