@@ -153,7 +153,8 @@ __device__ __forceinline__ T mf_out(T ax, T d, T xc, T bb, T o, bool use_wd) {
   return use_wd ? o * bb : o * (bb / d);
 }
 
-constexpr int kFX = 32, kFY = 16, kFZ = 32;   // tile: nodes along x, y; planes per CTA
+constexpr int kFX = 32, kFY = 16;             // tile: nodes along x, y
+constexpr int kFZ0 = 32, kFZ1 = 8;            // planes per CTA on large and on small grids
 constexpr int kFRows = kFY + 2;               // x rows of a plane (y0-1 .. y0+16)
 constexpr int kFCRows = kFY + 1;              // cell rows of a plane (y0-1 .. y0+15)
 constexpr int kFPW = kFX + 2;                 // packed row: x0-1 .. x0+32
@@ -173,6 +174,7 @@ struct CellBox {
 
 struct MftGeo {
   int nbx, nby, nbz, nmain;   // tiled box: nbx x nby x nbz tiles from the origin
+  int fz;                     // planes a tiled CTA marches through
   int nface;                  // face CTAs (they come first in the grid)
   long long X1, Y1, Z1;       // the tiled box's extents in nodes
   int ax, ay, az;             // the tiled CTAs write [ax, X1) x [ay, Y1) x [az, Z1) (1: the face at 0 is left out)
@@ -338,7 +340,8 @@ __device__ __forceinline__ void cpa_arrive(uint64_t* bar) {
 
 // OPT: 1 per-node damping present (g.wd or g.omega), 2 a second reduction
 // vector, 4 the damping already divided by the diagonal (g.wd)
-template <typename T, typename TV, typename TX, int MODE, bool RED, int OPT>
+// FZ: planes a CTA marches through (MftGeo::fz)
+template <typename T, typename TV, typename TX, int MODE, bool RED, int OPT, int FZ>
 __global__ void __launch_bounds__(kFThreads, (sizeof(T) == 4 && MODE != 2) ? 3 : 2)
 k_mfc(MFArgsT<T> g, const __grid_constant__ CUtensorMap tk_cells, const __grid_constant__ CUtensorMap tm_x,
       const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_o,
@@ -364,7 +367,7 @@ k_mfc(MFArgsT<T> g, const __grid_constant__ CUtensorMap tk_cells, const __grid_c
     const T hs = g.hs;
     const int bid = (int)blockIdx.x - geo.nface;
     const int bx = bid % geo.nbx, by = (bid / geo.nbx) % geo.nby, bz = bid / (geo.nbx * geo.nby);
-    const int x0 = bx * kFX, y0 = by * kFY, z0 = bz * kFZ;
+    const int x0 = bx * kFX, y0 = by * kFY, z0 = bz * FZ;
     const int lx = tid & 31, ly = tid >> 5;
     constexpr int NR = L::NR, LOOK = L::LOOK;
     uint64_t* full = reinterpret_cast<uint64_t*>(sm + NR * L::SB);
@@ -381,7 +384,7 @@ k_mfc(MFArgsT<T> g, const __grid_constant__ CUtensorMap tk_cells, const __grid_c
     const int lox = dm & 1, loy = (dm >> 2) & 1, loz = (dm >> 4) & 1;
     const int xoff = (3 - lox) & 3;
     const int fr = g.ol.front;  // operand boxes start at tensor x0: node x0 + c at column c + front
-    const int last = kFZ + 1;
+    constexpr int last = FZ + 1;
     // this thread's share of the x halo: elements tid, tid+256, tid+512 of 18 x 34
     int hoff[3];
     bool hok[3];
@@ -546,13 +549,13 @@ k_mfc(MFArgsT<T> g, const __grid_constant__ CUtensorMap tk_cells, const __grid_c
     typedef std::integral_constant<int, 5> Q5;
     int t = 0;
 #pragma unroll 1
-    for (; t + 3 <= kFZ; t += 3) {
+    for (; t + 3 <= FZ; t += 3) {
       step(Q0{}, t);
       step(Q1{}, t + 1);
       step(Q2{}, t + 2);
     }
-    if constexpr (kFZ % 3 > 0) step(Q0{}, t);
-    if constexpr (kFZ % 3 > 1) step(Q1{}, t + 1);
+    if constexpr (FZ % 3 > 0) step(Q0{}, t);
+    if constexpr (FZ % 3 > 1) step(Q1{}, t + 1);
     // every stage requested has been waited for; a wait that gave up voids the results
     asm volatile("cp.async.wait_all;" ::: "memory");
     if (__syncthreads_or(!ok) && tid == 0 && g.err) *g.err = 1.0;
@@ -586,15 +589,18 @@ __device__ __forceinline__ long long soff(int s, long long M) {
 // bandwidth-bound; one row per thread on the small, latency-bound ones (and
 // on the 125-slot 3D Q2 rows, whose four-row form would spill).  Each row
 // sums in slot order either way.
+// The one-row form of up to 27 slots fetches its coefficients while the
+// previous launch still runs and has all its loads in flight (the launch bound
+// keeps the compiler from sinking them).
 template <int D, int P, int MODE, typename TB, typename TY, bool RED, int RPT>
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kBlock, RPT == 1 && P == 1 ? 3 : 1)
 k_st32(const float* __restrict__ A, long long N, long long Np, long long M, float w, const float* __restrict__ om,
        const float* __restrict__ x, const TB* __restrict__ b, TY* __restrict__ y, const double* __restrict__ v,
        const double* __restrict__ v2, Reduce2 R) {
   pdl_next();
-  pdl_wait();
   constexpr int NS = St32<D, P>::NS;
   constexpr int C = St32<D, P>::CENTER;
+  constexpr bool STAGE = RPT == 1 && NS <= 27;
   static_assert(RPT == 1 || RPT == 4, "one or four rows per thread");
   __shared__ double smem[8];
   double acc0 = 0.0, acc1 = 0.0;
@@ -603,9 +609,26 @@ k_st32(const float* __restrict__ A, long long N, long long Np, long long M, floa
     float s[RPT], d[RPT], xc[RPT];
 #pragma unroll
     for (int r = 0; r < RPT; ++r) s[r] = xc[r] = 0.f;
+    if constexpr (STAGE) {
+      float a[NS], xv[NS];
+#pragma unroll
+      for (int k = 0; k < NS; ++k)
+        if (MODE != 3 || k == C) a[k] = __ldg(A + (long long)k * Np + i0);
+      d[0] = a[C];
+      pdl_wait();
+      if (MODE != 3) {
+#pragma unroll
+        for (int k = 0; k < NS; ++k) xv[k] = __ldg(x + clampi(i0 + soff<D, P>(k, M), N));
+#pragma unroll
+        for (int k = 0; k < NS; ++k) s[0] = fmaf(a[k], xv[k], s[0]);
+        xc[0] = xv[C];
+      }
+    } else {
+      pdl_wait();
+    }
 #pragma unroll
     for (int k = 0; k < NS; ++k) {
-      if (MODE == 3 && k != C) continue;
+      if (STAGE || (MODE == 3 && k != C)) continue;
       float a[RPT];
       if constexpr (RPT == 4) {
         const float4 a4 = __ldg(reinterpret_cast<const float4*>(A + (long long)k * Np + i0));
@@ -644,7 +667,10 @@ k_st32(const float* __restrict__ A, long long N, long long Np, long long M, floa
       }
     }
   }
-  if (RED) dr_finish2(acc0, acc1, R, smem);
+  if (RED) {
+    pdl_wait();
+    dr_finish2(acc0, acc1, R, smem);
+  }
 }
 
 __device__ __forceinline__ bool fdir(int c, int M, int k, int dmask) {
@@ -1102,11 +1128,30 @@ k_prolong_mx(int MF, int MC, int dmask, const float* __restrict__ xc, float* __r
 __global__ void __launch_bounds__(1024)
 k_coarse_mx(const double* __restrict__ AinvT, int n, const __nv_bfloat16* __restrict__ b, float* __restrict__ x) {
   pdl_next();
-  pdl_wait();
   __shared__ double rs[1024];
+  const int l8 = threadIdx.x & 7;
+  if (n <= 128) {  // a row per eight lanes, its coefficients fetched before the wait
+    const int i = threadIdx.x >> 3;
+    double a[16];
+#pragma unroll
+    for (int q = 0; q < 16; ++q)
+      if (i < n && l8 + 8 * q < n) a[q] = __ldg(AinvT + (long long)(l8 + 8 * q) * n + i);
+    pdl_wait();
+    if (threadIdx.x < n) rs[threadIdx.x] = (double)__bfloat162float(b[threadIdx.x]);
+    __syncthreads();
+    double acc = 0.0;
+#pragma unroll
+    for (int q = 0; q < 16; ++q)
+      if (i < n && l8 + 8 * q < n) acc = fma(a[q], rs[l8 + 8 * q], acc);
+    acc += __shfl_xor_sync(0xffffffffu, acc, 4);
+    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+    if (i < n && l8 == 0) x[i] = (float)acc;
+    return;
+  }
+  pdl_wait();
   for (int i = threadIdx.x; i < n; i += 1024) rs[i] = (double)__bfloat162float(b[i]);
   __syncthreads();
-  const int l8 = threadIdx.x & 7;
   for (int base = (threadIdx.x >> 5) * 4; base < n; base += 128) {  // warp-uniform: rows base .. base+3
     const int i = base + ((threadIdx.x >> 3) & 3);
     double acc = 0.0;
@@ -1254,19 +1299,24 @@ k_dot2_64(const double* __restrict__ xv, const float* __restrict__ yv, const dou
 
 static inline unsigned g1(long long n) { return (unsigned)((n + kBlock - 1) / kBlock); }
 
-// the tiled box (whole 32 x 16 x 32 tiles from the origin) and the nodes left
-// to the face CTAs: outside the box, and its Dirichlet faces x, y, z = 0
+// the tiled box (whole 32 x 16 x fz tiles from the origin) and the nodes left
+// to the face CTAs: outside the box, and its Dirichlet faces x, y, z = 0.  A
+// CTA marches through 32 planes where that gives two CTAs an SM, through 8 on
+// smaller grids, whose few long marches were the time (97^3 nodes: FP64
+// operator 25 -> 15 us, residual 19 -> 9, smoothing with the FCG dots 24 -> 14;
+// 16 planes give half of that, 4 lose some of it to the halo planes).
 static MftGeo mft_geo(int M, int dmask) {
   MftGeo q{};
   const int n = M - 1;
   q.nbx = n / kFX;
   q.nby = n / kFY;
-  q.nbz = n / kFZ;
+  q.fz = (long long)q.nbx * q.nby * (n / kFZ0) < 2 * 148 ? kFZ1 : kFZ0;
+  q.nbz = n / q.fz;
   if (q.nbx == 0 || q.nby == 0 || q.nbz == 0) q.nbx = q.nby = q.nbz = 0;
   q.nmain = q.nbx * q.nby * q.nbz;
   q.X1 = (long long)q.nbx * kFX;
   q.Y1 = (long long)q.nby * kFY;
-  q.Z1 = (long long)q.nbz * kFZ;
+  q.Z1 = (long long)q.nbz * q.fz;
   if (q.nmain > 0) {
     q.ax = (dmask & 1) ? 1 : 0;
     q.ay = (dmask & 4) ? 1 : 0;
@@ -1384,7 +1434,7 @@ static void mft_launch(const MFArgsT<T>& g, const TX* x, const T* b, T* y, const
            (!(L::HV && v2) || op_map<TV>(v2, g.ol, g.M, &tv2));
   }
   if (!maps) {
-    q = MftGeo{};
+    q = MftGeo{};  // every node by the face CTAs
     q.F = g.N;
     q.nface = (int)((q.F + kFaceNodes - 1) / kFaceNodes);
   }
@@ -1394,14 +1444,18 @@ static void mft_launch(const MFArgsT<T>& g, const TX* x, const T* b, T* y, const
   const int opt = (HO && (g.wd || g.omega) ? 1 : 0) | (RED && v2 ? 2 : 0) | (HO && g.wd ? 4 : 0);
   auto go = [&](auto oc) {
     constexpr int OPT = decltype(oc)::value;
-    auto kern = k_mfc<T, TV, TX, MODE, RED, OPT>;
-    constexpr int smem = L::SMEM;
-    static unsigned attr = 0;  // devices the shared-memory size was raised on
-    if (dev < 32 && !((attr >> dev) & 1u)) {
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      attr |= 1u << dev;
-    }
-    launch_pdl(kern, mft_blocks(q), kFThreads, smem, st, g, tk, tx, tb, to, tv, tv2, q, x, b, y, v, v2, R);
+    auto run = [&](auto fc) {
+      auto kern = k_mfc<T, TV, TX, MODE, RED, OPT, decltype(fc)::value>;
+      constexpr int smem = L::SMEM;
+      static unsigned attr = 0;  // devices the shared-memory size was raised on
+      if (dev < 32 && !((attr >> dev) & 1u)) {
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        attr |= 1u << dev;
+      }
+      launch_pdl(kern, mft_blocks(q), kFThreads, smem, st, g, tk, tx, tb, to, tv, tv2, q, x, b, y, v, v2, R);
+    };
+    if (q.fz == kFZ1) run(std::integral_constant<int, kFZ1>{});
+    else run(std::integral_constant<int, kFZ0>{});
   };
   switch (opt) {
     case 1: if constexpr (HO) go(std::integral_constant<int, 1>{}); break;
@@ -1556,7 +1610,7 @@ void st32_launch(const Lev32& L, const float* x, const void* b, void* y, const d
   if (W == 4 && L.N >= kSt32Wide)
     launch_pdl(k_st32<D, P, MODE, TB, TY, RED, W>, g1((L.N + W - 1) / W), kBlock, 0, st, L.A, L.N, L.Np, L.M, L.w, L.om, x, (const TB*)b, (TY*)y, v, v2, r0);
   else
-    launch_pdl(k_st32<D, P, MODE, TB, TY, RED, 1>, g1(L.N), kBlock, 0, st, L.A, L.N, L.Np, L.M, L.w, L.om, x,
+    launch_early(k_st32<D, P, MODE, TB, TY, RED, 1>, g1(L.N), kBlock, 0, st, L.A, L.N, L.Np, L.M, L.w, L.om, x,
                                                                     (const TB*)b, (TY*)y, v, v2, r0);
 }
 
