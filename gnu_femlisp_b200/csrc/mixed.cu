@@ -593,7 +593,7 @@ __device__ __forceinline__ long long soff(int s, long long M) {
 // previous launch still runs and has all its loads in flight (the launch bound
 // keeps the compiler from sinking them).
 template <int D, int P, int MODE, typename TB, typename TY, bool RED, int RPT>
-__global__ void __launch_bounds__(kBlock, RPT == 1 && P == 1 ? 3 : 1)
+__global__ void __launch_bounds__(kBlock, RPT == 1 && P == 1 ? 3 : P == 1 ? 2 : 0)
 k_st32(const float* __restrict__ A, long long N, long long Np, long long M, float w, const float* __restrict__ om,
        const float* __restrict__ x, const TB* __restrict__ b, TY* __restrict__ y, const double* __restrict__ v,
        const double* __restrict__ v2, Reduce2 R) {
