@@ -563,7 +563,7 @@ def run_mine(args, world, rank, local):
                      "top_level_kernels": top_kernels},
         "matvec_roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                             "frac": achieved / peak, "traffic": 233.7 * n,
-                            "kernel": "k_spmv<3,1> (top-level FP64 matvec of the assembled matrix, plain path)",
+                            "kernel": "k_row_q1<3> (top-level FP64 matvec of the assembled matrix, plain path)",
                             "peak_kind": peak_kind, "algorithmic_bytes": alg_bytes, "launch_ms": t_mv * 1e3},
         "e2e": {"value": world * n / t_e2e_max / 1e6, "unit": "MDoF/s to 1e-10 (N_top / time-to-solution)",
                 "h2d_bytes_per_step": int(k_np.nbytes), "d2h_bytes_per_step": int(x_np.nbytes),
@@ -1036,7 +1036,7 @@ def run_c2(args):
             "vcycle_ms": t_cycle * 1e3, "mdof_per_s_per_vcycle": n / t_cycle / 1e6,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": None,
-                         "kernel": "k_spmv<3,2> (top-level FP64 Q2 matvec)", "peak_kind": peak_kind,
+                         "kernel": "k_spmv_q2c<3> (top-level FP64 Q2 matvec)", "peak_kind": peak_kind,
                          "algorithmic_bytes": alg_bytes, "launch_ms": t_mv * 1e3},
             "cpu_baseline": cpu, "parity": par, "clocks": clk,
             "history_tail": [float(v) for v in hist[-3:]], "ssc": ssc}
@@ -1186,7 +1186,7 @@ def run_c5(args):
             "vcycle_ms": t_cycle * 1e3, "mdof_per_s_per_vcycle": nd / t_cycle / 1e6,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": None,
-                         "kernel": "k_spmv3<2> (top-level FP64 block matvec)", "peak_kind": peak_kind,
+                         "kernel": "k_row3<2> (top-level FP64 block matvec)", "peak_kind": peak_kind,
                          "algorithmic_bytes": alg_bytes, "launch_ms": t_mv * 1e3},
             "cpu_baseline": cpu, "clocks": clk,
             "history_tail": [float(v) for v in hist[-3:]]}

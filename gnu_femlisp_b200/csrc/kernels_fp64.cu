@@ -127,36 +127,6 @@ __host__ __device__ __forceinline__ void q2_rows(const long long c[3], long long
   }
 }
 
-// Visits the stored slots of Q2 node c in ascending slot order (the order of
-// every row sum): f(slot, neighbour offset, position in the slot's array).
-// The z and y offsets are loops, the 5 x offsets unrolled; the row's index
-// in a slot array depends only on which directions the slot restricts.
-template <int D, typename F>
-__device__ __forceinline__ void q2_row(const long long c[3], long long M, F&& f) {
-  const long long H = (M + 1) / 2;
-  const bool ex = !(c[0] & 1), ey = D > 1 && !(c[1] & 1), ez = D > 2 && !(c[2] & 1);
-  for (int sz = 0; sz < (D > 2 ? 5 : 1); ++sz) {
-    const int oz = D > 2 ? sz - 2 : 0;
-    const bool rz = oz == 2 || oz == -2;
-    if (rz && !ez) continue;
-    for (int sy = 0; sy < (D > 1 ? 5 : 1); ++sy) {
-      const int oy = D > 1 ? sy - 2 : 0;
-      const bool ry = oy == 2 || oy == -2;
-      if (ry && !ey) continue;
-      const long long yz = (ry ? c[1] / 2 : c[1]) + (ry ? H : M) * (rz ? c[2] / 2 : c[2]);
-      const long long p0 = c[0] + M * yz, p1 = c[0] / 2 + H * yz;
-      const long long obase = (long long)oy * M + (long long)oz * M * M;
-#pragma unroll
-      for (int sx = 0; sx < 5; ++sx) {
-        const int ox = sx - 2;
-        const bool rx = ox == 2 || ox == -2;
-        if (rx && !ex) continue;
-        f(sx + 5 * (sy + 5 * sz), obase + ox, rx ? p1 : p0);
-      }
-    }
-  }
-}
-
 // Scalar Q2 levels go one step further: rows are grouped by colour class
 // (coordinates mod 3 -- the classes of the multicolour <sor>), classes in
 // ascending order, and inside a class a slot array holds the rows that admit
@@ -222,50 +192,10 @@ __host__ __device__ __forceinline__ long long q2c_pos(const Q2Layout& L, const l
   return L.off[col][r] + p;
 }
 
-// q2_row for the colour-major layout of scalar Q2 levels
-template <int D, typename F>
-__device__ __forceinline__ void q2c_row(const Q2Layout& L, const long long c[3], long long M, F&& f) {
-  int col = 0, m3 = 1;
-  long long j[3][2] = {{0, 0}, {0, 0}, {0, 0}}, e[3][2] = {{1, 1}, {1, 1}, {1, 1}};
-  bool ev[3] = {false, false, false};
-  for (int k = 0; k < D; ++k) {
-    const int d = (int)(c[k] % 3);
-    col += d * m3;
-    m3 *= 3;
-    ev[k] = !(c[k] & 1);
-    for (int rk = 0; rk < 2; ++rk) {
-      j[k][rk] = q2c_j(c[k], d, rk);
-      e[k][rk] = q2c_ext(M, d, rk);
-    }
-  }
-  for (int sz = 0; sz < (D > 2 ? 5 : 1); ++sz) {
-    const int oz = D > 2 ? sz - 2 : 0;
-    const int rz = (oz == 2 || oz == -2) ? 1 : 0;
-    if (rz && !ev[2]) continue;
-    for (int sy = 0; sy < (D > 1 ? 5 : 1); ++sy) {
-      const int oy = D > 1 ? sy - 2 : 0;
-      const int ry = (oy == 2 || oy == -2) ? 1 : 0;
-      if (ry && !ev[1]) continue;
-      const long long yz = j[1][ry] + e[1][ry] * j[2][rz];
-      const long long b0 = L.off[col][(ry << 1) | (rz << 2)] + j[0][0] + e[0][0] * yz;
-      const long long b1 = L.off[col][1 | (ry << 1) | (rz << 2)] + j[0][1] + e[0][1] * yz;
-      const long long obase = (long long)oy * M + (long long)oz * M * M;
-#pragma unroll
-      for (int sx = 0; sx < 5; ++sx) {
-        const int ox = sx - 2;
-        const bool rx = ox == 2 || ox == -2;
-        if (rx && !ev[0]) continue;
-        f(sx + 5 * (sy + 5 * sz), obase + ox, rx ? b1 : b0);
-      }
-    }
-  }
-}
-
 // A node's position in the slot arrays of every pattern (32-bit: levels have
 // fewer than 2^31 nodes) and the patterns it admits, in the colour-major
 // layout of scalar Q2 levels (colour) or the natural sliced one (vector
-// levels); visited with every slot unrolled, so the pattern of a slot is a
-// compile-time constant and the loads can be issued ahead.
+// levels).
 template <int D>
 struct Q2Base {
   int p[1 << D];
@@ -311,25 +241,6 @@ __device__ __forceinline__ void q2_base(const Q2Layout& lay, const long long c[3
     const int p = j[0][rx] + e[0][rx] * (j[1][ry] + e[1][ry] * j[2][rz]);
     const int q = COLOUR ? lay.off[col][r] + p : p;
     b.p[r] = (CLAMP && q >= nmax) ? nmax - 1 : q;
-  }
-}
-
-// Visits every slot (structural zeros too): f(slot, neighbour offset,
-// position, stored).  A position is in bounds even where the slot is not
-// stored for the node (the halved coordinate of an odd one), so callers load
-// unconditionally and use 0 where !stored -- the structural zero the full
-// layout would hold, in the same place of the row sum -- which lets the
-// loads be issued ahead.
-// ALL = false visits only the stored slots (the streaming kernels); ALL =
-// true every slot, for the latency-bound colour sweeps of the SOR.
-template <int D, bool ALL, typename F>
-__device__ __forceinline__ void q2_visit(const Q2Base<D>& b, long long M, F&& f) {
-  constexpr int NS = D == 1 ? 5 : (D == 2 ? 25 : 125);
-#pragma unroll
-  for (int s = 0; s < NS; ++s) {
-    const int r = q2_pattern<D>(s);
-    const bool st = ((b.valid >> r) & 1) != 0;
-    if (ALL || st) f(s, slot_off<D, 2>(s, M), (long long)b.p[r], st);
   }
 }
 
@@ -1551,6 +1462,63 @@ k_restrict(int MC, int MF, int dmask, const double* __restrict__ rf, double* __r
   solc[J] = 0.0;
 }
 
+// The same on Q1 levels, a thread per pair of fine nodes 2 j, 2 j + 1 along x: the
+// pair shares its coarse values, every thread of a warp takes the same terms
+// (y and z are the warp's), and the loads and stores are coalesced.  Terms and
+// their order are prolong_node's.  Bound by HBM and the issue of its loads
+// (257^3 fine nodes: 99 us, 197 us with a thread per fine node).
+template <int D>
+__global__ void __launch_bounds__(kBlock)
+k_prolong_q1f(int MF, int MC, int dmask, const double* __restrict__ xc, double* __restrict__ xf, long long fs,
+              long long cs) {
+  pdl_next();
+  pdl_wait();
+  if (D == 1 && threadIdx.y != 0) return;
+  if (D < 3) {  // problem of a batched level
+    const long long bq = blockIdx.z;
+    xc += bq * cs;
+    xf += bq * fs;
+  }
+  const int j = blockIdx.x * 32 + threadIdx.x;
+  const int fy = D > 1 ? (int)(blockIdx.y * 8 + threadIdx.y) : 0, fz = D > 2 ? (int)blockIdx.z : 0;
+  if (j >= MC || fy >= MF) return;
+  if (D > 1 && face_dir(fy, MF, 1, dmask)) return;
+  if (D > 2 && face_dir(fz, MF, 2, dmask)) return;
+  const int ny = D > 1 && (fy & 1) ? 2 : 1, nz = D > 2 && (fz & 1) ? 2 : 1;
+  const bool x0 = !face_dir(j, MC, 0, dmask), x1 = j + 1 < MC && !face_dir(j + 1, MC, 0, dmask);
+  constexpr int NY = D > 1 ? 2 : 1, NZ = D > 2 ? 2 : 1;
+  bool on[NZ][NY];
+  double v[NZ][NY][2];
+#pragma unroll
+  for (int z = 0; z < NZ; ++z)
+#pragma unroll
+    for (int y = 0; y < NY; ++y) {
+      const int cy = (fy >> 1) + y, cz = (fz >> 1) + z;
+      on[z][y] = y < ny && z < nz && (D < 2 || !face_dir(cy, MC, 1, dmask)) && (D < 3 || !face_dir(cz, MC, 2, dmask));
+      const double* c = xc + j + (long long)MC * (cy + (long long)MC * cz);
+      v[z][y][0] = on[z][y] && x0 ? __ldg(c) : 0.0;
+      v[z][y][1] = on[z][y] && x1 ? __ldg(c + 1) : 0.0;
+    }
+  double* f = xf + 2 * j + (long long)MF * (fy + (long long)MF * fz);
+  const bool w0 = !face_dir(2 * j, MF, 0, dmask), w1 = j + 1 < MC;  // an odd node lies on no face
+  const double f0 = w0 ? f[0] : 0.0, f1 = w1 ? f[1] : 0.0;
+  double e = 0.0, o = 0.0;
+#pragma unroll
+  for (int z = 0; z < NZ; ++z)
+#pragma unroll
+    for (int y = 0; y < NY; ++y)
+      if (on[z][y]) {
+        const double w = (ny == 2 ? 0.5 : 1.0) * (nz == 2 ? 0.5 : 1.0);
+        if (x0) {
+          e = fma(w, v[z][y][0], e);
+          o = fma(0.5 * w, v[z][y][0], o);
+        }
+        if (x1) o = fma(0.5 * w, v[z][y][1], o);
+      }
+  if (w0) f[0] = f0 + e;
+  if (w1) f[1] = f1 + o;
+}
+
 // xf := xf + I xc (constrained) (prolongate, multigrid.lisp:237-239)
 template <int D, int P>
 __global__ void __launch_bounds__(kBlock)
@@ -1924,7 +1892,7 @@ __global__ void k_axpy(double alpha, const double* __restrict__ sc, int aslot, c
 }
 
 // DR4096 dot product (x, y)
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kBlock, 4)
 k_dot(const double* __restrict__ x, const double* __restrict__ y, long long n, Reduce R, long long vs) {
   pdl_next();
   pdl_wait();
@@ -1934,19 +1902,36 @@ k_dot(const double* __restrict__ x, const double* __restrict__ y, long long n, R
   y += bq * vs;
   R = batch_reduce(R, (unsigned)bq);
   const long long base = (long long)blockIdx.x * kChunk + 2 * threadIdx.x;
+  // pairs by 16-byte loads (every vector starts on 16 bytes), four at a time
+  // before their terms
   double acc = 0.0;
 #pragma unroll
-  for (int m = 0; m < kPairsPerThread; ++m) {
-    const long long i0 = base + 512LL * m;
-    if (i0 < n) acc = fma(x[i0], y[i0], acc);
-    if (i0 + 1 < n) acc = fma(x[i0 + 1], y[i0 + 1], acc);
+  for (int m0 = 0; m0 < kPairsPerThread; m0 += 4) {
+    double2 u[4], v[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const long long i0 = base + 512LL * (m0 + m);
+      if (i0 + 1 < n) {
+        u[m] = __ldg(reinterpret_cast<const double2*>(x + i0));
+        v[m] = __ldg(reinterpret_cast<const double2*>(y + i0));
+      } else if (i0 < n) {
+        u[m].x = __ldg(x + i0);
+        v[m].x = __ldg(y + i0);
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const long long i0 = base + 512LL * (m0 + m);
+      if (i0 < n) acc = fma(u[m].x, v[m].x, acc);
+      if (i0 + 1 < n) acc = fma(u[m].y, v[m].y, acc);
+    }
   }
   dr_finish(acc, R, smem);
 }
 
 // CG update (krylow.lisp:117-121): x += lam p; r -= lam a; fused (r,r);
 // then w := r and (optionally) w2 := r, q := 0 for the preconditioner call
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kBlock, 3)
 k_cg_update(const double* __restrict__ sc, double* __restrict__ x, const double* __restrict__ p,
             double* __restrict__ r, const double* __restrict__ a, double* __restrict__ w,
             double* __restrict__ w2, double* __restrict__ q, long long n, Reduce R, long long vs,
@@ -1968,22 +1953,35 @@ k_cg_update(const double* __restrict__ sc, double* __restrict__ x, const double*
   const double lam = sc[S_LAM], nlam = sc[S_NEGLAM];
   const long long base = (long long)blockIdx.x * kChunk + 2 * threadIdx.x;
   double acc = 0.0;
-#pragma unroll 2
+  // pairs by 16-byte accesses (every vector starts on 16 bytes), several in flight
+#pragma unroll 4
   for (int m = 0; m < kPairsPerThread; ++m) {
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const long long i = base + 512LL * m + u;
-      if (i < n) {
-        const double rn = fz ? r[i] : fma(nlam, a[i], r[i]);
-        if (!fz) {
-          x[i] = fma(lam, p[i], x[i]);
-          r[i] = rn;
-        }
-        acc = fma(rn, rn, acc);
-        if (w) w[i] = rn;
-        if (w2) w2[i] = rn;
-        if (q) q[i] = 0.0;
+    const long long i = base + 512LL * m;
+    if (i + 1 < n) {
+      const double2 ri = *reinterpret_cast<const double2*>(r + i);
+      double2 rn = ri;
+      if (!fz) {
+        const double2 ai = *reinterpret_cast<const double2*>(a + i), pi = *reinterpret_cast<const double2*>(p + i),
+                      xi = *reinterpret_cast<const double2*>(x + i);
+        rn = make_double2(fma(nlam, ai.x, ri.x), fma(nlam, ai.y, ri.y));
+        *reinterpret_cast<double2*>(x + i) = make_double2(fma(lam, pi.x, xi.x), fma(lam, pi.y, xi.y));
+        *reinterpret_cast<double2*>(r + i) = rn;
       }
+      acc = fma(rn.x, rn.x, acc);
+      acc = fma(rn.y, rn.y, acc);
+      if (w) *reinterpret_cast<double2*>(w + i) = rn;
+      if (w2) *reinterpret_cast<double2*>(w2 + i) = rn;
+      if (q) *reinterpret_cast<double2*>(q + i) = make_double2(0.0, 0.0);
+    } else if (i < n) {
+      const double rn = fz ? r[i] : fma(nlam, a[i], r[i]);
+      if (!fz) {
+        x[i] = fma(lam, p[i], x[i]);
+        r[i] = rn;
+      }
+      acc = fma(rn, rn, acc);
+      if (w) w[i] = rn;
+      if (w2) w2[i] = rn;
+      if (q) q[i] = 0.0;
     }
   }
   dr_finish(acc, R, smem);
@@ -2519,7 +2517,8 @@ static void launch_row3(int order, const T* A, long long N, long long Np, long l
     }
     if (smem > 48 * 1024)
       cudaFuncSetAttribute(k_row3<P, T, OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_late(k_row3<P, T, OP>, grid, kRow3T, smem, st, A, (int)N, Np, (int)M, damp, omega, x, b, y, r, write_r ? 1 : 0);
+    launch_late(k_row3<P, T, OP>, grid, kRow3T, smem, st,
+                A, (int)N, Np, (int)M, damp, omega, x, b, y, r, write_r ? 1 : 0);
   };
   if (order == 2) go(std::integral_constant<int, 2>{});
   else go(std::integral_constant<int, 1>{});
@@ -3349,7 +3348,8 @@ void launch_jacobi(const LevelView& L, double damp, double* x, double* r, bool w
   if (L.order == 2) {  // colour-major sliced storage
     const Q2Layout lay = q2_layout(L.dim, L.M);
     Q2_DISPATCH(L.dim, {
-      launch_early(k_jacobi_q2<D>, grid1(L.N), kBlock, 0, st, L.A, L.N, L.Np, L.M, damp, L.omega, x, r, write_r ? 1 : 0, lay);
+      launch_early(k_jacobi_q2<D>, grid1(L.N), kBlock, 0, st,
+                   L.A, L.N, L.Np, L.M, damp, L.omega, x, r, write_r ? 1 : 0, lay);
     });
     return;
   }
@@ -3377,7 +3377,8 @@ void launch_jacobi_res(const LevelView& L, double damp, const double* x, const d
   if (L.order == 2) {  // rows by colour class and parity
     const Q2Layout lay = q2_layout(L.dim, L.M);
     Q2_DISPATCH(L.dim, {
-      launch_pdl(k_jacobi_res_q2c<D>, q2_grid<D>((int)L.M), kQ2T, 0, st, L.A, L.Np, (int)L.M, damp, L.omega, x, b, xout, r,
+      launch_pdl(k_jacobi_res_q2c<D>, q2_grid<D>((int)L.M), kQ2T, 0, st,
+                 L.A, L.Np, (int)L.M, damp, L.omega, x, b, xout, r,
                                                                  write_r ? 1 : 0, lay);
     });
     if (dv) launch_dot(xout, dv, L.N, *R, st);
@@ -3397,7 +3398,8 @@ static void launch_csr_sor(const LevelView& L, double omega, const double* om, d
   for (int c = 0; c < L.ncol; ++c) {
     const long long cnt = L.coff[c + 1] - L.coff[c];
     if (cnt > 0)
-      launch_early(k_csr_sor, grid1(cnt, kCsrT), kCsrT, 0, st, L.crow + L.coff[c], cnt, L.a, L.diag, omega, om, x, b, r, ssc ? 1 : 0);
+      launch_early(k_csr_sor, grid1(cnt, kCsrT), kCsrT, 0, st,
+                   L.crow + L.coff[c], cnt, L.a, L.diag, omega, om, x, b, r, ssc ? 1 : 0);
   }
 }
 
@@ -3426,7 +3428,8 @@ void launch_sor(const LevelView& L, double omega, double* x, const double* b, do
       });
     } else {
       Q1_DISPATCH(L.dim, {
-        launch_early(k_sor_colour<D, 1>, grid1(cnt, kRowT), kRowT, 0, st, L.A, L.N, L.Np, L.M, col, omega, L.omega, x, b, r);
+        launch_early(k_sor_colour<D, 1>, grid1(cnt, kRowT), kRowT, 0, st,
+                     L.A, L.N, L.Np, L.M, col, omega, L.omega, x, b, r);
       });
     }
   }
@@ -3464,7 +3467,8 @@ void launch_ssc(const LevelView& L, double omega, double* x, const double* b, do
       if (L.dim > 1) cnt *= (L.M - cy + 1) / 2;
       if (L.dim > 2) cnt *= (L.M - cz + 1) / 2;
       Q1_DISPATCH(L.dim, {
-        launch_early(k_sor_colour<D, 1, true>, grid1(cnt, kRowT), kRowT, 0, st, L.A, L.N, L.Np, L.M, col, omega, nullptr, x, b, r);
+        launch_early(k_sor_colour<D, 1, true>, grid1(cnt, kRowT), kRowT, 0, st,
+                     L.A, L.N, L.Np, L.M, col, omega, nullptr, x, b, r);
       });
     }
     return;
@@ -3523,7 +3527,8 @@ void launch_restrict(const LevelView& F, const LevelView& Cl, const double* rf, 
   FMG_DISPATCH(F.dim, F.order, {
     dim3 gr = xfer_grid(Cl.M, D);
     if (D < 3) gr.z = (unsigned)F.nb;  // the problems of a batched level
-    launch_early(k_restrict<D, P>, gr, dim3(32, 8), 0, st, (int)Cl.M, (int)F.M, F.dmask, rf, rc, rhsc, solc, F.Np, Cl.Np);
+    launch_early(k_restrict<D, P>, gr, dim3(32, 8), 0, st,
+                 (int)Cl.M, (int)F.M, F.dmask, rf, rc, rhsc, solc, F.Np, Cl.Np);
   });
 }
 
@@ -3540,6 +3545,10 @@ void launch_prolong(const LevelView& Cl, const LevelView& F, const double* xc, d
   FMG_DISPATCH(F.dim, F.order, {
     dim3 gr = xfer_grid(F.M, D);
     if (D < 3) gr.z = (unsigned)F.nb;
+    if constexpr (P == 1) {
+      gr.x = (unsigned)((Cl.M + 31) / 32);
+      launch_early(k_prolong_q1f<D>, gr, dim3(32, 8), 0, st, (int)F.M, (int)Cl.M, F.dmask, xc, xf, F.Np, Cl.Np);
+    } else
     launch_early(k_prolong<D, P>, gr, dim3(32, 8), 0, st, (int)F.M, (int)Cl.M, F.dmask, xc, xf, F.Np, Cl.Np);
   });
 }

@@ -1608,7 +1608,8 @@ void st32_launch(const Lev32& L, const float* x, const void* b, void* y, const d
                  const Reduce2& r0, cudaStream_t st) {
   constexpr int W = (D == 3 && P == 2) ? 1 : 4;
   if (W == 4 && L.N >= kSt32Wide)
-    launch_pdl(k_st32<D, P, MODE, TB, TY, RED, W>, g1((L.N + W - 1) / W), kBlock, 0, st, L.A, L.N, L.Np, L.M, L.w, L.om, x, (const TB*)b, (TY*)y, v, v2, r0);
+    launch_pdl(k_st32<D, P, MODE, TB, TY, RED, W>, g1((L.N + W - 1) / W), kBlock, 0, st,
+               L.A, L.N, L.Np, L.M, L.w, L.om, x, (const TB*)b, (TY*)y, v, v2, r0);
   else
     launch_early(k_st32<D, P, MODE, TB, TY, RED, 1>, g1(L.N), kBlock, 0, st, L.A, L.N, L.Np, L.M, L.w, L.om, x,
                                                                     (const TB*)b, (TY*)y, v, v2, r0);
@@ -1668,7 +1669,8 @@ void mx_restrict(const Lev32& F, const Lev32& C, const void* rf, bool rf_bf16, _
     return;
   }
   MX_DISPATCH(F.dim, F.order, {
-    if (rf_bf16) launch_pdl(k_restrict_mx<D, P, __nv_bfloat16>, gr, bl, 0, st, (int)C.M, (int)F.M, F.dmask, (const __nv_bfloat16*)rf, bc, xc);
+    if (rf_bf16) launch_pdl(k_restrict_mx<D, P, __nv_bfloat16>, gr, bl, 0, st,
+                            (int)C.M, (int)F.M, F.dmask, (const __nv_bfloat16*)rf, bc, xc);
     else launch_pdl(k_restrict_mx<D, P, float>, gr, bl, 0, st, (int)C.M, (int)F.M, F.dmask, (const float*)rf, bc, xc);
   });
 }
@@ -1678,9 +1680,11 @@ void mx_prolong(const Lev32& C, const Lev32& F, const float* xc, float* xf, cuda
   const dim3 gr = xgrid(F.M, F.dim), bl(32, 8);
   if (F.order == 1) {
     if (F.dim == 3 && xfl && xfl->py % 4 == 0 && xfl->pz % 4 == 0 && ((uintptr_t)xf & 15) == 0)
-      launch_pdl(k_prolong_q1v, dim3((unsigned)((xfl->py / 4 * C.M + kBlock - 1) / kBlock), (unsigned)C.M), kBlock, 0, st, (int)F.M, (int)C.M, F.dmask, xc, xf, *xfl);
+      launch_pdl(k_prolong_q1v, dim3((unsigned)((xfl->py / 4 * C.M + kBlock - 1) / kBlock), (unsigned)C.M), kBlock,
+                 0, st, (int)F.M, (int)C.M, F.dmask, xc, xf, *xfl);
     else if (F.dim == 3)
-      launch_pdl(k_prolong_q1c, dim3((unsigned)((C.M + 31) / 32), (unsigned)((C.M + 7) / 8), (unsigned)C.M), bl, 0, st, (int)F.M, (int)C.M, F.dmask, xc, xf, xfl ? *xfl : natural_lay((int)F.M, 3));
+      launch_pdl(k_prolong_q1c, dim3((unsigned)((C.M + 31) / 32), (unsigned)((C.M + 7) / 8), (unsigned)C.M), bl, 0,
+                 st, (int)F.M, (int)C.M, F.dmask, xc, xf, xfl ? *xfl : natural_lay((int)F.M, 3));
     else if (F.dim == 2) launch_pdl(k_prolong_q1<2>, gr, bl, 0, st, (int)F.M, (int)C.M, F.dmask, xc, xf);
     else launch_pdl(k_prolong_q1<1>, gr, bl, 0, st, (int)F.M, (int)C.M, F.dmask, xc, xf);
     return;
