@@ -430,7 +430,7 @@ struct MG {
       tail_top = -1;
       long long need = 0;
       const bool q1 = g->nc == 1 && (g->algebraic || g->order == 1);
-      for (int k = g->base; q1 && k <= g->top && k < g->base + Tail::kLev - 1; ++k) {
+      for (int k = g->base; q1 && k <= g->top && k < g->base + Tail::kLev - 2; ++k) {
         need += tail_need(view(g, k));
         if (need > tail_room(g->algebraic ? 1 : g->dim, g->nb)) break;
         tail_top = k;

@@ -1029,8 +1029,8 @@ k_ssc_factor_q2(const double* __restrict__ A, long long Np, long long M, int dma
 // direction) share no node and read no unknown another one writes, so the
 // residuals are those each block would form for itself.  Formed by the block's
 // own lanes, 27 rows of a warp scattered over the classes' arrays, they took
-// most of the colour's time: 65^3 nodes 107 us a colour, SSC65 us so; 17^3
-// 28 us, SSC17 us.
+// most of the colour's time: 65^3 nodes 107 us a colour, 45-54 us so; 17^3
+// 28 us, 8 us.
 // A Dirichlet node belongs to no block but its own.
 template <int D>
 __global__ void __launch_bounds__(kQ2T, kQ2MinBlocks<D>)
