@@ -1902,8 +1902,10 @@ k_dot(const double* __restrict__ x, const double* __restrict__ y, long long n, R
   y += bq * vs;
   R = batch_reduce(R, (unsigned)bq);
   const long long base = (long long)blockIdx.x * kChunk + 2 * threadIdx.x;
-  // pairs by 16-byte loads (every vector starts on 16 bytes), four at a time
-  // before their terms
+  // pairs by 16-byte loads, four at a time before their terms.  The library's
+  // own vectors start on 16 bytes; those a caller hands to fmg_dot_noalloc
+  // need only the 8 of a double, and then come one by one.
+  const bool wide = (((uintptr_t)x | (uintptr_t)y) & 15) == 0;
   double acc = 0.0;
 #pragma unroll
   for (int m0 = 0; m0 < kPairsPerThread; m0 += 4) {
@@ -1911,12 +1913,18 @@ k_dot(const double* __restrict__ x, const double* __restrict__ y, long long n, R
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
       const long long i0 = base + 512LL * (m0 + m);
-      if (i0 + 1 < n) {
+      if (wide && i0 + 1 < n) {
         u[m] = __ldg(reinterpret_cast<const double2*>(x + i0));
         v[m] = __ldg(reinterpret_cast<const double2*>(y + i0));
-      } else if (i0 < n) {
-        u[m].x = __ldg(x + i0);
-        v[m].x = __ldg(y + i0);
+      } else {
+        if (i0 < n) {
+          u[m].x = __ldg(x + i0);
+          v[m].x = __ldg(y + i0);
+        }
+        if (i0 + 1 < n) {
+          u[m].y = __ldg(x + i0 + 1);
+          v[m].y = __ldg(y + i0 + 1);
+        }
       }
     }
 #pragma unroll
