@@ -118,7 +118,12 @@ __device__ __forceinline__ void dr_finish(double lane_sum, const Reduce& R, doub
 // predecessor has finished and its writes are visible.  Every kernel launched
 // so calls both, pdl_wait before its first access to anything that a kernel
 // of the same sequence writes; before it, only what was in place when the
-// sequence began (matrices, damping, factors, indices) is read.  At least one
+// sequence began (matrices, damping, factors, indices) is read.  __ldg and
+// `const T* __restrict__` (which lets the compiler use it) are for those alone:
+// the read-only path is defined for data nobody writes while the kernel lives,
+// and a kernel started early lives while its predecessor still writes vectors
+// and scalars.  They are read by plain loads from unrestricted pointers, which
+// neither the compiler nor the caches serve from before the wait.  At least one
 // thread of every launch passes pdl_wait, so a launch never ends before its
 // predecessor and waiting for one kernel is waiting for all before it.
 __device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -41,14 +41,6 @@ __device__ __forceinline__ void cp_async8(double* dst, const double* src) {
                : "memory");
 }
 
-// an input vector's element: in global memory and read-only, or (OWN) in
-// shared memory
-template <bool OWN, typename T>
-__device__ __forceinline__ T load_in(const T* p) {
-  if constexpr (OWN) return *p;
-  else return __ldg(p);
-}
-
 template <int D, int P>
 __device__ __forceinline__ long long slot_off(int s, long long M) {
   constexpr int W = 2 * P + 1;
@@ -271,7 +263,7 @@ __device__ __forceinline__ Reduce batch_reduce(Reduce R, unsigned bq) {
 // a pass of its own (257^3: 42 us, less than the fused form lost).
 template <int D>
 __device__ __forceinline__ double q1_row_sum(const double* __restrict__ A, long long Np, int N, int M,
-                                             const double* __restrict__ x, int i, double& dg) {
+                                             const double* x, int i, double& dg) {
   constexpr int NS = St<D, 1>::NS, C = St<D, 1>::CENTER;
   double av[NS], xv[NS];
   const double* a = A + i;
@@ -281,7 +273,7 @@ __device__ __forceinline__ double q1_row_sum(const double* __restrict__ A, long 
 #pragma unroll
   for (int s = 0; s < NS; ++s) {
     const int o = (s % 3 - 1) + (D > 1 ? M * ((s / 3) % 3 - 1) : 0) + (D > 2 ? M * M * (s / 9 - 1) : 0);
-    xv[s] = __ldg(x + min(max(i + o, 0), N - 1));
+    xv[s] = x[min(max(i + o, 0), N - 1)];
   }
   dg = av[C];
   double sum = 0.0;
@@ -294,7 +286,7 @@ __device__ __forceinline__ double q1_row_sum(const double* __restrict__ A, long 
 // level, one row per thread
 template <int D, bool RES>
 __global__ void __launch_bounds__(kRowT, kRowMinBlocks)
-k_row_q1(const double* __restrict__ A, int N, long long Np, int M, const double* __restrict__ x, const double* b,
+k_row_q1(const double* __restrict__ A, int N, long long Np, int M, const double* x, const double* b,
          double* y) {
   pdl_next();
   const int i = blockIdx.x * kRowT + threadIdx.x;
@@ -313,7 +305,7 @@ k_row_q1(const double* __restrict__ A, int N, long long Np, int M, const double*
 template <int D>
 __global__ void __launch_bounds__(kRowT, kRowMinBlocks)
 k_row_jacobi_q1(const double* __restrict__ A, int N, long long Np, int M, double damp,
-                const double* __restrict__ omega, const double* __restrict__ x, const double* b,
+                const double* __restrict__ omega, const double* x, const double* b,
                 double* __restrict__ xout, double* r, int write_r) {
   pdl_next();
   const int i = blockIdx.x * kRowT + threadIdx.x;
@@ -326,7 +318,7 @@ k_row_jacobi_q1(const double* __restrict__ A, int N, long long Np, int M, double
   const double s = q1_row_sum<D>(A, Np, N, M, x, i, dg);
   const double t = (b[bq * Np + i] - s) / dg;
   if (write_r) r[bq * Np + i] = t;
-  xout[bq * Np + i] = fma(w, t, __ldg(x + i));
+  xout[bq * Np + i] = fma(w, t, x[i]);
 }
 
 // k_jacobi on a scalar Q2 level (the diagonal sits at the node's colour-major place)
@@ -463,9 +455,8 @@ __device__ __forceinline__ long long q2_place(const Q2Layout& lay, int M, int co
 
 // sum over the row's stored slots, in slot order, of A(i, s) x(i + off_s).
 // PAT: the row's parity pattern.  Neighbour coordinates are clamped into the
-// grid per direction (a slot reaching outside holds a zero).  XL: how x is
-// read -- 0 plain loads (x is written by the kernel), 1 the read-only path
-template <int D, int PAT, int XL>
+// grid per direction (a slot reaching outside holds a zero).
+template <int D, int PAT>
 __device__ __forceinline__ double q2_row_sum(const double* __restrict__ A, long long Np, const double* x, int M,
                                              const int c[3], const int (&p)[1 << D]) {
   int cl[3][5];
@@ -496,7 +487,7 @@ __device__ __forceinline__ double q2_row_sum(const double* __restrict__ A, long 
           const int slot = sx + 5 * (sy + 5 * sz);
           const int r = (rx ? 1 : 0) | (ry ? 2 : 0) | (rz ? 4 : 0);
           av[q] = __ldg(A + (long long)slot * Np + p[r]);
-          xv[q] = XL == 1 ? __ldg(xl + cl[0][sx]) : xl[cl[0][sx]];
+          xv[q] = xl[cl[0][sx]];
           ++q;
         }
       }
@@ -692,7 +683,7 @@ static void launch_q2_tile(const LevelView& L, int col, double damp, double* x, 
 
 // the rows of block blk of colour class `colour` in the multicolour <sor>
 // sweep of a scalar Q2 level (linit.lisp:288-323): r = (b - A x)/d, x += w r
-template <int D, int XL>
+template <int D>
 __device__ __forceinline__ void sor_q2_block(const double* __restrict__ A, long long Np, int M, int colour,
                                              long long blk, double omega_s, const double* __restrict__ omega,
                                              double* x, const double* b, double* r, const Q2Layout& lay) {
@@ -707,7 +698,7 @@ __device__ __forceinline__ void sor_q2_block(const double* __restrict__ A, long 
   const double d = __ldg(A + (long long)C * Np + p[0]);
   const double bi = b[i], xi = x[i], wi = omega ? __ldg(omega + i) : omega_s;
   double s = 0.0;
-  q2_pat_dispatch<D>(pat, [&](auto P) { s = q2_row_sum<D, decltype(P)::value, XL>(A, Np, x, M, c, p); });
+  q2_pat_dispatch<D>(pat, [&](auto P) { s = q2_row_sum<D, decltype(P)::value>(A, Np, x, M, c, p); });
   const double tt = (bi - s) / d;
   r[i] = tt;
   x[i] = fma(wi, tt, xi);
@@ -721,13 +712,13 @@ k_sor_q2(const double* __restrict__ A, long long Np, int M, int colour, double o
          const __grid_constant__ Q2Layout lay) {
   pdl_next();
   pdl_wait();
-  sor_q2_block<D, 0>(A, Np, M, colour, blockIdx.x, omega_s, omega, x, b, r, lay);
+  sor_q2_block<D>(A, Np, M, colour, blockIdx.x, omega_s, omega, x, b, r, lay);
 }
 
 // y = A x or r = b - A x on a scalar Q2 level, rows by class (blockIdx.y) and parity
 template <int D, bool RES>
 __global__ void __launch_bounds__(kQ2T, kQ2MinBlocks<D>)
-k_spmv_q2c(const double* __restrict__ A, long long Np, int M, const double* __restrict__ x, const double* b,
+k_spmv_q2c(const double* __restrict__ A, long long Np, int M, const double* x, const double* b,
            double* y, const __grid_constant__ Q2Layout lay) {
   pdl_next();
   pdl_wait();
@@ -739,15 +730,15 @@ k_spmv_q2c(const double* __restrict__ A, long long Np, int M, const double* __re
   int c[3], p[1 << D];
   const long long i = q2_place<D>(lay, M, colour, sub, u, c, p);
   double s = 0.0;
-  q2_pat_dispatch<D>(pat, [&](auto P) { s = q2_row_sum<D, decltype(P)::value, 1>(A, Np, x, M, c, p); });
+  q2_pat_dispatch<D>(pat, [&](auto P) { s = q2_row_sum<D, decltype(P)::value>(A, Np, x, M, c, p); });
   y[i] = RES ? b[i] - s : s;
 }
 
-// k_jacobi_res on a scalar Q2 level, rows by class and parity
+// k_row_jacobi_q1 on a scalar Q2 level, rows by class and parity
 template <int D>
 __global__ void __launch_bounds__(kQ2T, kQ2MinBlocks<D>)
 k_jacobi_res_q2c(const double* __restrict__ A, long long Np, int M, double damp, const double* __restrict__ omega,
-                 const double* __restrict__ x, const double* b, double* __restrict__ xout, double* r, int write_r,
+                 const double* x, const double* b, double* __restrict__ xout, double* r, int write_r,
                  const __grid_constant__ Q2Layout lay) {
   pdl_next();
   pdl_wait();
@@ -761,7 +752,7 @@ k_jacobi_res_q2c(const double* __restrict__ A, long long Np, int M, double damp,
   constexpr int C = St<D, 2>::CENTER;
   const double d = __ldg(A + (long long)C * Np + p[0]);
   double s = 0.0;
-  q2_pat_dispatch<D>(pat, [&](auto P) { s = q2_row_sum<D, decltype(P)::value, 1>(A, Np, x, M, c, p); });
+  q2_pat_dispatch<D>(pat, [&](auto P) { s = q2_row_sum<D, decltype(P)::value>(A, Np, x, M, c, p); });
   const double t = (b[i] - s) / d;
   if (write_r) r[i] = t;
   xout[i] = fma(omega ? omega[i] : damp, t, x[i]);
@@ -1048,7 +1039,7 @@ k_ssc_res_q2(const double* __restrict__ A, long long Np, int M, int ssc, int dma
   const long long i = q2_place<D>(lay, M, colour, sub, u, c, p);
   const double bi = b[i];
   double s = 0.0;
-  q2_pat_dispatch<D>(pat, [&](auto P) { s = q2_row_sum<D, decltype(P)::value, 0>(A, Np, x, M, c, p); });
+  q2_pat_dispatch<D>(pat, [&](auto P) { s = q2_row_sum<D, decltype(P)::value>(A, Np, x, M, c, p); });
   if (pat == 0 || !q2_face(c, M, dmask)) r[i] = bi - s;
 }
 
@@ -1105,7 +1096,7 @@ k_psc_q1(const double* __restrict__ A, long long N, long long Np, double damp, d
 // correction goes to C[block][t] (zero for padded members).
 template <int D>
 __global__ void __launch_bounds__(128, 6)
-k_psc_block_q2(long long M, int dmask, const double* __restrict__ r, const double* __restrict__ F,
+k_psc_block_q2(long long M, int dmask, const double* r, const double* __restrict__ F,
                const unsigned char* __restrict__ P, double* __restrict__ C) {
   pdl_next();
   pdl_wait();
@@ -1135,7 +1126,7 @@ k_psc_block_q2(long long M, int dmask, const double* __restrict__ r, const doubl
 // of it along every direction; a Dirichlet node belongs to its own block only)
 template <int D>
 __global__ void __launch_bounds__(kBlock)
-k_psc_gather_q2(long long N, long long M, int dmask, double damp, const double* __restrict__ C, double* x) {
+k_psc_gather_q2(long long N, long long M, int dmask, double damp, const double* C, double* x) {
   pdl_next();
   pdl_wait();
   constexpr int NB = D == 1 ? 3 : (D == 2 ? 9 : 27);
@@ -1188,10 +1179,7 @@ k_psc_gather_q2(long long N, long long M, int dmask, double damp, const double* 
 // The row sums fetch eight entries at a time -- indices and values, then the
 // unknowns -- so a row of up to eight entries waits for memory twice (entry by
 // entry it was twice per few entries), and the first eight are fetched while
-// the previous launch still runs.  ROX: x by the read-only path (a sweep that
-// updates x in place reads it plainly).  Every caller's thread passes pdl_wait
-// here.
-template <bool ROX>
+// the previous launch still runs.  Every caller's thread passes pdl_wait here.
 __device__ __forceinline__ double csr_row_sum(const CsrView& a, long long i, const double* x) {
   constexpr int K = 8;
   const long long e1 = a.start[i + 1];
@@ -1213,7 +1201,7 @@ __device__ __forceinline__ double csr_row_sum(const CsrView& a, long long i, con
     double xv[K];
 #pragma unroll
     for (int q = 0; q < K; ++q)
-      if (e + q < e1) xv[q] = ROX ? __ldg(x + ix[q]) : x[ix[q]];
+      if (e + q < e1) xv[q] = x[ix[q]];
 #pragma unroll
     for (int q = 0; q < K; ++q)
       if (e + q < e1) s = fma(v[q], xv[q], s);
@@ -1226,24 +1214,24 @@ constexpr int kCsrT = 64;  // threads per block of the compressed-row kernels: s
 
 // y = A x, or r = b - A x (b may alias r)
 __global__ void __launch_bounds__(kCsrT, 8)
-k_csr_spmv(long long N, CsrView a, const double* __restrict__ x, const double* b, double* y, int res) {
+k_csr_spmv(long long N, CsrView a, const double* x, const double* b, double* y, int res) {
   pdl_next();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  const double s = csr_row_sum<true>(a, i, x);
+  const double s = csr_row_sum(a, i, x);
   y[i] = res ? b[i] - s : s;
 }
 
 // compute-residual fused with the following <jacobi> step (as k_row_jacobi_q1)
 __global__ void __launch_bounds__(kCsrT, 8)
 k_csr_jacobi_res(long long N, CsrView a, const double* __restrict__ diag, double damp,
-                 const double* __restrict__ omega, const double* __restrict__ x, const double* b,
+                 const double* __restrict__ omega, const double* x, const double* b,
                  double* __restrict__ xout, double* r, int write_r) {
   pdl_next();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   const double d = __ldg(diag + i), w = omega ? __ldg(omega + i) : damp;
-  const double s = csr_row_sum<true>(a, i, x);
+  const double s = csr_row_sum(a, i, x);
   const double t = (b[i] - s) / d;
   if (write_r) r[i] = t;
   xout[i] = fma(w, t, x[i]);
@@ -1262,7 +1250,7 @@ k_csr_sor(const int* __restrict__ rows, long long cnt, CsrView a, const double* 
   if (t >= cnt) return;
   const long long i = __ldg(rows + t);
   const double d = __ldg(diag + i), w = omega ? __ldg(omega + i) : omega_s;
-  const double s = csr_row_sum<false>(a, i, x);
+  const double s = csr_row_sum(a, i, x);
   const double rr = b[i] - s;
   const double tt = rr / d;
   r[i] = ssc ? rr : tt;
@@ -1272,11 +1260,11 @@ k_csr_sor(const int* __restrict__ rows, long long cnt, CsrView a, const double* 
 // rc = I^T rf row by row of I^T (fine entries ascending); the coarse rhs
 // takes rc, the coarse solution 0 (the :after methods of restrict)
 __global__ void __launch_bounds__(kCsrT, 8)
-k_csr_restrict(long long NC, CsrView pt, const double* __restrict__ rf, double* rc, double* rhsc, double* solc) {
+k_csr_restrict(long long NC, CsrView pt, const double* rf, double* rc, double* rhsc, double* solc) {
   pdl_next();
   const long long J = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (J >= NC) return;
-  const double s = csr_row_sum<true>(pt, J, rf);
+  const double s = csr_row_sum(pt, J, rf);
   rc[J] = s;
   if (rhsc) rhsc[J] = s;
   if (solc) solc[J] = 0.0;
@@ -1284,14 +1272,14 @@ k_csr_restrict(long long NC, CsrView pt, const double* __restrict__ rf, double* 
 
 // xf += I xc (coarse entries ascending)
 __global__ void __launch_bounds__(kCsrT, 8)
-k_csr_prolong(long long NF, CsrView p, const double* __restrict__ xc, double* xf) {
+k_csr_prolong(long long NF, CsrView p, const double* xc, double* xf) {
   pdl_next();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= NF || p.start[i] == p.start[i + 1]) {  // constrained rows keep their value
     pdl_wait();  // (were all rows empty, the launch would otherwise end before its predecessor)
     return;
   }
-  const double s = csr_row_sum<true>(p, i, xc);
+  const double s = csr_row_sum(p, i, xc);
   xf[i] = xf[i] + s;
 }
 
@@ -1339,9 +1327,10 @@ __device__ __forceinline__ bool face_dir(int c, int M, int k, int dmask) {
 // outside the level and Dirichlet nodes are skipped.  (3D Q1, 129^3 coarse
 // nodes: 64 us, 138 us with each load waiting for the previous term; one
 // memory wait per plane on small levels, 12.4 -> 6 us at 33^3.)
-// NC: components per node; rf points at the component summed; CG: see load_in.
-template <int D, int P, int NC = 1, typename T = double, bool OWN = false>
-__device__ __forceinline__ T restrict_node(const int cJ[3], int MC, int MF, int dmask, const T* __restrict__ rf) {
+// NC: components per node; rf points at the component summed (global or, in
+// k_tail, shared memory).
+template <int D, int P, int NC = 1, typename T = double>
+__device__ __forceinline__ T restrict_node(const int cJ[3], int MC, int MF, int dmask, const T* rf) {
 #pragma unroll
   for (int k = 0; k < D; ++k)
     if (face_dir(cJ[k], MC, k, dmask)) return T(0);
@@ -1372,8 +1361,8 @@ __device__ __forceinline__ T restrict_node(const int cJ[3], int MC, int MF, int 
 #pragma unroll
       for (int q = 0; q < R; ++q)
         if (on[0][q] && (D < 2 || on[1][y]) && (D < 3 || on[2][z]))
-          v[y * R + q] = load_in<OWN>(rf + NC * (f[0][q] + (long long)MF * ((D > 1 ? f[1][y] : 0) +
-                                                                     (long long)MF * (D > 2 ? f[2][z] : 0))));
+          v[y * R + q] = rf[NC * (f[0][q] + (long long)MF * ((D > 1 ? f[1][y] : 0) +
+                                                             (long long)MF * (D > 2 ? f[2][z] : 0)))];
 #pragma unroll
     for (int y = 0; y < (D > 1 ? R : 1); ++y)
 #pragma unroll
@@ -1390,8 +1379,8 @@ __device__ __forceinline__ T restrict_node(const int cJ[3], int MC, int MF, int 
 
 // (I xc) at fine node fi, not a Dirichlet node (constrained); all loads first
 // (3D Q1, 257^3 fine nodes: 197 us, 469 us with a load per term)
-template <int D, int P, int NC = 1, typename T = double, bool OWN = false>
-__device__ __forceinline__ T prolong_node(const int fi[3], int MF, int MC, int dmask, const T* __restrict__ xc) {
+template <int D, int P, int NC = 1, typename T = double>
+__device__ __forceinline__ T prolong_node(const int fi[3], int MF, int MC, int dmask, const T* xc) {
   constexpr int R = P == 1 ? 2 : 3;
   int j[3][R];
   double w[3][R];
@@ -1418,8 +1407,8 @@ __device__ __forceinline__ T prolong_node(const int fi[3], int MF, int MC, int d
 #pragma unroll
       for (int q = 0; q < R; ++q)
         if (on[0][q] && (D < 2 || on[1][y]) && (D < 3 || on[2][z]))
-          v[(z * NY + y) * R + q] = load_in<OWN>(xc + NC * (j[0][q] + (long long)MC * ((D > 1 ? j[1][y] : 0) +
-                                                                                (long long)MC * (D > 2 ? j[2][z] : 0))));
+          v[(z * NY + y) * R + q] = xc[NC * (j[0][q] + (long long)MC * ((D > 1 ? j[1][y] : 0) +
+                                                                        (long long)MC * (D > 2 ? j[2][z] : 0)))];
   T acc = T(0);
 #pragma unroll
   for (int z = 0; z < NZ; ++z)
@@ -1440,7 +1429,7 @@ __device__ __forceinline__ T prolong_node(const int fi[3], int MF, int MC, int d
 // methods for the correction scheme, multigrid.lisp:202-224)
 template <int D, int P>
 __global__ void __launch_bounds__(kBlock)
-k_restrict(int MC, int MF, int dmask, const double* __restrict__ rf, double* __restrict__ rc,
+k_restrict(int MC, int MF, int dmask, const double* rf, double* __restrict__ rc,
            double* __restrict__ rhsc, double* __restrict__ solc, long long fs, long long cs) {
   pdl_next();
   pdl_wait();
@@ -1469,7 +1458,7 @@ k_restrict(int MC, int MF, int dmask, const double* __restrict__ rf, double* __r
 // (257^3 fine nodes: 99 us, 197 us with a thread per fine node).
 template <int D>
 __global__ void __launch_bounds__(kBlock)
-k_prolong_q1f(int MF, int MC, int dmask, const double* __restrict__ xc, double* __restrict__ xf, long long fs,
+k_prolong_q1f(int MF, int MC, int dmask, const double* xc, double* __restrict__ xf, long long fs,
               long long cs) {
   pdl_next();
   pdl_wait();
@@ -1496,8 +1485,8 @@ k_prolong_q1f(int MF, int MC, int dmask, const double* __restrict__ xc, double* 
       const int cy = (fy >> 1) + y, cz = (fz >> 1) + z;
       on[z][y] = y < ny && z < nz && (D < 2 || !face_dir(cy, MC, 1, dmask)) && (D < 3 || !face_dir(cz, MC, 2, dmask));
       const double* c = xc + j + (long long)MC * (cy + (long long)MC * cz);
-      v[z][y][0] = on[z][y] && x0 ? __ldg(c) : 0.0;
-      v[z][y][1] = on[z][y] && x1 ? __ldg(c + 1) : 0.0;
+      v[z][y][0] = on[z][y] && x0 ? c[0] : 0.0;
+      v[z][y][1] = on[z][y] && x1 ? c[1] : 0.0;
     }
   double* f = xf + 2 * j + (long long)MF * (fy + (long long)MF * fz);
   const bool w0 = !face_dir(2 * j, MF, 0, dmask), w1 = j + 1 < MC;  // an odd node lies on no face
@@ -1522,7 +1511,7 @@ k_prolong_q1f(int MF, int MC, int dmask, const double* __restrict__ xc, double* 
 // xf := xf + I xc (constrained) (prolongate, multigrid.lisp:237-239)
 template <int D, int P>
 __global__ void __launch_bounds__(kBlock)
-k_prolong(int MF, int MC, int dmask, const double* __restrict__ xc, double* __restrict__ xf, long long fs,
+k_prolong(int MF, int MC, int dmask, const double* xc, double* __restrict__ xf, long long fs,
           long long cs) {
   pdl_next();
   pdl_wait();
@@ -1873,7 +1862,7 @@ __global__ void k_fill(double* x, long long n, double v) {
   if (i < n) x[i] = v;
 }
 
-__global__ void k_copy(const double* __restrict__ x, double* __restrict__ y, long long n) {
+__global__ void k_copy(const double* x, double* __restrict__ y, long long n) {
   pdl_next();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1881,7 +1870,7 @@ __global__ void k_copy(const double* __restrict__ x, double* __restrict__ y, lon
 }
 
 // axpy!: y := y + alpha x (alpha from a device slot when aslot >= 0)
-__global__ void k_axpy(double alpha, const double* __restrict__ sc, int aslot, const double* __restrict__ x,
+__global__ void k_axpy(double alpha, const double* sc, int aslot, const double* x,
                        double* y, long long n) {
   pdl_next();
   pdl_wait();
@@ -1893,7 +1882,7 @@ __global__ void k_axpy(double alpha, const double* __restrict__ sc, int aslot, c
 
 // DR4096 dot product (x, y)
 __global__ void __launch_bounds__(kBlock, 4)
-k_dot(const double* __restrict__ x, const double* __restrict__ y, long long n, Reduce R, long long vs) {
+k_dot(const double* x, const double* y, long long n, Reduce R, long long vs) {
   pdl_next();
   pdl_wait();
   __shared__ double smem[8];
@@ -1914,16 +1903,16 @@ k_dot(const double* __restrict__ x, const double* __restrict__ y, long long n, R
     for (int m = 0; m < 4; ++m) {
       const long long i0 = base + 512LL * (m0 + m);
       if (wide && i0 + 1 < n) {
-        u[m] = __ldg(reinterpret_cast<const double2*>(x + i0));
-        v[m] = __ldg(reinterpret_cast<const double2*>(y + i0));
+        u[m] = *reinterpret_cast<const double2*>(x + i0);
+        v[m] = *reinterpret_cast<const double2*>(y + i0);
       } else {
         if (i0 < n) {
-          u[m].x = __ldg(x + i0);
-          v[m].x = __ldg(y + i0);
+          u[m].x = x[i0];
+          v[m].x = y[i0];
         }
         if (i0 + 1 < n) {
-          u[m].y = __ldg(x + i0 + 1);
-          v[m].y = __ldg(y + i0 + 1);
+          u[m].y = x[i0 + 1];
+          v[m].y = y[i0 + 1];
         }
       }
     }
@@ -1940,10 +1929,9 @@ k_dot(const double* __restrict__ x, const double* __restrict__ y, long long n, R
 // CG update (krylow.lisp:117-121): x += lam p; r -= lam a; fused (r,r);
 // then w := r and (optionally) w2 := r, q := 0 for the preconditioner call
 __global__ void __launch_bounds__(kBlock, 3)
-k_cg_update(const double* __restrict__ sc, double* __restrict__ x, const double* __restrict__ p,
-            double* __restrict__ r, const double* __restrict__ a, double* __restrict__ w,
-            double* __restrict__ w2, double* __restrict__ q, long long n, Reduce R, long long vs,
-            const double* __restrict__ frozen) {
+k_cg_update(const double* sc, double* __restrict__ x, const double* p, double* __restrict__ r, const double* a,
+            double* __restrict__ w, double* __restrict__ w2, double* __restrict__ q, long long n, Reduce R, long long vs,
+            const double* frozen) {
   pdl_next();
   pdl_wait();
   __shared__ double smem[8];
@@ -1996,8 +1984,8 @@ k_cg_update(const double* __restrict__ sc, double* __restrict__ x, const double*
 }
 
 // p := (new_alpha/alpha) p (scal!), then p := p + q (m+!)
-__global__ void k_p_update(const double* __restrict__ sc, double* __restrict__ p, const double* __restrict__ q,
-                           long long n, long long vs, const double* __restrict__ frozen) {
+__global__ void k_p_update(const double* sc, double* __restrict__ p, const double* q, long long n, long long vs,
+                           const double* frozen) {
   pdl_next();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -2301,7 +2289,7 @@ constexpr int kRow3Nodes = 64, kRow3T = 3 * kRow3Nodes;
 template <int P, typename T, int OP>
 __global__ void __launch_bounds__(kRow3T, sizeof(T) == 8 ? 3 : 4)
 k_row3(const T* __restrict__ A, int N, long long Np, int M, double damp, const double* __restrict__ omega,
-       const T* __restrict__ x, const T* b, T* y, T* r, int write_r) {
+       const T* x, const T* b, T* y, T* r, int write_r) {
   pdl_next();
   constexpr int W = 2 * P + 1, Q = W * W, SEG = 3 * (kRow3Nodes + 2 * P);
   extern __shared__ unsigned char row3_sm[];
@@ -2348,7 +2336,7 @@ k_row3(const T* __restrict__ A, int N, long long Np, int M, double damp, const d
     for (int t = 0; t < BATCH; ++t) {
       const int f = (f0 + t) * kRow3T + threadIdx.x, q = f / SEG, e = f - q * SEG;
       const long long g = 3LL * (i0 + (q % W - P) * M + (q / W - P) * M * M - P) + e;
-      v[t] = f < Q * SEG && g >= 0 && g < 3LL * N ? __ldg(x + g) : T(0);
+      v[t] = f < Q * SEG && g >= 0 && g < 3LL * N ? x[g] : T(0);
     }
 #pragma unroll
     for (int t = 0; t < BATCH; ++t) {
@@ -2418,7 +2406,7 @@ k_row3(const T* __restrict__ A, int N, long long Np, int M, double damp, const d
 template <int P, typename T, int OP>
 __global__ void __launch_bounds__(kRow3Nodes, 8)
 k_node3(const T* __restrict__ A, int N, long long Np, int M, double damp, const double* __restrict__ omega,
-        const T* __restrict__ x, const T* b, T* y, T* r, int write_r) {
+        const T* x, const T* b, T* y, T* r, int write_r) {
   pdl_next();
   pdl_wait();
   constexpr int W = 2 * P + 1, Q = W * W, SEG = 3 * (kRow3Nodes + 2 * P);
@@ -2438,7 +2426,7 @@ k_node3(const T* __restrict__ A, int N, long long Np, int M, double damp, const 
     for (int t = 0; t < BATCH; ++t) {
       const int f = (f0 + t) * kRow3Nodes + threadIdx.x, q = f / SEG, e = f - q * SEG;
       const long long g = 3LL * (i0 + (q % W - P) * M + (q / W - P) * M * M - P) + e;
-      v[t] = f < Q * SEG && g >= 0 && g < 3LL * N ? __ldg(x + g) : T(0);
+      v[t] = f < Q * SEG && g >= 0 && g < 3LL * N ? x[g] : T(0);
     }
 #pragma unroll
     for (int t = 0; t < BATCH; ++t) {
@@ -2562,7 +2550,7 @@ k_jacobi3(const double* __restrict__ A, long long N, long long Np, int center, d
 constexpr long long kXferLoopMin = 30000;
 
 template <int P, typename T>
-__device__ __forceinline__ void restrict3_loop(const int cJ[3], int MC, int MF, int dmask, const T* __restrict__ rf,
+__device__ __forceinline__ void restrict3_loop(const int cJ[3], int MC, int MF, int dmask, const T* rf,
                                               T (&acc)[3]) {
 #pragma unroll
   for (int c = 0; c < 3; ++c) acc[c] = T(0);
@@ -2588,7 +2576,7 @@ __device__ __forceinline__ void restrict3_loop(const int cJ[3], int MC, int MF, 
 }
 
 template <int P, typename T>
-__device__ __forceinline__ void prolong3_loop(const int fi[3], int MC, int dmask, const T* __restrict__ xc,
+__device__ __forceinline__ void prolong3_loop(const int fi[3], int MC, int dmask, const T* xc,
                                              T (&acc)[3]) {
 #pragma unroll
   for (int c = 0; c < 3; ++c) acc[c] = T(0);
@@ -2616,7 +2604,7 @@ __device__ __forceinline__ void prolong3_loop(const int fi[3], int MC, int dmask
 // per scalar unknown (x: node and component)
 template <int P, bool LOOP, typename T = double>
 __global__ void __launch_bounds__(kBlock)
-k_restrict3(int MC, int MF, int dmask, const T* __restrict__ rf, T* __restrict__ rc,
+k_restrict3(int MC, int MF, int dmask, const T* rf, T* __restrict__ rc,
             T* __restrict__ rhsc, T* __restrict__ solc) {
   pdl_next();
   pdl_wait();
@@ -2639,7 +2627,7 @@ k_restrict3(int MC, int MF, int dmask, const T* __restrict__ rf, T* __restrict__
 // xf := xf + I xc per component (constrained)
 template <int P, bool LOOP, typename T = double>
 __global__ void __launch_bounds__(kBlock)
-k_prolong3(int MF, int MC, int dmask, const T* __restrict__ xc, T* __restrict__ xf) {
+k_prolong3(int MF, int MC, int dmask, const T* xc, T* __restrict__ xf) {
   pdl_next();
   pdl_wait();
   constexpr int CT = LOOP ? 3 : 1;
@@ -2957,7 +2945,7 @@ k_galerkin(const double* __restrict__ AF, long long NpF, int MF, double* __restr
 // (B_i the 3 x 3 diagonal block, symmetric, so the same solve serves the adjoint)
 __global__ void __launch_bounds__(kBlock)
 k_bdiag3(const double* __restrict__ A, long long N, long long Np, int center, int mode,
-         const double* __restrict__ w, const double* __restrict__ x, double* __restrict__ y) {
+         const double* w, const double* x, double* __restrict__ y) {
   pdl_next();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -2976,7 +2964,7 @@ k_bdiag3(const double* __restrict__ A, long long N, long long Np, int center, in
 }
 
 // y = x + w .* v with w per node (y may be x)
-__global__ void k_xpwv3(const double* x, const double* __restrict__ w, const double* __restrict__ v, double* y,
+__global__ void k_xpwv3(const double* x, const double* w, const double* v, double* y,
                         long long N) {
   pdl_next();
   pdl_wait();
@@ -2987,7 +2975,7 @@ __global__ void k_xpwv3(const double* x, const double* __restrict__ w, const dou
 }
 
 // acc_i += sum_k a_ik b_ik (per-node dot of two vectors)
-__global__ void k_acc_prod3(double* __restrict__ acc, const double* __restrict__ a, const double* __restrict__ b,
+__global__ void k_acc_prod3(double* __restrict__ acc, const double* a, const double* b,
                             long long N) {
   pdl_next();
   pdl_wait();
@@ -3004,7 +2992,7 @@ __global__ void k_acc_prod3(double* __restrict__ acc, const double* __restrict__
 template <typename T>
 __global__ void __launch_bounds__(kBlock)
 k_jacobi0_3(const T* __restrict__ A, long long N, long long Np, int center, float damp,
-            const double* __restrict__ omega, const T* __restrict__ b, T* __restrict__ x) {
+            const double* __restrict__ omega, const T* b, T* __restrict__ x) {
   pdl_next();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -3021,7 +3009,7 @@ k_jacobi0_3(const T* __restrict__ A, long long N, long long Np, int center, floa
 
 // y = f x with f from a grid scalar: mode 0: 1, mode 1: 1/sqrt(sc[slot]), mode 2: sqrt(sc[slot])
 template <typename TI, typename TO>
-__global__ void k_vscale(const TI* __restrict__ x, const double* __restrict__ sc, int slot, int mode,
+__global__ void k_vscale(const TI* x, const double* sc, int slot, int mode,
                          TO* __restrict__ y, long long n) {
   pdl_next();
   pdl_wait();
@@ -3220,7 +3208,7 @@ k_tail(const __grid_constant__ TailArgs<CAP> g) {
           } else {
             const int q = j / C.M;
             const int c[3] = {j - q * C.M, D > 1 ? q % C.M : 0, D > 2 ? q / C.M : 0};
-            acc = restrict_node<D, 1, 1, double, true>(c, C.M, L.M, dmask, x);
+            acc = restrict_node<D, 1>(c, C.M, L.M, dmask, x);
           }
           r[j] = acc;
           b[j] = acc;
@@ -3241,7 +3229,7 @@ k_tail(const __grid_constant__ TailArgs<CAP> g) {
 #pragma unroll
             for (int k = 0; k < D; ++k) dir = dir || face_dir(c[k], L.M, k, dmask);
             if (dir) continue;
-            y[i] = y[i] + prolong_node<D, 1, 1, double, true>(c, L.M, C.M, dmask, x);
+            y[i] = y[i] + prolong_node<D, 1>(c, L.M, C.M, dmask, x);
           }
         }
         break;

@@ -216,9 +216,9 @@ __device__ __forceinline__ void face_node(long long f, const MftGeo& q, int M, i
 }
 
 template <typename T, typename TV, typename TX, int MODE, bool RED>
-__device__ __forceinline__ void mf_face_cta(const MFArgsT<T>& g, const MftGeo& geo, int fb, const TX* __restrict__ x,
-                                            const T* __restrict__ b, T* __restrict__ y, const TV* __restrict__ v,
-                                            const TV* __restrict__ v2, double& acc0, double& acc1) {
+__device__ __forceinline__ void mf_face_cta(const MFArgsT<T>& g, const MftGeo& geo, int fb, const TX* x,
+                                            const T* b, T* __restrict__ y, const TV* v, const TV* v2, double& acc0,
+                                            double& acc1) {
   constexpr bool HX = MODE != 3;
   constexpr bool HB = MODE != 0;
   constexpr bool DIFF = sizeof(T) == 8;
@@ -261,8 +261,8 @@ __device__ __forceinline__ void mf_face_cta(const MFArgsT<T>& g, const MftGeo& g
       };
       mf_row<T, HX, DIFF>(k, X, g.hs, ax, d, xc);
     }
-    const T bb = HB ? __ldg(b + io) : T(0);
-    const T o = (HO && uwd) ? __ldg(g.wd + io) : ((HO && g.omega) ? __ldg(g.omega + in) : g.w);
+    const T bb = HB ? b[io] : T(0);
+    const T o = (HO && uwd) ? g.wd[io] : ((HO && g.omega) ? __ldg(g.omega + in) : g.w);
     const T out = mf_out<MODE>(ax, d, xc, bb, o, uwd);
     y[g.yl.at(ix, iy, iz)] = out;
     if (RED) {
@@ -346,8 +346,7 @@ __global__ void __launch_bounds__(kFThreads, (sizeof(T) == 4 && MODE != 2) ? 3 :
 k_mfc(MFArgsT<T> g, const __grid_constant__ CUtensorMap tk_cells, const __grid_constant__ CUtensorMap tm_x,
       const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_o,
       const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_v2, MftGeo geo,
-      const TX* __restrict__ x, const T* __restrict__ b, T* __restrict__ y, const TV* __restrict__ v,
-      const TV* __restrict__ v2, Reduce2 R) {
+      const TX* x, const T* b, T* __restrict__ y, const TV* v, const TV* v2, Reduce2 R) {
   typedef MfcLayout<T, TV, TX, MODE, RED> L;
   typedef CellBox<T> LC;
   constexpr bool DIFF = sizeof(T) == 8;  // the FP64 operator in difference form
@@ -595,8 +594,7 @@ __device__ __forceinline__ long long soff(int s, long long M) {
 template <int D, int P, int MODE, typename TB, typename TY, bool RED, int RPT>
 __global__ void __launch_bounds__(kBlock, RPT == 1 && P == 1 ? 3 : P == 1 ? 2 : 0)
 k_st32(const float* __restrict__ A, long long N, long long Np, long long M, float w, const float* __restrict__ om,
-       const float* __restrict__ x, const TB* __restrict__ b, TY* __restrict__ y, const double* __restrict__ v,
-       const double* __restrict__ v2, Reduce2 R) {
+       const float* x, const TB* b, TY* __restrict__ y, const double* v, const double* v2, Reduce2 R) {
   pdl_next();
   constexpr int NS = St32<D, P>::NS;
   constexpr int C = St32<D, P>::CENTER;
@@ -618,7 +616,7 @@ k_st32(const float* __restrict__ A, long long N, long long Np, long long M, floa
       pdl_wait();
       if (MODE != 3) {
 #pragma unroll
-        for (int k = 0; k < NS; ++k) xv[k] = __ldg(x + clampi(i0 + soff<D, P>(k, M), N));
+        for (int k = 0; k < NS; ++k) xv[k] = x[clampi(i0 + soff<D, P>(k, M), N)];
 #pragma unroll
         for (int k = 0; k < NS; ++k) s[0] = fmaf(a[k], xv[k], s[0]);
         xc[0] = xv[C];
@@ -645,7 +643,7 @@ k_st32(const float* __restrict__ A, long long N, long long Np, long long M, floa
       const long long o = soff<D, P>(k, M);
 #pragma unroll
       for (int r = 0; r < RPT; ++r) {
-        const float xv = __ldg(x + clampi(i0 + r + o, N));
+        const float xv = x[clampi(i0 + r + o, N)];
         s[r] = fmaf(a[r], xv, s[r]);
         if (k == C) xc[r] = xv;
       }
@@ -680,7 +678,7 @@ __device__ __forceinline__ bool fdir(int c, int M, int k, int dmask) {
 // Q1 restriction: three fine nodes per direction with weights 1/2, 1, 1/2,
 // fixed-size loops in registers
 template <int D, typename TR>
-__device__ __forceinline__ void restrict_q1_node(int MC, int MF, int dmask, const TR* __restrict__ rf,
+__device__ __forceinline__ void restrict_q1_node(int MC, int MF, int dmask, const TR* rf,
                                                  __nv_bfloat16* __restrict__ bc, float* __restrict__ xc, int c0,
                                                  int c1, int c2) {
   const int cJ[3] = {c0, c1, c2};
@@ -738,7 +736,7 @@ __device__ __forceinline__ void restrict_q1_node(int MC, int MF, int dmask, cons
 
 template <int D, typename TR>
 __global__ void __launch_bounds__(kBlock)
-k_restrict_q1(int MC, int MF, int dmask, const TR* __restrict__ rf, __nv_bfloat16* __restrict__ bc,
+k_restrict_q1(int MC, int MF, int dmask, const TR* rf, __nv_bfloat16* __restrict__ bc,
               float* __restrict__ xc) {
   pdl_next();
   pdl_wait();
@@ -756,7 +754,7 @@ k_restrict_q1(int MC, int MF, int dmask, const TR* __restrict__ rf, __nv_bfloat1
 // takes k_restrict_q1's per-node form
 template <typename TR>
 __global__ void __launch_bounds__(kBlock)
-k_restrict_q1b(int MC, int MF, int dmask, const TR* __restrict__ rf, __nv_bfloat16* __restrict__ bc,
+k_restrict_q1b(int MC, int MF, int dmask, const TR* rf, __nv_bfloat16* __restrict__ bc,
                float* __restrict__ xc) {
   pdl_next();
   pdl_wait();
@@ -800,7 +798,7 @@ k_restrict_q1b(int MC, int MF, int dmask, const TR* __restrict__ rf, __nv_bfloat
 // solution zeroed; blocks (32, 8) over x, y and one z plane per blockIdx.z
 template <int D, int P, typename TR>
 __global__ void __launch_bounds__(kBlock)
-k_restrict_mx(int MC, int MF, int dmask, const TR* __restrict__ rf, __nv_bfloat16* __restrict__ bc,
+k_restrict_mx(int MC, int MF, int dmask, const TR* rf, __nv_bfloat16* __restrict__ bc,
               float* __restrict__ xc) {
   pdl_next();
   pdl_wait();
@@ -848,7 +846,7 @@ k_restrict_mx(int MC, int MF, int dmask, const TR* __restrict__ rf, __nv_bfloat1
 // second weight zero, so the loops are fixed-size and stay in registers.
 template <int D>
 __global__ void __launch_bounds__(kBlock)
-k_prolong_q1(int MF, int MC, int dmask, const float* __restrict__ xc, float* __restrict__ xf) {
+k_prolong_q1(int MF, int MC, int dmask, const float* xc, float* __restrict__ xf) {
   pdl_next();
   pdl_wait();
   if (D == 1 && threadIdx.y != 0) return;
@@ -879,7 +877,7 @@ k_prolong_q1(int MF, int MC, int dmask, const float* __restrict__ xc, float* __r
     const int bx = c & 1, by = (c >> 1) & 1, bz = c >> 2;
     const float ww = (bx ? w1[0] : w0[0]) * (by ? w1[1] : w0[1]) * (bz ? w1[2] : w0[2]);
     const long long j = (bx ? J1[0] : J0[0]) + (long long)MC * ((by ? J1[1] : J0[1]) + (long long)MC * (bz ? J1[2] : J0[2]));
-    acc = fmaf(ww, __ldg(xc + j), acc);
+    acc = fmaf(ww, xc[j], acc);
   }
   const long long i = fi[0] + (long long)MF * (fi[1] + (long long)MF * fi[2]);
   xf[i] += acc;
@@ -892,7 +890,7 @@ k_prolong_q1(int MF, int MC, int dmask, const float* __restrict__ xc, float* __r
 // all off the faces interpolate one direction at a time; the others sum each
 // fine node with the weights and in the order of k_prolong_q1.
 __global__ void __launch_bounds__(kBlock)
-k_prolong_q1c(int MF, int MC, int dmask, const float* __restrict__ xc, float* __restrict__ xf, VLay fl) {
+k_prolong_q1c(int MF, int MC, int dmask, const float* xc, float* __restrict__ xf, VLay fl) {
   pdl_next();
   pdl_wait();
   const int I = blockIdx.x * 32 + threadIdx.x, J = blockIdx.y * 8 + threadIdx.y, K = blockIdx.z;
@@ -913,7 +911,7 @@ k_prolong_q1c(int MF, int MC, int dmask, const float* __restrict__ xc, float* __
       for (int dy = 0; dy < 2; ++dy) {
         const bool ok = (dz == 0 || hz) && (dy == 0 || hy);
         const float* q = c0 + MC2 * dz + (long long)MC * dy;
-        const float v0 = ok ? __ldg(q) : 0.f, v1 = ok && hx ? __ldg(q + 1) : 0.f;
+        const float v0 = ok ? q[0] : 0.f, v1 = ok && hx ? q[1] : 0.f;
         e[dz][dy][0] = v0;
         e[dz][dy][1] = .5f * (v0 + v1);
       }
@@ -952,7 +950,7 @@ k_prolong_q1c(int MF, int MC, int dmask, const float* __restrict__ xc, float* __
         const int ci = I + dx, cj = J + dy, ck = K + dz;
         const bool ok = ci < MC && cj < MC && ck < MC && !fdir(ci, MC, 0, dmask) && !fdir(cj, MC, 1, dmask) &&
                         !fdir(ck, MC, 2, dmask);
-        v[dz][dy][dx] = ok ? __ldg(xc + ck * MC2 + (long long)cj * MC + ci) : 0.f;
+        v[dz][dy][dx] = ok ? xc[ck * MC2 + (long long)cj * MC + ci] : 0.f;
       }
   // the eight fine values are read before any is written (the compiler
   // cannot tell that the eight layout offsets differ), so their loads overlap
@@ -1004,7 +1002,7 @@ k_prolong_q1c(int MF, int MC, int dmask, const float* __restrict__ xc, float* __
 // columns the four fine x need and interpolated over y, z, then x (coarse
 // Dirichlet values read as zero).
 __global__ void __launch_bounds__(kBlock)
-k_prolong_q1v(int MF, int MC, int dmask, const float* __restrict__ xc, float* __restrict__ xf, VLay fl) {
+k_prolong_q1v(int MF, int MC, int dmask, const float* xc, float* __restrict__ xf, VLay fl) {
   pdl_next();
   pdl_wait();
   const unsigned q = (unsigned)fl.py >> 2;
@@ -1029,7 +1027,7 @@ k_prolong_q1v(int MF, int MC, int dmask, const float* __restrict__ xc, float* __
     for (int dy = 0; dy < 2; ++dy) {
       const float* row = xc + (K + dz) * MC2 + (long long)(J + dy) * MC + c0;
 #pragma unroll
-      for (int t = 0; t < 3; ++t) R[dz][dy][t] = okz[dz] && oky[dy] && okc[t] ? __ldg(row + t) : 0.f;
+      for (int t = 0; t < 3; ++t) R[dz][dy][t] = okz[dz] && oky[dy] && okc[t] ? row[t] : 0.f;
     }
   // over y, then z: R[c][b][t] becomes the value on fine row (2J + b, 2K + c)
 #pragma unroll
@@ -1083,7 +1081,7 @@ k_prolong_q1v(int MF, int MC, int dmask, const float* __restrict__ xc, float* __
 // Q2 (and any order): generic stencil with runtime lengths
 template <int D, int P>
 __global__ void __launch_bounds__(kBlock)
-k_prolong_mx(int MF, int MC, int dmask, const float* __restrict__ xc, float* __restrict__ xf) {
+k_prolong_mx(int MF, int MC, int dmask, const float* xc, float* __restrict__ xf) {
   pdl_next();
   pdl_wait();
   if (D == 1 && threadIdx.y != 0) return;
@@ -1126,7 +1124,7 @@ k_prolong_mx(int MF, int MC, int dmask, const float* __restrict__ xc, float* __r
 // shuffle sum), 128 rows at a time, so the coefficient loads of all rows
 // are in flight together
 __global__ void __launch_bounds__(1024)
-k_coarse_mx(const double* __restrict__ AinvT, int n, const __nv_bfloat16* __restrict__ b, float* __restrict__ x) {
+k_coarse_mx(const double* __restrict__ AinvT, int n, const __nv_bfloat16* b, float* __restrict__ x) {
   pdl_next();
   __shared__ double rs[1024];
   const int l8 = threadIdx.x & 7;
@@ -1167,7 +1165,7 @@ k_coarse_mx(const double* __restrict__ AinvT, int n, const __nv_bfloat16* __rest
 }
 
 // ------------------------------------------------------------ vector ops
-__global__ void k_f64_to_f32(const double* __restrict__ a, float* __restrict__ b, long long n) {
+__global__ void k_f64_to_f32(const double* a, float* __restrict__ b, long long n) {
   pdl_next();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1201,8 +1199,8 @@ __global__ void k_scale_out(const float* __restrict__ e32, const double* __restr
 // not depend on the GPU.
 constexpr int kUpdBlocks = 1184;  // eight per SM of a B200
 __global__ void __launch_bounds__(kBlock)
-k_fcg64_update(double* sc, double* __restrict__ x, const float* __restrict__ p, double* __restrict__ r,
-               const double* __restrict__ a, float* __restrict__ r32, long long n, Reduce2 R) {
+k_fcg64_update(double* sc, double* __restrict__ x, const float* p, double* __restrict__ r,
+               const double* a, float* __restrict__ r32, long long n, Reduce2 R) {
   pdl_next();
   pdl_wait();
   __shared__ double smem[8];
@@ -1230,7 +1228,7 @@ k_fcg64_update(double* sc, double* __restrict__ x, const float* __restrict__ p, 
 // p = q / s + beta p  (first: p = q / s), s the scale of the FP32 residual,
 // computed in FP64 and stored in FP32: the search direction only has to be
 // the same vector in a = A p and in x += lam p, which it is
-__global__ void k_fcg64_p(const double* __restrict__ sc, float* __restrict__ p, const float* __restrict__ q,
+__global__ void k_fcg64_p(const double* sc, float* __restrict__ p, const float* q,
                           long long n, int first) {
   pdl_next();
   pdl_wait();
@@ -1254,7 +1252,7 @@ __global__ void k_fcg64_p(const double* __restrict__ sc, float* __restrict__ p, 
   }
 }
 
-__global__ void k_f32_to_f64(const float* __restrict__ a, double* __restrict__ b, long long n) {
+__global__ void k_f32_to_f64(const float* a, double* __restrict__ b, long long n) {
   pdl_next();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1262,7 +1260,7 @@ __global__ void k_f32_to_f64(const float* __restrict__ a, double* __restrict__ b
 }
 
 // r32 = r * sc[slot]
-__global__ void k_scale_to32(const double* __restrict__ r, const double* __restrict__ sc, int slot,
+__global__ void k_scale_to32(const double* r, const double* sc, int slot,
                              float* __restrict__ r32, long long n) {
   pdl_next();
   pdl_wait();
@@ -1272,7 +1270,7 @@ __global__ void k_scale_to32(const double* __restrict__ r, const double* __restr
 
 // two FP64 dot products (x, y) and (x, y2) with the epilogue of R
 __global__ void __launch_bounds__(kBlock)
-k_dot2_64(const double* __restrict__ xv, const float* __restrict__ yv, const double* __restrict__ y2,
+k_dot2_64(const double* xv, const float* yv, const double* y2,
           long long n, Reduce2 R) {
   pdl_next();
   pdl_wait();
@@ -1494,18 +1492,18 @@ static void mf_launch(int mode, const MFArgsT<T>& g, const TX* x, const T* b, T*
 
 // pre-smoothing from zero with the damping over the diagonal formed: y = wd b,
 // four nodes per thread (16-byte accesses when all three vectors allow them)
-__global__ void __launch_bounds__(kBlock) k_wd_scale(const float* __restrict__ wd, const float* __restrict__ b,
+__global__ void __launch_bounds__(kBlock) k_wd_scale(const float* wd, const float* b,
                                                      float* __restrict__ y, long long n) {
   pdl_next();
   pdl_wait();
   const long long i0 = ((long long)blockIdx.x * kBlock + threadIdx.x) * 4;
   if (i0 >= n) return;
   if (i0 + 4 <= n && (((uintptr_t)wd | (uintptr_t)b | (uintptr_t)y) & 15) == 0) {
-    const float4 w = __ldg(reinterpret_cast<const float4*>(wd + i0));
-    const float4 v = __ldg(reinterpret_cast<const float4*>(b + i0));
+    const float4 w = *reinterpret_cast<const float4*>(wd + i0);
+    const float4 v = *reinterpret_cast<const float4*>(b + i0);
     *reinterpret_cast<float4*>(y + i0) = make_float4(w.x * v.x, w.y * v.y, w.z * v.z, w.w * v.w);
   } else {
-    for (long long i = i0; i < n && i < i0 + 4; ++i) y[i] = __ldg(wd + i) * __ldg(b + i);
+    for (long long i = i0; i < n && i < i0 + 4; ++i) y[i] = wd[i] * b[i];
   }
 }
 
@@ -1712,7 +1710,7 @@ void mx_fcg64_update(double* sc, double* x, const float* p, double* r, const dou
 // b (layout bl) = a (natural), 3D, M nodes a side: FP64 to FP32, and FP64
 // copied (grids of plane_node)
 
-__global__ void k_f64_to_f32_lay(const double* __restrict__ a, float* __restrict__ b, VLay bl, int M) {
+__global__ void k_f64_to_f32_lay(const double* a, float* __restrict__ b, VLay bl, int M) {
   pdl_next();
   pdl_wait();
   int ix, iy, iz;
@@ -1721,7 +1719,7 @@ __global__ void k_f64_to_f32_lay(const double* __restrict__ a, float* __restrict
   b[bl.at(ix, iy, iz)] = (float)a[i];
 }
 
-__global__ void k_f64_copy_lay(const double* __restrict__ a, double* __restrict__ b, VLay bl, int M) {
+__global__ void k_f64_copy_lay(const double* a, double* __restrict__ b, VLay bl, int M) {
   pdl_next();
   pdl_wait();
   int ix, iy, iz;
@@ -1731,7 +1729,7 @@ __global__ void k_f64_copy_lay(const double* __restrict__ a, double* __restrict_
 }
 
 // b (natural) = a (layout al), FP64, 3D
-__global__ void k_f64_from_lay(const double* __restrict__ a, VLay al, double* __restrict__ b, int M) {
+__global__ void k_f64_from_lay(const double* a, VLay al, double* __restrict__ b, int M) {
   pdl_next();
   pdl_wait();
   int ix, iy, iz;
