@@ -866,7 +866,7 @@ __device__ __forceinline__ double div_by(double a, double u, double y) {
 }
 __device__ __forceinline__ bool div_by_ok(double a, double u, double q) {
   auto mid = [](double v) { return (((unsigned)__double2hiint(v) >> 20) & 0x7ff) - 300u < 1400u; };
-  return a == 0.0 || (mid(a) && mid(u) && mid(q));
+  return mid(u) && (a == 0.0 || (mid(a) && mid(q)));  // 1 / u may be infinite: then not even 0 / u holds
 }
 
 // A_BB c = r_B of a vertex block with its stored factors: lane t brings member
