@@ -538,13 +538,14 @@ __device__ __forceinline__ bool q2_face(const int c[3], int M, int dmask) {
 // colour still runs, only the unknowns wait for it.
 constexpr int kTileRows = 32, kTileT = 256;
 constexpr size_t kTileSmem = 2 * 125 * kTileRows * sizeof(double);
-// rows of a colour up to which a level takes this form; beyond, the strided
-// reads of x bound it and a thread per row is faster
-constexpr long long kTileMax = 12000;
-#ifndef SSCT
-#define SSCT 100000
-#endif
-constexpr long long kSscTileMax = SSCT;
+// Rows of a colour up to which an SOR sweep takes this form, and nodes up to
+// which an SSC sweep does; beyond, the strided reads of x bound it and a thread
+// per row is faster.  A coarse level of at most 1,024 unknowns leaves 2^k and
+// 3 2^k cells a side.  SOR sweep by tiles and by rows, us: 49^3 nodes 112 and
+// 198, 65^3 (10,648 rows) 130 and 238, 97^3 (35,937 rows) 310 and 314, 129^3
+// 688 and 440.  SSC sweep: 25^3 90 and 132, 33^3 128 and 141, 49^3 232 and 189,
+// 65^3 490 and 328.
+constexpr long long kTileMax = 12000, kSscTileMax = 40000;
 
 // SSC: the residuals r = b - A x of the rows of one <geometric-ssc> colour
 // instead (every class, blockIdx.z; b may be r): see k_ssc_solve_q2.
