@@ -2279,11 +2279,14 @@ __device__ __forceinline__ void block_solve3(const T* B, const T* r, T* t) {
 // where the stored coefficients are 0 too).  FP64 Q2 matvec: 49^3 nodes 191 ->
 // 138 us, 25^3 58 -> 25 us, 13^3 41 -> 20 us against a thread per node with
 // the slots unrolled.
-// nodes from which the FP32 form takes a thread per node (97^3 nodes: 443 us so,
-// 814 us a thread per scalar row, 656 us before either; 49^3: 82, 122, 140 us;
-// 25^3: 26 and 24 us); in FP64 the scalar rows are as fast there (921 us, 0.69
-// of the copy peak; a thread per node 1,128 us) and faster below
-constexpr long long kNode3Min = 50000;
+// Nodes from which the FP32 form takes a thread per node.  A sweep by scalar
+// rows and by nodes, us (all levels of the hierarchy, the top one by either):
+// Q2 17^3 55 and 61 (the levels below by nodes too), 25^3 42 and 39, 33^3 98
+// and 87, 49^3 160 and 120; Q1 21^3 16.4 and 16.4, 29^3 20.6 and 16.7, 41^3 39
+// and 29.  At 97^3 nodes 814 and 443 us.  In FP64 the scalar rows are as fast
+// there (921 us, 0.69 of the copy peak; a thread per node 1,128 us) and faster
+// below.
+constexpr long long kNode3Min = 12000;
 enum Row3Op { ROW3_MUL, ROW3_RES, ROW3_JACOBI };
 constexpr int kRow3Nodes = 64, kRow3T = 3 * kRow3Nodes;
 
@@ -2543,12 +2546,15 @@ k_jacobi3(const double* __restrict__ A, long long N, long long Np, int center, d
 }
 
 // The transfer sums of a node's three components with the terms in loops, for
-// large levels: a thread per scalar unknown repeats the node's indices and
-// weights three times and is bound by them there (Q2, 49^3 coarse nodes:
-// restriction 150 us, 74 so; prolongation to 97^3 105 and 57 us; the other
-// way round on small levels, where memory waits are the time: 19 and 31 us
-// at 13^3).
-constexpr long long kXferLoopMin = 30000;
+// large Q2 levels: a thread per scalar unknown repeats the node's indices and
+// weights three times and is bound by them there, while on small levels memory
+// waits are the time.  Thread per unknown and loops, us: restriction to 25^3
+// nodes 33.2 and 33.7, to 33^3 59 and 55, to 49^3 150 and 77; prolongation to
+// 33^3 10.6 and 14.6, to 49^3 18.9 and 18.4, to 65^3 37 and 27, to 97^3 105 and
+// 59.  Q1 has a quarter of the terms and stays per unknown: restriction to 33^3
+// 8.7 and 15.7, to 57^3 23 and 31; prolongation to 65^3 14.7 and 18.7, to 113^3
+// 56 and 61.
+constexpr long long kRestrictLoopMin = 30000, kProlongLoopMin = 100000;
 
 template <int P, typename T>
 __device__ __forceinline__ void restrict3_loop(const int cJ[3], int MC, int MF, int dmask, const T* rf,
@@ -2649,23 +2655,21 @@ k_prolong3(int MF, int MC, int dmask, const T* xc, T* __restrict__ xf) {
 template <typename T>
 static void launch_restrict3(int order, long long MC, long long MF, int dmask, const T* rf, T* rc, T* rhsc, T* solc,
                              cudaStream_t st) {
-  const bool big = MC * MC * MC >= kXferLoopMin;
+  const bool big = order == 2 && MC * MC * MC >= kRestrictLoopMin;
   const dim3 g((unsigned)(((big ? 1 : 3) * MC + 31) / 32), (unsigned)((MC + 7) / 8), (unsigned)MC), t(32, 8);
   const int mc = (int)MC, mf = (int)MF;
-  if (order == 2 && big) launch_pdl(k_restrict3<2, true, T>, g, t, 0, st, mc, mf, dmask, rf, rc, rhsc, solc);
+  if (big) launch_pdl(k_restrict3<2, true, T>, g, t, 0, st, mc, mf, dmask, rf, rc, rhsc, solc);
   else if (order == 2) launch_pdl(k_restrict3<2, false, T>, g, t, 0, st, mc, mf, dmask, rf, rc, rhsc, solc);
-  else if (big) launch_pdl(k_restrict3<1, true, T>, g, t, 0, st, mc, mf, dmask, rf, rc, rhsc, solc);
   else launch_pdl(k_restrict3<1, false, T>, g, t, 0, st, mc, mf, dmask, rf, rc, rhsc, solc);
 }
 
 template <typename T>
 static void launch_prolong3(int order, long long MF, long long MC, int dmask, const T* xc, T* xf, cudaStream_t st) {
-  const bool big = MF * MF * MF >= kXferLoopMin;
+  const bool big = order == 2 && MF * MF * MF >= kProlongLoopMin;
   const dim3 g((unsigned)(((big ? 1 : 3) * MF + 31) / 32), (unsigned)((MF + 7) / 8), (unsigned)MF), t(32, 8);
   const int mc = (int)MC, mf = (int)MF;
-  if (order == 2 && big) launch_pdl(k_prolong3<2, true, T>, g, t, 0, st, mf, mc, dmask, xc, xf);
+  if (big) launch_pdl(k_prolong3<2, true, T>, g, t, 0, st, mf, mc, dmask, xc, xf);
   else if (order == 2) launch_pdl(k_prolong3<2, false, T>, g, t, 0, st, mf, mc, dmask, xc, xf);
-  else if (big) launch_pdl(k_prolong3<1, true, T>, g, t, 0, st, mf, mc, dmask, xc, xf);
   else launch_pdl(k_prolong3<1, false, T>, g, t, 0, st, mf, mc, dmask, xc, xf);
 }
 

@@ -55,7 +55,7 @@ def test_q2_sweeps(oracle_mod, G, ctx, n0, level, mask):
     assert np.array_equal(Y.get(), o.residual(x, b))
 
 
-# coarse nodes a side 25 and 33 (Q2), 29 and 33 (Q1): a thread per scalar unknown below 30,000 nodes, per node above
+# Q2 by threads per scalar unknown and, from 33^3 coarse and 49^3 fine nodes on, per node; Q1 per unknown
 @pytest.mark.parametrize("order,n0,level", [(2, 3, 3), (2, 1, 5), (1, 7, 3), (1, 1, 6)])
 def test_vector_transfers(oracle_mod, G, ctx, order, n0, level):
     o, g = make_pair(oracle_mod, G, ctx, order, 3, n0, level, 0b011001, assemble=False)
@@ -69,8 +69,8 @@ def test_vector_transfers(oracle_mod, G, ctx, order, n0, level):
         assert np.array_equal(X.get(), o.prolongate(xc, x, l - 1)), f"prolongate {l}"
 
 
-# nodes a side 29 and 41 (Q1), 33 and 49 (Q2): FP32 rows a thread per scalar row below 50,000 nodes, per node above
-@pytest.mark.parametrize("order,n0,level", [(1, 7, 2), (1, 5, 3), (2, 1, 4), (2, 3, 3)])
+# nodes a side 21 to 41 (Q1), 17 to 49 (Q2): FP32 rows a thread per scalar row below 12,000 nodes, per node above
+@pytest.mark.parametrize("order,n0,level", [(1, 5, 2), (1, 3, 3), (1, 7, 2), (1, 5, 3), (2, 1, 3), (2, 3, 2), (2, 1, 4), (2, 3, 3)])
 def test_mixed_vector_step(oracle_mod, G, ctx, order, n0, level):
     O, C = oracle_mod, G._capi
     o, g = make_pair(O, G, ctx, order, 3, n0, level, 0b000001)
