@@ -3874,11 +3874,18 @@ long long tail_need(const LevelView& L) {  // the matrix and four vectors
   return (ns + 4) * L.N;
 }
 
-// One CTA has 208 KB for the levels, half of it used in 3D: there a cycle takes
-// few steps for the matrix it brings in (9^3 and 5^3 nodes, 183 KB and seven
-// Jacobi steps: a 128^3-cell solve 8.0 -> 8.3 ms; 7^3 and 4^3 with their colours:
-// a cycle on 48^3 273 -> 258 us).  The problems of a batch share an SM where
-// there are more of them than SMs (a second wave would double the time).
+// One CTA has 208 KB for the levels, half of it used in 3D: the only levels
+// that fit the whole and not the half are 9^3 and 5^3 nodes together (183 KB),
+// and a cycle takes few steps there for the matrices it brings in.  A cycle
+// with the half and the whole, us: Jacobi V(1,1) of 32^3 cells 57 and 48, 64^3
+// 75 and 79, 128^3 292 and 296, 256^3 1,876 and 1,881; SOR V(1,1) 145 and 127,
+// 229 and 216, 765 and 749, 4,540 and 4,535; a 128^3-cell CG solve 8.0 and 8.3
+// ms.  A CTA has an SM to itself (512 threads of 96 registers), so the problems
+// of a batch of more than 148 take turns, and what they bring into the launch
+// is done once per turn: the room is divided by the turns, and the levels left
+// out run in launches over the whole batch.  Ten CG steps with the room divided
+// and whole, us: 32^2 cells x 149 845 and 879, x 297 1,054 and 1,122; 64^2 x 160
+// 1,371 and 1,386, x 400 2,546 and 2,572; 128^2 x 297 5,749 and 5,846.
 long long tail_room(int dim, int nb) { return (dim == 3 ? 104 : 208) * 1024 / 8 / ((nb + 147) / 148); }
 
 template <int CAP>
