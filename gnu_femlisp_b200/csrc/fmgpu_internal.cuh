@@ -116,7 +116,7 @@ __device__ __forceinline__ void dr_finish(double lane_sum, const Reduce& R, doub
 // launch_pdl (on a small grid) may start while its predecessor in the stream
 // still runs.  pdl_next lets the successor start; pdl_wait waits until the
 // predecessor has finished and its writes are visible.  Every kernel launched
-// so calls both, pdl_wait before its first access to anything that a kernel
+// so calls pdl_next (or pdl_next_light) and pdl_wait, pdl_wait before its first access to anything that a kernel
 // of the same sequence writes; before it, only what was in place when the
 // sequence began (matrices, damping, factors, indices) is read.  __ldg and
 // `const T* __restrict__` (which lets the compiler use it) are for those alone:
@@ -126,8 +126,17 @@ __device__ __forceinline__ void dr_finish(double lane_sum, const Reduce& R, doub
 // neither the compiler nor the caches serve from before the wait.  At least one
 // thread of every launch passes pdl_wait, so a launch never ends before its
 // predecessor and waiting for one kernel is waiting for all before it.
+constexpr unsigned kPdlBlocks = 148;  // a small grid: at most a block per SM
 __device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Letting the successor start takes a block's turn at issuing: on a large grid
+// of blocks that do a few accesses a thread it is 40 % of their time (FP64 to
+// FP32 of 2^27 elements 383 us, 541 so; 2^22 12.4 and 19.4), and such blocks end
+// as soon as they could tell.  On small grids their successors gain by it (a
+// 64^2-cell solve 787 us, 795 without).
+__device__ __forceinline__ void pdl_next_light() {
+  if (gridDim.x * gridDim.y * gridDim.z <= kPdlBlocks) pdl_next();
+}
 
 // The stream this thread's last such launch went to.  A sequence begins with a
 // launch that waits for everything before it (the first one on a stream, and
@@ -143,8 +152,6 @@ inline void pdl_break() { t_pdl_stream = nullptr; }
 // on large ones (launch_pdl: Q2 residual among the SOR sweeps of 129^3 nodes,
 // 31.9 -> 34.9 ms a solve with all launches early; FCG update of 97^3 nodes,
 // 3.83 -> 4.07 ms), and the elasticity rows lose always (launch_late).
-constexpr long long kPdlBlocks = 148;
-
 template <typename... KA, typename... A>
 inline void launch_after(bool early, void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                          A... args) {

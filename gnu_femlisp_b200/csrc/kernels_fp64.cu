@@ -326,7 +326,7 @@ template <int D>
 __global__ void __launch_bounds__(kBlock)
 k_jacobi_q2(const double* __restrict__ A, long long N, long long Np, long long M, double damp,
             const double* __restrict__ omega, double* x, double* r, int write_r, const __grid_constant__ Q2Layout lay) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   constexpr int C = St<D, 2>::CENTER;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -764,7 +764,7 @@ k_jacobi_res_q2c(const double* __restrict__ A, long long Np, int M, double damp,
 __global__ void __launch_bounds__(kBlock)
 k_jacobi(const double* __restrict__ Dg, long long N, double damp, const double* __restrict__ omega,
          double* x, double* r, int write_r, long long vs, long long as) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
@@ -1083,7 +1083,7 @@ k_ssc_solve_q2(int Mi, int dmask, int colour, double omega, double* x, const dou
 template <int D>
 __global__ void __launch_bounds__(kBlock)
 k_psc_q1(const double* __restrict__ A, long long N, long long Np, double damp, double* x, const double* r) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   constexpr int C = St<D, 1>::CENTER;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1128,7 +1128,7 @@ k_psc_block_q2(long long M, int dmask, const double* r, const double* __restrict
 template <int D>
 __global__ void __launch_bounds__(kBlock)
 k_psc_gather_q2(long long N, long long M, int dmask, double damp, const double* C, double* x) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   constexpr int NB = D == 1 ? 3 : (D == 2 ? 9 : 27);
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1857,14 +1857,14 @@ k_coarse_solve(const double* __restrict__ AinvT, int n, double damp, double* x, 
 
 // ------------------------------------------------------------ vector ops
 __global__ void k_fill(double* x, long long n, double v) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) x[i] = v;
 }
 
 __global__ void k_copy(const double* x, double* __restrict__ y, long long n) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) y[i] = x[i];
@@ -1873,7 +1873,7 @@ __global__ void k_copy(const double* x, double* __restrict__ y, long long n) {
 // axpy!: y := y + alpha x (alpha from a device slot when aslot >= 0)
 __global__ void k_axpy(double alpha, const double* sc, int aslot, const double* x,
                        double* y, long long n) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -1987,7 +1987,7 @@ k_cg_update(const double* sc, double* __restrict__ x, const double* p, double* _
 // p := (new_alpha/alpha) p (scal!), then p := p + q (m+!)
 __global__ void k_p_update(const double* sc, double* __restrict__ p, const double* q, long long n, long long vs,
                            const double* frozen) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -2528,7 +2528,7 @@ static void launch_row3(int order, const T* A, long long N, long long Np, long l
 __global__ void __launch_bounds__(kBlock)
 k_jacobi3(const double* __restrict__ A, long long N, long long Np, int center, double damp,
           const double* __restrict__ omega, double* x, double* r, int write_r) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
@@ -2951,7 +2951,7 @@ k_galerkin(const double* __restrict__ AF, long long NpF, int MF, double* __restr
 __global__ void __launch_bounds__(kBlock)
 k_bdiag3(const double* __restrict__ A, long long N, long long Np, int center, int mode,
          const double* w, const double* x, double* __restrict__ y) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
@@ -2971,7 +2971,7 @@ k_bdiag3(const double* __restrict__ A, long long N, long long Np, int center, in
 // y = x + w .* v with w per node (y may be x)
 __global__ void k_xpwv3(const double* x, const double* w, const double* v, double* y,
                         long long N) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
@@ -2982,7 +2982,7 @@ __global__ void k_xpwv3(const double* x, const double* w, const double* v, doubl
 // acc_i += sum_k a_ik b_ik (per-node dot of two vectors)
 __global__ void k_acc_prod3(double* __restrict__ acc, const double* a, const double* b,
                             long long N) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
@@ -2998,7 +2998,7 @@ template <typename T>
 __global__ void __launch_bounds__(kBlock)
 k_jacobi0_3(const T* __restrict__ A, long long N, long long Np, int center, float damp,
             const double* __restrict__ omega, const T* b, T* __restrict__ x) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
@@ -3016,7 +3016,7 @@ k_jacobi0_3(const T* __restrict__ A, long long N, long long Np, int center, floa
 template <typename TI, typename TO>
 __global__ void k_vscale(const TI* x, const double* sc, int slot, int mode,
                          TO* __restrict__ y, long long n) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;

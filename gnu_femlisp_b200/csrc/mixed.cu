@@ -1166,7 +1166,7 @@ k_coarse_mx(const double* __restrict__ AinvT, int n, const __nv_bfloat16* b, flo
 
 // ------------------------------------------------------------ vector ops
 __global__ void k_f64_to_f32(const double* a, float* __restrict__ b, long long n) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) b[i] = (float)a[i];
@@ -1230,7 +1230,7 @@ k_fcg64_update(double* sc, double* __restrict__ x, const float* p, double* __res
 // the same vector in a = A p and in x += lam p, which it is
 __global__ void k_fcg64_p(const double* sc, float* __restrict__ p, const float* q,
                           long long n, int first) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   const long long i0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i0 >= n) return;
@@ -1253,7 +1253,7 @@ __global__ void k_fcg64_p(const double* sc, float* __restrict__ p, const float* 
 }
 
 __global__ void k_f32_to_f64(const float* a, double* __restrict__ b, long long n) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) b[i] = (double)a[i];
@@ -1262,7 +1262,7 @@ __global__ void k_f32_to_f64(const float* a, double* __restrict__ b, long long n
 // r32 = r * sc[slot]
 __global__ void k_scale_to32(const double* r, const double* sc, int slot,
                              float* __restrict__ r32, long long n) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) r32[i] = (float)(r[i] * sc[slot]);
@@ -1494,7 +1494,7 @@ static void mf_launch(int mode, const MFArgsT<T>& g, const TX* x, const T* b, T*
 // four nodes per thread (16-byte accesses when all three vectors allow them)
 __global__ void __launch_bounds__(kBlock) k_wd_scale(const float* wd, const float* b,
                                                      float* __restrict__ y, long long n) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   const long long i0 = ((long long)blockIdx.x * kBlock + threadIdx.x) * 4;
   if (i0 >= n) return;
@@ -1525,7 +1525,7 @@ __device__ __forceinline__ bool plane_node(int M, int& ix, int& iy, int& iz, lon
 // in the same order; cells outside the grid count zero); Dirichlet nodes
 // (identity rows) get the damping itself
 __global__ void __launch_bounds__(kBlock) k_mf_wd(MFArgs g, float* __restrict__ wd) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   const int M = g.M, n = g.n, dm = g.dmask;
   int ix, iy, iz;
@@ -1711,7 +1711,7 @@ void mx_fcg64_update(double* sc, double* x, const float* p, double* r, const dou
 // copied (grids of plane_node)
 
 __global__ void k_f64_to_f32_lay(const double* a, float* __restrict__ b, VLay bl, int M) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   int ix, iy, iz;
   long long i;
@@ -1720,7 +1720,7 @@ __global__ void k_f64_to_f32_lay(const double* a, float* __restrict__ b, VLay bl
 }
 
 __global__ void k_f64_copy_lay(const double* a, double* __restrict__ b, VLay bl, int M) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   int ix, iy, iz;
   long long i;
@@ -1730,7 +1730,7 @@ __global__ void k_f64_copy_lay(const double* a, double* __restrict__ b, VLay bl,
 
 // b (natural) = a (layout al), FP64, 3D
 __global__ void k_f64_from_lay(const double* a, VLay al, double* __restrict__ b, int M) {
-  pdl_next();
+  pdl_next_light();
   pdl_wait();
   int ix, iy, iz;
   long long i;
