@@ -590,9 +590,13 @@ __device__ __forceinline__ long long soff(int s, long long M) {
 // sums in slot order either way.
 // The one-row form of up to 27 slots fetches its coefficients while the
 // previous launch still runs and has all its loads in flight (the launch bound
-// keeps the compiler from sinking them).
+// keeps the compiler from sinking them).  The four-row form wants warps more
+// than loads in flight: with a bound of four blocks per SM (64 registers), of
+// three, of two (128) and none (40-60), the residual of 129^3 nodes from BF16 to
+// BF16 takes 47, 53, 63 and 55 us, of 161^3 in FP32 86, 99, 133 and 96 us, the
+// smoothing with its dot products there 108, 115, 130 and 114 us.
 template <int D, int P, int MODE, typename TB, typename TY, bool RED, int RPT>
-__global__ void __launch_bounds__(kBlock, RPT == 1 && P == 1 ? 3 : P == 1 ? 2 : 0)
+__global__ void __launch_bounds__(kBlock, P == 2 ? 0 : RPT == 4 ? 4 : 3)
 k_st32(const float* __restrict__ A, long long N, long long Np, long long M, float w, const float* __restrict__ om,
        const float* x, const TB* b, TY* __restrict__ y, const double* v, const double* v2, Reduce2 R) {
   pdl_next();
