@@ -1613,8 +1613,11 @@ void st32_launch(const Lev32& L, const float* x, const void* b, void* y, const d
     launch_pdl(k_st32<D, P, MODE, TB, TY, RED, W>, g1((L.N + W - 1) / W), kBlock, 0, st,
                L.A, L.N, L.Np, L.M, L.w, L.om, x, (const TB*)b, (TY*)y, v, v2, r0);
   else
-    launch_early(k_st32<D, P, MODE, TB, TY, RED, 1>, g1(L.N), kBlock, 0, st, L.A, L.N, L.Np, L.M, L.w, L.om, x,
-                                                                    (const TB*)b, (TY*)y, v, v2, r0);
+    // the 3D Q2 rows do not fetch before they wait: an early start only takes
+    // room from the previous launch (a mixed CG step of 16^3 cells 137 us, 143
+    // so, of 24^3 207 and 213, of 32^3 322 and 330)
+    launch_after(St32<D, P>::NS <= 27, k_st32<D, P, MODE, TB, TY, RED, 1>, g1(L.N), kBlock, 0, st, L.A, L.N, L.Np,
+                 L.M, L.w, L.om, x, (const TB*)b, (TY*)y, v, v2, r0);
 }
 
 void mx_level_apply(int mode, const Lev32& L, const float* x, const void* b, bool b_bf16, void* y, bool y_bf16,
@@ -1696,7 +1699,10 @@ void mx_prolong(const Lev32& C, const Lev32& F, const float* xc, float* xf, cuda
 
 void mx_coarse(const double* AinvT, int n, const __nv_bfloat16* b, float* x, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  launch_pdl(k_coarse_mx, 1, 1024, 0, st, AinvT, n, b, x);
+  // beyond 128 unknowns nothing is fetched before the wait, and 1,024 waiting
+  // threads cost the previous launch (343 unknowns: a mixed CG step of 12^3 Q2
+  // cells 110 us, 118 with an early start; 216: 160^3 Q1 634 and 638)
+  launch_after(n <= 128, k_coarse_mx, 1, 1024, 0, st, AinvT, n, b, x);
 }
 
 void mx_f64_to_f32(const double* a, float* b, long long n, cudaStream_t st) {
