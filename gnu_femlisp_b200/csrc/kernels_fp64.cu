@@ -1881,8 +1881,14 @@ __global__ void k_axpy(double alpha, const double* sc, int aslot, const double* 
   y[i] = fma(a, x[i], y[i]);
 }
 
-// DR4096 dot product (x, y)
-__global__ void __launch_bounds__(kBlock, 4)
+// DR4096 dot product (x, y).  Q pairs of elements in flight a thread, MB blocks
+// per SM: four and four while the blocks fit one wave so (one chunk 4.5 us, 4.8
+// with two pairs and eight blocks), two and eight beyond, where the second wave
+// would be nearly empty (669 chunks 7.8 us and 9.0 in the other form, 1,019 9.5
+// and 11.0, 1,184 9.3 and 11.0; from 1,500 on alike).
+constexpr unsigned kDotWave = 4 * 148;
+template <int Q, int MB>
+__global__ void __launch_bounds__(kBlock, MB)
 k_dot(const double* x, const double* y, long long n, Reduce R, long long vs) {
   pdl_next();
   pdl_wait();
@@ -1892,16 +1898,16 @@ k_dot(const double* x, const double* y, long long n, Reduce R, long long vs) {
   y += bq * vs;
   R = batch_reduce(R, (unsigned)bq);
   const long long base = (long long)blockIdx.x * kChunk + 2 * threadIdx.x;
-  // pairs by 16-byte loads, four at a time before their terms.  The library's
+  // pairs by 16-byte loads, Q at a time before their terms.  The library's
   // own vectors start on 16 bytes; those a caller hands to fmg_dot_noalloc
   // need only the 8 of a double, and then come one by one.
   const bool wide = (((uintptr_t)x | (uintptr_t)y) & 15) == 0;
   double acc = 0.0;
 #pragma unroll
-  for (int m0 = 0; m0 < kPairsPerThread; m0 += 4) {
-    double2 u[4], v[4];
+  for (int m0 = 0; m0 < kPairsPerThread; m0 += Q) {
+    double2 u[Q], v[Q];
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
+    for (int m = 0; m < Q; ++m) {
       const long long i0 = base + 512LL * (m0 + m);
       if (wide && i0 + 1 < n) {
         u[m] = *reinterpret_cast<const double2*>(x + i0);
@@ -1918,7 +1924,7 @@ k_dot(const double* x, const double* y, long long n, Reduce R, long long vs) {
       }
     }
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
+    for (int m = 0; m < Q; ++m) {
       const long long i0 = base + 512LL * (m0 + m);
       if (i0 < n) acc = fma(u[m].x, v[m].x, acc);
       if (i0 + 1 < n) acc = fma(u[m].y, v[m].y, acc);
@@ -3637,13 +3643,14 @@ void launch_axpy(double alpha, const double* sc, int aslot, const double* x, dou
   if (n > 0) launch_early(k_axpy, grid1(n), kBlock, 0, st, alpha, sc, aslot, x, y, n);
 }
 void launch_dot(const double* x, const double* y, long long n, const Reduce& R, cudaStream_t st) {
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  launch_early(k_dot, nchunks(n), kBlock, 0, st, x, y, n, R, 0);
+  launch_dot_b(x, y, n, 0, 1, R, st);
 }
 void launch_dot_b(const double* x, const double* y, long long n, long long vs, int nb, const Reduce& R,
                   cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  launch_early(k_dot, dim3(nchunks(n), (unsigned)nb), kBlock, 0, st, x, y, n, R, vs);
+  const dim3 g(nchunks(n), (unsigned)nb);
+  if (g.x * g.y <= kDotWave) launch_early(k_dot<4, 4>, g, kBlock, 0, st, x, y, n, R, vs);
+  else launch_early(k_dot<2, 8>, g, kBlock, 0, st, x, y, n, R, vs);
 }
 void launch_cg_update(const double* sc, double* x, const double* p, double* r, const double* a, double* w,
                       double* w2, double* q, long long n, const Reduce& R, cudaStream_t st) {

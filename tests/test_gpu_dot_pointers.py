@@ -17,7 +17,7 @@ def test_dot_noalloc_of_slices(oracle_mod, ox, oy):
     ctx = G.Context(0)
     lib = G._capi.load()
     out = torch.zeros(1, dtype=torch.float64, device="cuda")
-    for n in (1, 2, 511, 4095, 4096, 4097, 3 * 4096 + 2):
+    for n in (1, 2, 511, 4095, 4096, 4097, 3 * 4096 + 2, 592 * 4096, 592 * 4096 + 3):  # the last: more than a wave
         rng = np.random.default_rng(10 * n + ox)
         x, y = rng.standard_normal(n + 4), rng.standard_normal(n + 4)
         xd, yd = torch.from_numpy(x).to("cuda"), torch.from_numpy(y).to("cuda")
