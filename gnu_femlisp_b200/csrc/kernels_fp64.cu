@@ -1432,7 +1432,8 @@ template <int D, int P>
 __global__ void __launch_bounds__(kBlock)
 k_restrict(int MC, int MF, int dmask, const double* rf, double* __restrict__ rc,
            double* __restrict__ rhsc, double* __restrict__ solc, long long fs, long long cs) {
-  pdl_next();
+  if (D == 1) pdl_next_light();  // 32 of 256 threads have work there
+  else pdl_next();
   pdl_wait();
   if (D == 1 && threadIdx.y != 0) return;
   if (D < 3) {  // problem of a batched level: fine stride fs, coarse stride cs
@@ -1461,7 +1462,8 @@ template <int D>
 __global__ void __launch_bounds__(kBlock)
 k_prolong_q1f(int MF, int MC, int dmask, const double* xc, double* __restrict__ xf, long long fs,
               long long cs) {
-  pdl_next();
+  if (D == 1) pdl_next_light();  // 32 of 256 threads have work there
+  else pdl_next();
   pdl_wait();
   if (D == 1 && threadIdx.y != 0) return;
   if (D < 3) {  // problem of a batched level
@@ -1514,7 +1516,8 @@ template <int D, int P>
 __global__ void __launch_bounds__(kBlock)
 k_prolong(int MF, int MC, int dmask, const double* xc, double* __restrict__ xf, long long fs,
           long long cs) {
-  pdl_next();
+  if (D == 1) pdl_next_light();  // 32 of 256 threads have work there
+  else pdl_next();
   pdl_wait();
   if (D == 1 && threadIdx.y != 0) return;
   if (D < 3) {  // problem of a batched level

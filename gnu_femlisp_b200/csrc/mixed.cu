@@ -590,16 +590,18 @@ __device__ __forceinline__ long long soff(int s, long long M) {
 // sums in slot order either way.
 // The one-row form of up to 27 slots fetches its coefficients while the
 // previous launch still runs and has all its loads in flight (the launch bound
-// keeps the compiler from sinking them).  The four-row form wants warps more
+// keeps the compiler from sinking them; 1D rows have three and want warps:
+// smoothing of 2^20 nodes with its dot products 18 us, 28 with the bound).  The four-row form wants warps more
 // than loads in flight: with a bound of four blocks per SM (64 registers), of
 // three, of two (128) and none (40-60), the residual of 129^3 nodes from BF16 to
 // BF16 takes 47, 53, 63 and 55 us, of 161^3 in FP32 86, 99, 133 and 96 us, the
 // smoothing with its dot products there 108, 115, 130 and 114 us.
 template <int D, int P, int MODE, typename TB, typename TY, bool RED, int RPT>
-__global__ void __launch_bounds__(kBlock, P == 2 ? 0 : RPT == 4 ? 4 : 3)
+__global__ void __launch_bounds__(kBlock, P == 2 || D == 1 ? 0 : RPT == 4 ? 4 : 3)
 k_st32(const float* __restrict__ A, long long N, long long Np, long long M, float w, const float* __restrict__ om,
        const float* x, const TB* b, TY* __restrict__ y, const double* v, const double* v2, Reduce2 R) {
-  pdl_next();
+  if (D == 1 || MODE == 3) pdl_next_light();
+  else pdl_next();
   constexpr int NS = St32<D, P>::NS;
   constexpr int C = St32<D, P>::CENTER;
   constexpr bool STAGE = RPT == 1 && NS <= 27;
@@ -742,7 +744,8 @@ template <int D, typename TR>
 __global__ void __launch_bounds__(kBlock)
 k_restrict_q1(int MC, int MF, int dmask, const TR* rf, __nv_bfloat16* __restrict__ bc,
               float* __restrict__ xc) {
-  pdl_next();
+  if (D == 1) pdl_next_light();  // 32 of 256 threads have work there
+  else pdl_next();
   pdl_wait();
   if (D == 1 && threadIdx.y != 0) return;
   const int c0 = (int)(blockIdx.x * 32 + threadIdx.x), c1 = D > 1 ? (int)(blockIdx.y * 8 + threadIdx.y) : 0;
@@ -804,7 +807,8 @@ template <int D, int P, typename TR>
 __global__ void __launch_bounds__(kBlock)
 k_restrict_mx(int MC, int MF, int dmask, const TR* rf, __nv_bfloat16* __restrict__ bc,
               float* __restrict__ xc) {
-  pdl_next();
+  if (D == 1) pdl_next_light();  // 32 of 256 threads have work there
+  else pdl_next();
   pdl_wait();
   if (D == 1 && threadIdx.y != 0) return;
   const int cJ[3] = {(int)(blockIdx.x * 32 + threadIdx.x), D > 1 ? (int)(blockIdx.y * 8 + threadIdx.y) : 0,
@@ -851,7 +855,8 @@ k_restrict_mx(int MC, int MF, int dmask, const TR* rf, __nv_bfloat16* __restrict
 template <int D>
 __global__ void __launch_bounds__(kBlock)
 k_prolong_q1(int MF, int MC, int dmask, const float* xc, float* __restrict__ xf) {
-  pdl_next();
+  if (D == 1) pdl_next_light();  // 32 of 256 threads have work there
+  else pdl_next();
   pdl_wait();
   if (D == 1 && threadIdx.y != 0) return;
   const int fi[3] = {(int)(blockIdx.x * 32 + threadIdx.x), D > 1 ? (int)(blockIdx.y * 8 + threadIdx.y) : 0,
@@ -1086,7 +1091,8 @@ k_prolong_q1v(int MF, int MC, int dmask, const float* xc, float* __restrict__ xf
 template <int D, int P>
 __global__ void __launch_bounds__(kBlock)
 k_prolong_mx(int MF, int MC, int dmask, const float* xc, float* __restrict__ xf) {
-  pdl_next();
+  if (D == 1) pdl_next_light();  // 32 of 256 threads have work there
+  else pdl_next();
   pdl_wait();
   if (D == 1 && threadIdx.y != 0) return;
   const int fi[3] = {(int)(blockIdx.x * 32 + threadIdx.x), D > 1 ? (int)(blockIdx.y * 8 + threadIdx.y) : 0,
