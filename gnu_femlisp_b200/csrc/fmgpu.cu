@@ -1410,6 +1410,7 @@ int fmg_set_node_damping(fmg_grid* g, int level, const double* host, long n) {
   int rc;
   if (!L.omega && (rc = dalloc(g, &L.omega, L.Np))) return rc;
   FMG_CK(g->ctx, cudaMemcpyAsync(L.omega, host, L.N * sizeof(double), cudaMemcpyHostToDevice, g->ctx->stream));
+  pdl_break();  // later launches fetch the damping early
   return FMG_OK;
 }
 

@@ -106,6 +106,7 @@ extern "C" int fmg_dot_noalloc(fmg_ctx* ctx, const double* x, const double* y, l
   R.epi = EPI_STORE;
   R.slot = 0;
   launch_dot(x, y, (long long)n, R, st);
+  pdl_break();  // the caller's next launch begins a sequence of its own
   e = cudaGetLastError();
   return e == cudaSuccess ? FMG_OK : ctx_error(ctx, FMG_ERR_CUDA, cudaGetErrorString(e));
 }
