@@ -1453,10 +1453,10 @@ k_restrict(int MC, int MF, int dmask, const double* rf, double* __restrict__ rc,
   solc[J] = 0.0;
 }
 
-// The same on Q1 levels, a thread per pair of fine nodes 2 j, 2 j + 1 along x: the
-// pair shares its coarse values, every thread of a warp takes the same terms
-// (y and z are the warp's), and the loads and stores are coalesced.  Terms and
-// their order are prolong_node's.  Bound by HBM and the issue of its loads
+// xf := xf + I xc (see k_prolong) on Q1 levels, a thread per pair of fine nodes
+// 2 j, 2 j + 1 along x: the pair shares its coarse values, every thread of a warp
+// takes the same terms (y and z are the warp's), and the loads and stores are
+// coalesced.  Terms and their order are prolong_node's.  Bound by HBM and the issue of its loads
 // (257^3 fine nodes: 99 us, 197 us with a thread per fine node).
 template <int D>
 __global__ void __launch_bounds__(kBlock)
