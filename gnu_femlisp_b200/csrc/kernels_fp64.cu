@@ -288,7 +288,8 @@ template <int D, bool RES>
 __global__ void __launch_bounds__(kRowT, kRowMinBlocks)
 k_row_q1(const double* __restrict__ A, int N, long long Np, int M, const double* x, const double* b,
          double* y) {
-  pdl_next();
+  if (D == 1) pdl_next_light();
+  else pdl_next();
   const int i = blockIdx.x * kRowT + threadIdx.x;
   if (i >= N) return;
   const long long bq = blockIdx.y;  // problem of a batched level
@@ -307,7 +308,8 @@ __global__ void __launch_bounds__(kRowT, kRowMinBlocks)
 k_row_jacobi_q1(const double* __restrict__ A, int N, long long Np, int M, double damp,
                 const double* __restrict__ omega, const double* x, const double* b,
                 double* __restrict__ xout, double* r, int write_r) {
-  pdl_next();
+  if (D == 1) pdl_next_light();
+  else pdl_next();
   const int i = blockIdx.x * kRowT + threadIdx.x;
   if (i >= N) return;
   const long long bq = blockIdx.y;  // problem of a batched level
@@ -788,7 +790,8 @@ template <int D, int P, bool SSC = false>
 __global__ void __launch_bounds__(kRowT, kRowMinBlocks)
 k_sor_colour(const double* __restrict__ A, long long N, long long Np, long long M, int colour,
              double omega_s, const double* __restrict__ omega, double* x, const double* b, double* r) {
-  pdl_next();
+  if (D == 1) pdl_next_light();
+  else pdl_next();
   constexpr int NS = St<D, P>::NS;
   constexpr int C = St<D, P>::CENTER;
   constexpr int Q = P + 1;
