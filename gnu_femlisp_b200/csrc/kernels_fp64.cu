@@ -1180,13 +1180,26 @@ k_psc_gather_q2(long long N, long long M, int dmask, double damp, const double* 
 // order in which the stencil forms sum their slots, so a structured level
 // given as compressed rows yields the structured results bit for bit.
 
-// The row sums fetch eight entries at a time -- indices and values, then the
-// unknowns -- so a row of up to eight entries waits for memory twice (entry by
-// entry it was twice per few entries), and the first eight are fetched while
-// the previous launch still runs.  Every caller's thread passes pdl_wait here.
+// K = 8: the row sums fetch eight entries at a time -- indices and values, then
+// the unknowns -- so a row of up to eight entries waits for memory twice (entry
+// by entry it was twice per few entries), and the first eight are fetched while
+// the previous launch still runs.  K = 1: entry by entry, for launches of many
+// rows, whose time is instructions and warps and not a row's waits.  1,046,592
+// rows of five entries, eight at a time and one: matvec 25 and 17 us, residual +
+// Jacobi 29 and 21, prolongation 25 and 14; 250,000 rows 7.0 and 5.9, 7.4 and
+// 5.9, 7.2 and 5.1; 125,000 rows of a colour 6.6 both; 65,000 rows 3.9 and 3.8,
+// where the early start gives the eight 1-2 us.  Every caller's thread passes
+// pdl_wait here.
+constexpr long long kCsrWide = 150000;
+template <int K>
 __device__ __forceinline__ double csr_row_sum(const CsrView& a, long long i, const double* x) {
-  constexpr int K = 8;
   const long long e1 = a.start[i + 1];
+  if constexpr (K == 1) {
+    pdl_wait();
+    double s = 0.0;
+    for (long long e = a.start[i]; e < e1; ++e) s = fma(a.value[e], x[a.index[e]], s);
+    return s;
+  }
   long long e = a.start[i];
   int ix[K];
   double v[K];
@@ -1214,28 +1227,47 @@ __device__ __forceinline__ double csr_row_sum(const CsrView& a, long long i, con
   }
   return s;
 }
-constexpr int kCsrT = 64;  // threads per block of the compressed-row kernels: small levels spread over more SMs
+// threads per block: small levels spread over more SMs
+template <int K>
+constexpr int kCsrT = K > 1 ? 64 : kBlock;
+template <int K>
+__device__ __forceinline__ void csr_next() {
+  if (K > 1) pdl_next();
+  else pdl_next_light();
+}
+
+// a row's diagonal and damping: before the wait with K = 8, when they are needed
+// with K = 1 (523,000 rows of a colour 16.6 us, 18.1 early)
+__device__ __forceinline__ void csr_own(const double* diag, const double* omega, double damp, long long i, double& d,
+                                        double& w) {
+  d = __ldg(diag + i);
+  w = omega ? __ldg(omega + i) : damp;
+}
 
 // y = A x, or r = b - A x (b may alias r)
-__global__ void __launch_bounds__(kCsrT, 8)
+template <int K>
+__global__ void __launch_bounds__(kCsrT<K>, K > 1 ? 8 : 0)
 k_csr_spmv(long long N, CsrView a, const double* x, const double* b, double* y, int res) {
-  pdl_next();
+  csr_next<K>();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  const double s = csr_row_sum(a, i, x);
+  const double s = csr_row_sum<K>(a, i, x);
   y[i] = res ? b[i] - s : s;
 }
 
 // compute-residual fused with the following <jacobi> step (as k_row_jacobi_q1)
-__global__ void __launch_bounds__(kCsrT, 8)
+template <int K>
+__global__ void __launch_bounds__(kCsrT<K>, K > 1 ? 8 : 0)
 k_csr_jacobi_res(long long N, CsrView a, const double* __restrict__ diag, double damp,
                  const double* __restrict__ omega, const double* x, const double* b,
                  double* __restrict__ xout, double* r, int write_r) {
-  pdl_next();
+  csr_next<K>();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  const double d = __ldg(diag + i), w = omega ? __ldg(omega + i) : damp;
-  const double s = csr_row_sum(a, i, x);
+  double d, w;
+  if (K > 1) csr_own(diag, omega, damp, i, d, w);
+  const double s = csr_row_sum<K>(a, i, x);
+  if (K == 1) csr_own(diag, omega, damp, i, d, w);
   const double t = (b[i] - s) / d;
   if (write_r) r[i] = t;
   xout[i] = fma(w, t, x[i]);
@@ -1246,15 +1278,18 @@ k_csr_jacobi_res(long long N, CsrView a, const double* __restrict__ diag, double
 // blockit.lisp:131-138) of an algebraic level: rows of the colour in any
 // order (they couple to none of each other), the row sum over the stored
 // entries, columns ascending
-__global__ void __launch_bounds__(kCsrT, 8)
+template <int K>
+__global__ void __launch_bounds__(kCsrT<K>, K > 1 ? 8 : 0)
 k_csr_sor(const int* __restrict__ rows, long long cnt, CsrView a, const double* __restrict__ diag, double omega_s,
           const double* __restrict__ omega, double* x, const double* b, double* r, int ssc) {
-  pdl_next();
+  csr_next<K>();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= cnt) return;
   const long long i = __ldg(rows + t);
-  const double d = __ldg(diag + i), w = omega ? __ldg(omega + i) : omega_s;
-  const double s = csr_row_sum(a, i, x);
+  double d, w;
+  if (K > 1) csr_own(diag, omega, omega_s, i, d, w);
+  const double s = csr_row_sum<K>(a, i, x);
+  if (K == 1) csr_own(diag, omega, omega_s, i, d, w);
   const double rr = b[i] - s;
   const double tt = rr / d;
   r[i] = ssc ? rr : tt;
@@ -1263,27 +1298,29 @@ k_csr_sor(const int* __restrict__ rows, long long cnt, CsrView a, const double* 
 
 // rc = I^T rf row by row of I^T (fine entries ascending); the coarse rhs
 // takes rc, the coarse solution 0 (the :after methods of restrict)
-__global__ void __launch_bounds__(kCsrT, 8)
+template <int K>
+__global__ void __launch_bounds__(kCsrT<K>, K > 1 ? 8 : 0)
 k_csr_restrict(long long NC, CsrView pt, const double* rf, double* rc, double* rhsc, double* solc) {
-  pdl_next();
+  csr_next<K>();
   const long long J = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (J >= NC) return;
-  const double s = csr_row_sum(pt, J, rf);
+  const double s = csr_row_sum<K>(pt, J, rf);
   rc[J] = s;
   if (rhsc) rhsc[J] = s;
   if (solc) solc[J] = 0.0;
 }
 
 // xf += I xc (coarse entries ascending)
-__global__ void __launch_bounds__(kCsrT, 8)
+template <int K>
+__global__ void __launch_bounds__(kCsrT<K>, K > 1 ? 8 : 0)
 k_csr_prolong(long long NF, CsrView p, const double* xc, double* xf) {
-  pdl_next();
+  csr_next<K>();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= NF || p.start[i] == p.start[i + 1]) {  // constrained rows keep their value
     pdl_wait();  // (were all rows empty, the launch would otherwise end before its predecessor)
     return;
   }
-  const double s = csr_row_sum(p, i, xc);
+  const double s = csr_row_sum<K>(p, i, xc);
   xf[i] = xf[i] + s;
 }
 
@@ -3314,11 +3351,18 @@ static dim3 q2_grid(int M, int ssc = -1) {
   return dim3((unsigned)nb, (unsigned)ncol);
 }
 
+// a compressed-row kernel over `rows` rows in the form for that many
+#define CSR_LAUNCH(kern, rows, ...)                                                                      \
+  do {                                                                                                   \
+    if ((rows) > kCsrWide) launch_pdl(kern<1>, grid1(rows, kCsrT<1>), kCsrT<1>, 0, st, __VA_ARGS__);       \
+    else launch_early(kern<8>, grid1(rows, kCsrT<8>), kCsrT<8>, 0, st, __VA_ARGS__);                       \
+  } while (0)
+
 void launch_spmv(const LevelView& L, const double* x, const double* b, double* y, const double* dv,
                  const Reduce* R, cudaStream_t st) {
   if (L.csr) {  // the reduction as a separate DR4096 pass
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    launch_early(k_csr_spmv, grid1(L.N, kCsrT), kCsrT, 0, st, L.N, L.a, x, b, y, b ? 1 : 0);
+    CSR_LAUNCH(k_csr_spmv, L.N, L.N, L.a, x, b, y, b ? 1 : 0);
     if (dv) launch_dot(y, dv, L.N, *R, st);
     return;
   }
@@ -3377,8 +3421,7 @@ void launch_jacobi_res(const LevelView& L, double damp, const double* x, const d
                        double* r, bool write_r, const double* dv, const Reduce* R, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
   if (L.csr) {
-    launch_early(k_csr_jacobi_res, grid1(L.N, kCsrT), kCsrT, 0, st, L.N, L.a, L.diag, damp, L.omega, x, b, xout, r,
-                                                      write_r ? 1 : 0);
+    CSR_LAUNCH(k_csr_jacobi_res, L.N, L.N, L.a, L.diag, damp, L.omega, x, b, xout, r, write_r ? 1 : 0);
     if (dv) launch_dot(xout, dv, L.N, *R, st);
     return;
   }
@@ -3411,8 +3454,7 @@ static void launch_csr_sor(const LevelView& L, double omega, const double* om, d
   for (int c = 0; c < L.ncol; ++c) {
     const long long cnt = L.coff[c + 1] - L.coff[c];
     if (cnt > 0)
-      launch_early(k_csr_sor, grid1(cnt, kCsrT), kCsrT, 0, st,
-                   L.crow + L.coff[c], cnt, L.a, L.diag, omega, om, x, b, r, ssc ? 1 : 0);
+      CSR_LAUNCH(k_csr_sor, cnt, L.crow + L.coff[c], cnt, L.a, L.diag, omega, om, x, b, r, ssc ? 1 : 0);
   }
 }
 
@@ -3530,7 +3572,7 @@ void launch_restrict(const LevelView& F, const LevelView& Cl, const double* rf, 
                      double* solc, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
   if (F.csr) {
-    launch_early(k_csr_restrict, grid1(Cl.N, kCsrT), kCsrT, 0, st, Cl.N, F.pt, rf, rc, rhsc, solc);
+    CSR_LAUNCH(k_csr_restrict, Cl.N, Cl.N, F.pt, rf, rc, rhsc, solc);
     return;
   }
   if (F.nc == 3) {
@@ -3548,7 +3590,7 @@ void launch_restrict(const LevelView& F, const LevelView& Cl, const double* rf, 
 void launch_prolong(const LevelView& Cl, const LevelView& F, const double* xc, double* xf, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
   if (F.csr) {
-    launch_early(k_csr_prolong, grid1(F.N, kCsrT), kCsrT, 0, st, F.N, F.p, xc, xf);
+    CSR_LAUNCH(k_csr_prolong, F.N, F.N, F.p, xc, xf);
     return;
   }
   if (F.nc == 3) {

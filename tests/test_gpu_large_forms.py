@@ -126,3 +126,39 @@ def test_matrix_free_operator(oracle_mod, G, ctx, n0, level, mask):
     diff = np.max(np.abs(X.get() - want)) / np.max(np.abs(want))
     print("relative difference", diff)
     assert diff <= 2 * (level + 1) * 2.0 ** -9
+
+
+def test_wide_compressed_rows(oracle_mod, G, ctx):
+    """A 1D chain of 400,001 unknowns, its two levels below and empty rows: the
+    compressed-row kernels entry by entry (more than 150,000 rows), of the
+    colours and the coarse level too, beside eight at a time below."""
+    import scipy.sparse as sp
+    from _hier import csr_of, oracle_of
+    O, C = oracle_mod, G._capi
+    rng = np.random.default_rng(2)
+    sizes, mats, interp = [800], {}, {}
+    for l, n in ((1, 200001), (2, 400001)):
+        coarse = rng.integers(0, sizes[-1], n)
+        w = rng.uniform(0.5, 1.0, n)
+        w[rng.integers(0, n, n // 50)] = 0.0  # constrained: no entry in the row
+        interp[l] = csr_of(sp.csr_matrix((w, (np.arange(n), coarse)), shape=(n, sizes[-1])))
+        sizes.append(n)
+    for l, n in enumerate(sizes):
+        off = rng.uniform(-1, 0, n - 1)
+        far = rng.uniform(-0.1, 0, n - 9)
+        mats[l] = csr_of(sp.diags([off, off, far, far, np.full(n, 4.0)], [-1, 1, -9, 9, 0]))
+    b = rng.standard_normal(sizes[-1])
+    o = oracle_of(O, sizes, mats, interp, b)
+    g = G.Grid.algebraic(ctx, sizes)
+    for l, m in mats.items():
+        g.set_matrix(l, *m)
+    for l, m in interp.items():
+        g.set_interpolation(l, *m, sizes[l - 1])
+    g.set_rhs(b)
+    for smoother, osm in ((C.FMG_JACOBI, O.JACOBI), (C.FMG_SOR, O.SOR)):
+        ref = o.solve(O.solve_cfg(method=O.METHOD_MG, smoother=osm, damp=0.8, pre=1, post=2, compat=False, rtol=1e-12,
+                                  maxsteps=2))
+        x = g.vector()
+        hist, steps, _ = g.solve(G.SolveCfg(C.FMG_METHOD_MG, smoother, 0.8, 1, 2, 1, 0, 1.0, 1e-12, 0.0, 2,
+                                            C.FMG_MULTIPLICATIVE), x)
+        assert steps == ref.steps and np.array_equal(hist, ref.history) and np.array_equal(x.get(), ref.x)
