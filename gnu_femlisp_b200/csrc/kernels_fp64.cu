@@ -820,7 +820,7 @@ k_sor_colour(const double* __restrict__ A, long long N, long long Np, long long 
   const double rr = b[i] - s;
   const double tt = rr / d;
   r[i] = SSC ? rr : tt;
-  x[i] = fma(w, tt, xv[C]);
+  x[i] = fma(w, tt, !SSC && x == r ? tt : xv[C]);  // one vector for both: x is what r has become
 }
 
 // Step K of the warp's LU factorisation of a vertex block (rows in lanes):
